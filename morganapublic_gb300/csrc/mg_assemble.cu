@@ -4,10 +4,11 @@
 //
 // Every element matrix is computed once, along the plan's Morton element order:
 //   P1 (one pass)  k_block_asm: one CTA per block of consecutive elements, their
-//                  matrices in shared memory, every diagonal or upper CSR entry
-//                  summed there (the plan's block map) and written to the entry
-//                  and its mirror; entries whose elements span blocks get a
-//                  partial sum per block, added in block order by k_shared_sum;
+//                  matrices (two per thread, packed) in shared memory, every
+//                  diagonal or upper CSR entry summed there (the plan's block map)
+//                  and written to the entry and its mirror; entries whose elements
+//                  span blocks get a partial sum per block, added in block order by
+//                  k_shared_sum;
 //   P2 (two passes) k_elem_mat: one thread per element, its 55 unique entries to
 //                  the plan's element-matrix array; k_slot_gather: one thread
 //                  per diagonal or upper CSR entry, the sum of its entries in
@@ -42,6 +43,8 @@
 
 #include "mg_ff.cuh"
 #include "mg_internal.h"
+#include "mg_launch.cuh"
+#include "mg_pair.cuh"
 
 namespace mg {
 
@@ -57,11 +60,11 @@ __device__ __forceinline__ ff operator/(ff a, ff b) { return ff_div(a, b); }
 // An element's scale factor inside the range where the double-word assembly is
 // FP64-accurate: zero, or |v| in 2^-96 .. 2^112 (the error terms of products
 // stay normal floats and no intermediate overflows).
-__device__ __forceinline__ bool dw_scale_ok(ff v)
+__device__ __forceinline__ bool dw_scale_ok(float hi)
 {
-  const uint32_t ex = (__float_as_uint(v.hi) >> 23) & 0xffu;
-  return v.hi == 0.0f || (ex >= 127u - 96u && ex <= 127u + 112u);
+  return hi == 0.0f || (fabsf(hi) >= 0x1p-96f && fabsf(hi) < 0x1p113f);
 }
+__device__ __forceinline__ bool dw_scale_ok(ff v) { return dw_scale_ok(v.hi); }
 
 template <int MODE> struct Arith;
 // sum_into(s, x): s += x for the phase-2 sums.  The double-word form defers
@@ -132,7 +135,7 @@ struct GeoPtrs {
   const float* loz;        // lz
 };
 
-struct FetchAbs {  // four vertices in the three-float form (staged or absolute)
+struct FetchAbs {  // four vertices in the three-float form
   float4 a[4], b[4];
   float lz[4];
 };
@@ -156,12 +159,6 @@ __device__ __forceinline__ void fetch(const GeoPtrs& g, int4 n, FetchAbs& F)
 __device__ __forceinline__ float rec_hi(const float4& a, int r) { return r == 0 ? a.x : (r == 1 ? a.y : a.z); }
 __device__ __forceinline__ float rec_mid(const float4& a, const float4& b, int r) { return r == 0 ? a.w : (r == 1 ? b.x : b.y); }
 __device__ __forceinline__ float rec_lo(const float4& b, float lz, int r) { return r == 0 ? b.z : (r == 1 ? b.w : lz); }
-// the coordinate as a double: hi + mid + lo, every partial sum exact
-__device__ __forceinline__ double rec_x(const float4& a, const float4& b, float lz, int r)
-{
-  return ((double)rec_hi(a, r) + (double)rec_mid(a, b, r)) + (double)rec_lo(b, lz, r);
-}
-
 __device__ __forceinline__ double comp(const double4_32a& v, int r) { return r == 0 ? v.x : (r == 1 ? v.y : v.z); }
 
 __device__ __forceinline__ void geometry(const Fetch<kF64>& F, Cof<double>& f)
@@ -179,7 +176,7 @@ __device__ __forceinline__ void geometry(const Fetch<kF64>& F, Cof<double>& f)
 // and of every entry scaled by 1/det, is that many times the arithmetic's own
 // (measured on GB300: double-word 2.3e-12 and FP32 7e-6 against the FP64 oracle
 // at a cancellation of ~230).  Such elements recompute J, the cofactors and det
-// in FP64 from the staged coordinates -- out of line, so that the rare FP64
+// in FP64 from the exact coordinates -- out of line, so that the rare FP64
 // path does not occupy the FP64 pipe of every other element.
 constexpr float kCancelTol = 16.0f;
 
@@ -200,35 +197,32 @@ __device__ __forceinline__ float hi_of<double>(const double& v) { return (float)
 //    (x3 - x1) x (x2 - x1), accurate to its own magnitude -- cheap in FP32, and
 //    the zero-row-sum form C_0 = -(C_1 + C_2 + C_3) would cost eps |C_max| / |C_0|
 //    relative on the entries of vertex 0, too much at FP32's eps;
-//  - double-word: the zero-row-sum form (eps 2^-47).
+//  - double-word and FP64: the zero-row-sum form (eps 2^-47).
 // Elements whose gradients differ by more than 8x (|C_max| > 8 |C_min| over all
-// four, or a cancelling determinant) take the rare path staged_rare_stiffness: a
+// four, or a cancelling determinant) take the rare path abs_rare_stiffness: a
 // cofactor is a 2x2 minor whose terms then cancel by about that ratio, and so does
 // the zero-row sum; the rare path computes the geometry in FP64 from the exact
 // coordinates, as the reference does.  On a Kuhn cube jittered by 0.25 h (12.6 M
 // tets, ratios up to 21) ~0.01 % of the elements are rare.
-enum { kP1Common = 0, kP1Fp64 = 1 };
-
-template <typename T>
-__device__ __forceinline__ int p1_class(const Cof<T>& f)
+__device__ __forceinline__ bool p1_class(const Cof<double>& f)
 {
   float n[4];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     float na = 0.0f;
 #pragma unroll
-    for (int r = 0; r < 3; ++r) na = fmaf(hi_of(f.c[r][a]), hi_of(f.c[r][a]), na);
+    for (int r = 0; r < 3; ++r) na = fmaf((float)f.c[r][a], (float)f.c[r][a], na);
     n[a + 1] = na;
   }
   n[0] = 0.0f;
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
-    const float s = hi_of(f.c[r][0]) + hi_of(f.c[r][1]) + hi_of(f.c[r][2]);
+    const float s = (float)f.c[r][0] + (float)f.c[r][1] + (float)f.c[r][2];
     n[0] = fmaf(s, s, n[0]);
   }
   const float nmax = fmaxf(fmaxf(n[0], n[1]), fmaxf(n[2], n[3]));
   const float nmin = fminf(fminf(n[0], n[1]), fminf(n[2], n[3]));
-  return nmax > 64.0f * nmin ? kP1Fp64 : kP1Common;
+  return nmax > 64.0f * nmin;
 }
 
 // |det| small against its expansion terms
@@ -289,17 +283,6 @@ __device__ __forceinline__ ff dw_diff3(float hb, float ha, float mb, float ma, f
   const float t = __fadd_rn(__fadd_rn(__fadd_rn(s.lo, s1.lo), s2.lo), __fsub_rn(lb, la));
   return two_sum(s.hi, t);
 }
-// FP64 geometry from three-float coordinates (exact as doubles)
-__device__ __forceinline__ void geometry_fp64(const FetchAbs& F, Cof<double>& d)
-{
-  Fetch<kF64> D;
-#pragma unroll
-  for (int s = 0; s < 4; ++s)
-    D.x[s] = make_double4_32a(rec_x(F.a[s], F.b[s], F.lz[s], 0), rec_x(F.a[s], F.b[s], F.lz[s], 1),
-                              rec_x(F.a[s], F.b[s], F.lz[s], 2), 0.0);
-  geometry(D, d);
-}
-
 // near-degenerate elements: FP64 geometry from the mesh's FP64 coordinates
 static __device__ __noinline__ void recompute_fp64_abs(const GeoPtrs& g, int4 n, Cof<ff>& f)
 {
@@ -331,10 +314,9 @@ __device__ __forceinline__ void geometry_abs(const GeoPtrs& g, int4 n, Cof<ff>& 
 // ------------------------------------------------------- element matrices --
 // P1 stiffness, unique entries in sym_index order:
 // (0,0) (0,1) (0,2) (0,3) (1,1) (1,2) (1,3) (2,2) (2,3) (3,3)
-template <typename T>
-__device__ __forceinline__ void p1_stiff_unique(const Cof<T>& f, T s, T K[10])
+__device__ __forceinline__ void p1_stiff_unique(const Cof<double>& f, double s, double K[10])
 {
-  T d[3][3];
+  double d[3][3];
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -349,34 +331,6 @@ __device__ __forceinline__ void p1_stiff_unique(const Cof<T>& f, T s, T K[10])
   K[8] = d[1][2];
   K[9] = d[2][2];
   K[1] = -(d[0][0] + d[1][0] + d[2][0]);  // rows sum to zero
-  K[2] = -(d[0][1] + d[1][1] + d[2][1]);
-  K[3] = -(d[0][2] + d[1][2] + d[2][2]);
-  K[0] = -(K[1] + K[2] + K[3]);
-}
-
-template <>
-__device__ __forceinline__ void p1_stiff_unique<ff>(const Cof<ff>& f, ff s, ff K[10])
-{
-  ff col[3][3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int r = 0; r < 3; ++r) col[a][r] = f.c[r][a];
-  ff d[3][3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = a; b < 3; ++b) {
-      d[a][b] = ff_mul(s, ff_dot3(col[a], col[b]));
-      d[b][a] = d[a][b];
-    }
-  K[4] = d[0][0];
-  K[5] = d[0][1];
-  K[6] = d[0][2];
-  K[7] = d[1][1];
-  K[8] = d[1][2];
-  K[9] = d[2][2];
-  K[1] = -(d[0][0] + d[1][0] + d[2][0]);
   K[2] = -(d[0][1] + d[1][1] + d[2][1]);
   K[3] = -(d[0][2] + d[1][2] + d[2][2]);
   K[0] = -(K[1] + K[2] + K[3]);
@@ -485,14 +439,12 @@ __device__ __forceinline__ ff metric_dot<ff>(const ff g[6], const ff* tab, int N
 // Geometry of an element from the mesh's absolute node records, in the mode's
 // arithmetic; returns whether the determinant cancels (det_cancels).
 //  FP32          edges (hi_k - hi_0) + (mid_k - mid_0), to a float ulp of the
-//                edge; with c0 (P1 stiffness) also C_0 = (x3 - x1) x (x2 - x1)
-//                from the edge columns;
+//                edge;
 //  double-word   edges dw_diff3 of the three floats: the exact FP64 difference
 //                of the mesh coordinates (the reference's x_k - x_0) to ~2^-47;
 //  FP64          from the FP64 coordinates.
 template <int MODE>
-__device__ __forceinline__ bool geometry_abs_lazy(const GeoPtrs& g, int4 n, Cof<typename Arith<MODE>::T>& f,
-                                                  float* c0)
+__device__ __forceinline__ bool geometry_abs_lazy(const GeoPtrs& g, int4 n, Cof<typename Arith<MODE>::T>& f)
 {
   using T = typename Arith<MODE>::T;
   T J[3][3];
@@ -525,19 +477,6 @@ __device__ __forceinline__ bool geometry_abs_lazy(const GeoPtrs& g, int4 n, Cof<
     }
     if constexpr (MODE == kDW) dw_cofactors(J, f);
     else cofactors<T>(J, f);
-    if constexpr (MODE == kF32) {
-      if (c0) {
-        float f2[3], f3[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          f2[r] = J[r][1] - J[r][0];
-          f3[r] = J[r][2] - J[r][0];
-        }
-        c0[0] = f3[1] * f2[2] - f3[2] * f2[1];
-        c0[1] = f3[2] * f2[0] - f3[0] * f2[2];
-        c0[2] = f3[0] * f2[1] - f3[1] * f2[0];
-      }
-    }
     return det_cancels<T>(J, f);
   }
 }
@@ -627,10 +566,17 @@ struct ElemArgs {
   double cconst;              // used when coeff is null
   const double* tables;       // unique-entry tables: stiff[6][nu] then mass[nu]
   double wsum;
+  float w_hi, w_lo;           // wsum as a double-word
   int stiff;
   void* em;                   // out: nu x n_elem entries
   uint32_t* flags;            // bit 0: NaN / Inf coefficient; bit 1: outside the double-word range
 };
+
+// NaN or Inf: recorded for mg_plan_status
+__device__ __forceinline__ bool coef_not_finite(double c)
+{
+  return ((__double_as_longlong(c) >> 52) & 0x7ff) == 0x7ff;
+}
 
 // The coefficient and the vertex dofs of Morton element p.
 __device__ __forceinline__ double elem_coef(const ElemArgs& a, int64_t p)
@@ -642,54 +588,364 @@ __device__ __forceinline__ int4 elem_nodes(const ElemArgs& a, int64_t p)
   return __ldg(reinterpret_cast<const int4*>(a.dofs_m) + p);
 }
 
-// The P1 element matrix from the element's vertex dofs n and coefficient coef_d
-// (loaded by the caller, elem_nodes / elem_coef).
-template <int MODE>
-__device__ __forceinline__ void p1_element(const ElemArgs& a, const typename Arith<MODE>::T* tab, int4 n,
-                                           double coef_d, typename Arith<MODE>::T K[10])
+// The P1 element matrix in native FP64 from the element's vertex dofs n and
+// coefficient coef.
+__device__ __forceinline__ void p1_element_f64(const ElemArgs& a, const double* mass, int4 n, double coef, double K[10])
 {
-  using A = Arith<MODE>;
-  using T = typename A::T;
-  constexpr int NU = 10;
-  Cof<T> f;
-  float c0[3];
-  const bool degenerate = geometry_abs_lazy<MODE>(a.geo, n, f, MODE == kF32 && a.stiff ? c0 : nullptr);
-  // NaN / Inf coefficient: recorded for mg_plan_status (checked after the
-  // geometry, where the load has long landed)
-  if (((__double_as_longlong(coef_d) >> 52) & 0x7ff) == 0x7ff) atomicOr(a.flags, 1u);
-  const T coef = A::from(coef_d);
+  Cof<double> f;
+  geometry_abs_lazy<kF64>(a.geo, n, f);
+  if (coef_not_finite(coef)) atomicOr(a.flags, 1u);
   if (a.stiff) {
-    // the rare elements (p1_class, or a cancelling determinant) go out of line,
-    // entered only when a lane of the warp has one (~0.01 % of the elements)
-    const bool rare = degenerate || p1_class<T>(f) != kP1Common;
+    // the rare elements (p1_class) go out of line, entered only when a lane of
+    // the warp has one
+    const bool rare = p1_class(f);
     if (__any_sync(__activemask(), rare)) {
       if (rare) {
-        const RareK<T> rk = abs_rare_stiffness<MODE>(a.geo.xyz, n, coef_d, a.wsum, a.flags);
+        const RareK<double> rk = abs_rare_stiffness<kF64>(a.geo.xyz, n, coef, a.wsum, a.flags);
 #pragma unroll
         for (int u = 0; u < 10; ++u) K[u] = rk.K[u];
       }
     }
-    if (!rare) {
-      const T sc = coef * A::from(a.wsum) / f.det;
-      if constexpr (MODE == kF32) {
-        p1_stiff_direct<T>(f, c0, sc, K);  // C_0 from the face opposite vertex 0
+    if (!rare) p1_stiff_unique(f, coef * a.wsum / f.det, K);
+  } else {
+    const double sc = coef * f.det;
+#pragma unroll
+    for (int u = 0; u < 10; ++u) K[u] = sc * mass[u];
+  }
+}
+
+// ------------------------------------------------- P1 elements, two per thread --
+// The same element math on packed pairs (mg_pair.cuh).  The rare elements are
+// found from the finished matrix: gradients that differ by more than 8x show as
+// diagonal entries that differ by more than 64x (K_aa = s |C_a|^2); a cancelling
+// determinant as before; and determinants outside 2^-100 .. 2^100, where the
+// reciprocal estimate would leave the normal floats.
+
+// |det| outside the range of the pair division
+__device__ __forceinline__ bool det_extreme(float det)
+{
+  return !(fabsf(det) >= 0x1p-100f && fabsf(det) <= 0x1p100f);
+}
+// one lane of |J_00 C_00| + |J_01 C_01| + |J_02 C_02| > kCancelTol |det|
+__device__ __forceinline__ bool cancels(float t0, float t1, float t2, float det)
+{
+  return fabsf(t0) + fabsf(t1) + fabsf(t2) > kCancelTol * fabsf(det);
+}
+__device__ __forceinline__ bool diag_spread(float k0, float k1, float k2, float k3)
+{
+  k0 = fabsf(k0), k1 = fabsf(k1), k2 = fabsf(k2), k3 = fabsf(k3);
+  return fmaxf(fmaxf(k0, k1), fmaxf(k2, k3)) > 64.0f * fminf(fminf(k0, k1), fminf(k2, k3));
+}
+
+// The node records of a block: its unique nodes staged in shared memory, indexed by
+// the element's local vertex numbers, or the mesh's in global memory.
+struct StagedNodes {
+  const float4 *a, *b;  // (hi.xyz, mid.x), (mid.yz, lo.xy)
+  const float* z;       // lo.z
+  __device__ __forceinline__ float4 first(int i) const { return a[i]; }
+  __device__ __forceinline__ float4 second(int i) const { return b[i]; }
+  __device__ __forceinline__ float last(int i) const { return z[i]; }
+};
+struct GlobalNodes {
+  GeoPtrs g;
+  __device__ __forceinline__ float4 first(int i) const { return __ldg(g.rec + 2 * (int64_t)i); }
+  __device__ __forceinline__ float4 second(int i) const { return __ldg(g.rec + 2 * (int64_t)i + 1); }
+  __device__ __forceinline__ float last(int i) const { return __ldg(g.loz + i); }
+};
+
+// Edge vectors x_k - x_0 of one element as double-words, component r of edge k at
+// 3 r + k.  SPLIT: the node records are split on per-axis grids (mg_mesh::grid_split),
+// so the differences of the high and of the middle parts are exact and ordered
+// (|d hi| >= |d mid| unless d hi = 0): 7 operations per component against 28.
+template <bool SPLIT, typename N>
+__device__ __forceinline__ void edges_dw(const N& g, int4 n, float (&hi)[9], float (&lo)[9])
+{
+  const float4 a0 = g.first(n.x), b0 = g.second(n.x);
+  const float z0 = g.last(n.x);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int id = k == 0 ? n.y : (k == 1 ? n.z : n.w);
+    const float4 ak = g.first(id), bk = g.second(id);
+    const float zk = g.last(id);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      ff d;
+      if constexpr (SPLIT) {
+        d = fast_two_sum(__fsub_rn(rec_hi(ak, r), rec_hi(a0, r)), __fsub_rn(rec_mid(ak, bk, r), rec_mid(a0, b0, r)));
+        d.lo = __fadd_rn(d.lo, __fsub_rn(rec_lo(bk, zk, r), rec_lo(b0, z0, r)));
       } else {
-        p1_stiff_unique<T>(f, sc, K);
-        if constexpr (MODE == kDW)
-          if (!dw_scale_ok(sc) || !dw_scale_ok(K[4])) atomicOr(a.flags, 2u);
+        d = dw_diff3(rec_hi(ak, r), rec_hi(a0, r), rec_mid(ak, bk, r), rec_mid(a0, b0, r), rec_lo(bk, zk, r),
+                     rec_lo(b0, z0, r));
+      }
+      hi[3 * r + k] = d.hi;
+      lo[3 * r + k] = d.lo;
+    }
+  }
+}
+// ... and as floats: (hi_k - hi_0) + (mid_k - mid_0), to a float ulp of the edge
+template <typename N>
+__device__ __forceinline__ void edges_f32(const N& g, int4 n, float (&x)[9])
+{
+  const float4 a0 = g.first(n.x), b0 = g.second(n.x);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int id = k == 0 ? n.y : (k == 1 ? n.z : n.w);
+    const float4 ak = g.first(id), bk = g.second(id);
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+      x[3 * r + k] = (rec_hi(ak, r) - rec_hi(a0, r)) + (rec_mid(ak, bk, r) - rec_mid(a0, b0, r));
+  }
+}
+template <int MODE> struct Pair;
+template <> struct Pair<kDW> { using T = ff2; };
+template <> struct Pair<kF32> { using T = f2; };
+// both elements' edges as packed pairs
+template <bool SPLIT, typename N>
+__device__ __forceinline__ void pair_edges(const N& g, int4 n0, int4 n1, ff2 (&J)[3][3])
+{
+  float h0[9], l0[9], h1[9], l1[9];
+  edges_dw<SPLIT>(g, n0, h0, l0);
+  edges_dw<SPLIT>(g, n1, h1, l1);
+#pragma unroll
+  for (int i = 0; i < 9; ++i) J[i / 3][i % 3] = ff2{f2_make(h0[i], h1[i]), f2_make(l0[i], l1[i])};
+}
+template <bool, typename N>
+__device__ __forceinline__ void pair_edges(const N& g, int4 n0, int4 n1, f2 (&J)[3][3])
+{
+  float x0[9], x1[9];
+  edges_f32(g, n0, x0);
+  edges_f32(g, n1, x1);
+#pragma unroll
+  for (int i = 0; i < 9; ++i) J[i / 3][i % 3] = f2_make(x0[i], x1[i]);
+}
+
+// Two element matrices into the block's shared array: entry u of the block's
+// element l at em[u kElemBlock + l], the pair at l = lp and lp + 32 (a warp's lanes
+// take consecutive elements: their vertices share cache lines, and the stores are
+// conflict-free).  Double-word low parts in a second array.
+__device__ __forceinline__ void em_pair(float* em, int u, int lp, f2 v)
+{
+  const float2 x = f2_get(v);
+  em[u * kElemBlock + lp] = x.x;
+  em[u * kElemBlock + lp + 32] = x.y;
+}
+
+// From the pair's edges J and coefficients; node(e): the global vertex ids of
+// element e of the pair (for the rare paths).
+template <typename Node>
+__device__ __forceinline__ void p1_pair_dw(const ElemArgs& a, const ff* mass, const ff2 (&J)[3][3], Node node, double coef0,
+                                           double coef1, int lp, float* em_hi, float* em_lo)
+{
+  ff2 C[3][3];  // C[k]: cofactor column k of J (C[k][r] = cofactor (r, k))
+  ff2 det;
+  bool degen0, degen1;
+  {
+    f2 nJ[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) nJ[r][k] = -J[r][k].hi;
+#define MG_COF(r, k, r1, k1, r2, k2) \
+  C[k][r] = ff2_cross(J[r1][k1], J[r2][k2], J[r1][k2], J[r2][k1], nJ[r1][k1], nJ[r1][k2], nJ[r2][k1])
+    MG_COF(0, 0, 1, 1, 2, 2);
+    MG_COF(0, 1, 1, 2, 2, 0);
+    MG_COF(0, 2, 1, 0, 2, 1);
+    MG_COF(1, 0, 2, 1, 0, 2);
+    MG_COF(1, 1, 2, 2, 0, 0);
+    MG_COF(1, 2, 2, 0, 0, 1);
+    MG_COF(2, 0, 0, 1, 1, 2);
+    MG_COF(2, 1, 0, 2, 1, 0);
+    MG_COF(2, 2, 0, 0, 1, 1);
+#undef MG_COF
+    const ff2 c0[3] = {C[0][0], C[1][0], C[2][0]};
+    const ff2 d = ff2_dot3(J[0], c0, nJ[0]);
+    det = f2_fast_two_sum(d.hi, d.lo);
+    const float2 dh = f2_get(det.hi), t0 = f2_get(J[0][0].hi * c0[0].hi), t1 = f2_get(J[0][1].hi * c0[1].hi),
+                 t2 = f2_get(J[0][2].hi * c0[2].hi);
+    degen0 = cancels(t0.x, t1.x, t2.x, dh.x);
+    degen1 = cancels(t0.y, t1.y, t2.y, dh.y);
+    if (a.stiff) {
+      degen0 |= det_extreme(dh.x);
+      degen1 |= det_extreme(dh.y);
+    }
+  }
+  if (coef_not_finite(coef0) || coef_not_finite(coef1)) atomicOr(a.flags, 1u);
+  const ff2 coef = ff2_make(ff_from_double_bits(coef0), ff_from_double_bits(coef1));
+  if (a.stiff) {
+    // s = coef w / det: quotient digits q1 + q2 + q3, the remainder of each by FMAs
+    ff2 s;
+    {
+      const f2 wh = f2_make(a.w_hi, a.w_hi), wl = f2_make(a.w_lo, a.w_lo);
+      const f2 nh = coef.hi * wh;
+      const f2 nl = fma2(coef.lo, wh, coef.hi * wl) - fma2(-coef.hi, wh, nh);
+      const f2 rb = f2_rcp(det.hi), nd = -det.hi;
+      const f2 q1 = nh * rb;
+      const f2 r1 = fma2(nd, q1, nh) + fma2(-det.lo, q1, nl);
+      const f2 q2 = r1 * rb;
+      const f2 q3 = fma2(nd, q2, r1) * rb;
+      s = f2_fast_two_sum(q1, q2 + q3);
+    }
+    ff2 K[10];
+    {
+      const f2 ns = -s.hi;
+      f2 nC[3][3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int r = 0; r < 3; ++r) nC[k][r] = -C[k][r].hi;
+      const int ui[6] = {4, 5, 6, 7, 8, 9}, ua[6] = {0, 0, 0, 1, 1, 2}, ub[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+      for (int t = 0; t < 6; ++t) {
+        ff2 d = ff2_dot3(C[ua[t]], C[ub[t]], nC[ua[t]]);
+        d = f2_fast_two_sum(d.hi, d.lo);
+        const f2 p = s.hi * d.hi;
+        const f2 lo = fma2(s.hi, d.lo, s.lo * d.hi) - fma2(ns, d.hi, p);
+        K[ui[t]] = f2_fast_two_sum(p, lo);
+      }
+      // vertex 0 from the zero row sums, the sums of the high parts error-free
+      const ff2* R[3][3] = {{&K[4], &K[5], &K[6]}, {&K[5], &K[7], &K[8]}, {&K[6], &K[8], &K[9]}};
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        const ff2 x = f2_two_sum(R[t][0]->hi, R[t][1]->hi), y = f2_two_sum(x.hi, R[t][2]->hi);
+        K[1 + t] = f2_fast_two_sum(y.hi, (R[t][0]->lo + R[t][1]->lo) + (R[t][2]->lo + (x.lo + y.lo)));
+      }
+      const ff2 x = f2_two_sum(K[1].hi, K[2].hi), y = f2_two_sum(x.hi, K[3].hi);
+      K[0] = f2_fast_two_sum(y.hi, (K[1].lo + K[2].lo) + (K[3].lo + (x.lo + y.lo)));
+    }
+#pragma unroll
+    for (int u = 0; u < 10; ++u) {
+      const bool neg = u >= 1 && u <= 3;
+      em_pair(em_hi, u, lp, neg ? -K[u].hi : K[u].hi);
+      em_pair(em_lo, u, lp, neg ? -K[u].lo : K[u].lo);
+    }
+    const float2 k0 = f2_get(K[0].hi), k1 = f2_get(K[4].hi), k2 = f2_get(K[7].hi), k3 = f2_get(K[9].hi),
+                 sh = f2_get(s.hi);
+    const bool rare0 = degen0 || diag_spread(k0.x, k1.x, k2.x, k3.x);
+    const bool rare1 = degen1 || diag_spread(k0.y, k1.y, k2.y, k3.y);
+    if ((!rare0 && !(dw_scale_ok(sh.x) && dw_scale_ok(k1.x))) || (!rare1 && !(dw_scale_ok(sh.y) && dw_scale_ok(k1.y))))
+      atomicOr(a.flags, 2u);
+    // the rare elements (~0.01 %) again, out of line in FP64 geometry
+    if (rare0 || rare1) {
+#pragma unroll 1
+      for (int e = rare0 ? 0 : 1; e < (rare1 ? 2 : 1); ++e) {
+        const RareK<ff> rk = abs_rare_stiffness<kDW>(a.geo.xyz, node(e), e ? coef1 : coef0, a.wsum, a.flags);
+#pragma unroll
+        for (int u = 0; u < 10; ++u) {
+          em_hi[u * kElemBlock + lp + 32 * e] = rk.K[u].hi;
+          em_lo[u * kElemBlock + lp + 32 * e] = rk.K[u].lo;
+        }
       }
     }
   } else {
-    if constexpr (MODE != kF64) {
-      if (__any_sync(__activemask(), degenerate)) {
-        if (degenerate) f = abs_geometry_fp64<T>(a.geo.xyz, n);
+    if (degen0 || degen1) {
+      const ff x = degen0 ? abs_geometry_fp64<ff>(a.geo.xyz, node(0)).det
+                          : ff{f2_get(det.hi).x, f2_get(det.lo).x};
+      const ff y = degen1 ? abs_geometry_fp64<ff>(a.geo.xyz, node(1)).det
+                          : ff{f2_get(det.hi).y, f2_get(det.lo).y};
+      det = ff2_make(x, y);
+    }
+    const f2 nc = -coef.hi, p = coef.hi * det.hi;
+    const f2 lo = fma2(coef.hi, det.lo, coef.lo * det.hi);
+    const ff2 sc = f2_fast_two_sum(p, lo - fma2(nc, det.hi, p));
+    const float2 sh = f2_get(sc.hi);
+    if (!dw_scale_ok(sh.x) || !dw_scale_ok(sh.y)) atomicOr(a.flags, 2u);
+    const f2 ns = -sc.hi;
+#pragma unroll
+    for (int u = 0; u < 10; ++u) {
+      const f2 th = f2_make(mass[u].hi, mass[u].hi), tl = f2_make(mass[u].lo, mass[u].lo);
+      const f2 q = sc.hi * th;
+      const ff2 k = f2_fast_two_sum(q, fma2(sc.hi, tl, sc.lo * th) - fma2(ns, th, q));
+      em_pair(em_hi, u, lp, k.hi);
+      em_pair(em_lo, u, lp, k.lo);
+    }
+  }
+}
+
+template <typename Node>
+__device__ __forceinline__ void p1_pair_f32(const ElemArgs& a, const float* mass, const f2 (&J)[3][3], Node node,
+                                            double coef0, double coef1, int lp, float* em)
+{
+  f2 C[3][3];  // cofactor columns
+  f2 nJ[3][3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) nJ[r][k] = -J[r][k];
+#define MG_COF(r, k, r1, k1, r2, k2) C[k][r] = f2_cross(J[r1][k1], J[r2][k2], J[r1][k2], J[r2][k1], nJ[r1][k2])
+  MG_COF(0, 0, 1, 1, 2, 2);
+  MG_COF(0, 1, 1, 2, 2, 0);
+  MG_COF(0, 2, 1, 0, 2, 1);
+  MG_COF(1, 0, 2, 1, 0, 2);
+  MG_COF(1, 1, 2, 2, 0, 0);
+  MG_COF(1, 2, 2, 0, 0, 1);
+  MG_COF(2, 0, 0, 1, 1, 2);
+  MG_COF(2, 1, 0, 2, 1, 0);
+  MG_COF(2, 2, 0, 0, 1, 1);
+#undef MG_COF
+  f2 det = fma2(J[0][2], C[2][0], fma2(J[0][1], C[1][0], J[0][0] * C[0][0]));
+  bool degen0, degen1;
+  {
+    const float2 dh = f2_get(det), t0 = f2_get(J[0][0] * C[0][0]), t1 = f2_get(J[0][1] * C[1][0]),
+                 t2 = f2_get(J[0][2] * C[2][0]);
+    degen0 = cancels(t0.x, t1.x, t2.x, dh.x);
+    degen1 = cancels(t0.y, t1.y, t2.y, dh.y);
+    if (a.stiff) {
+      degen0 |= det_extreme(dh.x);
+      degen1 |= det_extreme(dh.y);
+    }
+  }
+  if (coef_not_finite(coef0) || coef_not_finite(coef1)) atomicOr(a.flags, 1u);
+  const f2 coef = f2_make(Arith<kF32>::from(coef0), Arith<kF32>::from(coef1));
+  if (a.stiff) {
+    // C_0 from the face opposite vertex 0, (x3 - x1) x (x2 - x1)
+    f2 C0[3];
+    {
+      f2 e2[3], e3[3];
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        e2[r] = J[r][1] - J[r][0];
+        e3[r] = J[r][2] - J[r][0];
+      }
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const int r1 = (r + 1) % 3, r2 = (r + 2) % 3;
+        C0[r] = f2_cross(e3[r1], e2[r2], e3[r2], e2[r1], -e3[r2]);
       }
     }
-    const T sc = coef * f.det;
-    if constexpr (MODE == kDW)
-      if (!dw_scale_ok(sc)) atomicOr(a.flags, 2u);
+    // s = coef w / det, one correction of the quotient estimate
+    const f2 nu = coef * f2_make(a.w_hi, a.w_hi), rb = f2_rcp(det), q = nu * rb;
+    const f2 s = fma2(fma2(-det, q, nu), rb, q);
+    const f2* G[4] = {C0, C[0], C[1], C[2]};
+    f2 diag[4];
+    int u = 0;
 #pragma unroll
-    for (int u = 0; u < 10; ++u) K[u] = sc * tab[6 * NU + u];
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = i; j < 4; ++j, ++u) {
+        const f2 k = s * fma2(G[i][2], G[j][2], fma2(G[i][1], G[j][1], G[i][0] * G[j][0]));
+        if (j == i) diag[i] = k;
+        em_pair(em, u, lp, k);
+      }
+    const float2 k0 = f2_get(diag[0]), k1 = f2_get(diag[1]), k2 = f2_get(diag[2]), k3 = f2_get(diag[3]);
+    const bool rare0 = degen0 || diag_spread(k0.x, k1.x, k2.x, k3.x);
+    const bool rare1 = degen1 || diag_spread(k0.y, k1.y, k2.y, k3.y);
+    if (rare0 || rare1) {
+#pragma unroll 1
+      for (int e = rare0 ? 0 : 1; e < (rare1 ? 2 : 1); ++e) {
+        const RareK<float> rk = abs_rare_stiffness<kF32>(a.geo.xyz, node(e), e ? coef1 : coef0, a.wsum, a.flags);
+#pragma unroll
+        for (int v = 0; v < 10; ++v) em[v * kElemBlock + lp + 32 * e] = rk.K[v];
+      }
+    }
+  } else {
+    if (degen0 || degen1) {
+      const float2 d = f2_get(det);
+      det = f2_make(degen0 ? abs_geometry_fp64<float>(a.geo.xyz, node(0)).det : d.x,
+                    degen1 ? abs_geometry_fp64<float>(a.geo.xyz, node(1)).det : d.y);
+    }
+    const f2 sc = coef * det;
+#pragma unroll
+    for (int u = 0; u < 10; ++u) em_pair(em, u, lp, sc * f2_make(mass[u], mass[u]));
   }
 }
 
@@ -714,8 +970,8 @@ __global__ void __launch_bounds__(256, 1) k_elem_mat(ElemArgs a)
     const int32_t* dp = a.dofs_m + p * 10;
     const int4 n = make_int4(dp[0], dp[1], dp[2], dp[3]);
     Cof<T> f;
-    const bool degenerate = geometry_abs_lazy<MODE>(a.geo, n, f, nullptr);
-    if (((__double_as_longlong(coef_d) >> 52) & 0x7ff) == 0x7ff) atomicOr(a.flags, 1u);
+    const bool degenerate = geometry_abs_lazy<MODE>(a.geo, n, f);
+    if (coef_not_finite(coef_d)) atomicOr(a.flags, 1u);
     const T coef = A::from(coef_d);
     if constexpr (MODE != kF64) {
       if (__any_sync(__activemask(), degenerate)) {
@@ -790,68 +1046,90 @@ __global__ void __launch_bounds__(256) k_slot_gather(int64_t n_groups, int64_t n
 
 // ---------------------------------------------------- one-pass assembly (P1) --
 // k_block_asm: one CTA per block of kElemBlock consecutive Morton positions.
-//   1. each thread computes the element matrices of one or two elements into
-//      shared memory (10 unique entries each);
+//   1. the records of the block's unique nodes, its coefficients and its part of
+//      the block map come into shared memory by cp.async; each thread computes the
+//      matrices of two elements as packed pairs into shared memory (10 unique
+//      entries each);
 //   2. each warp takes groups of 32 of the block's local entries (the block map):
-//      lane l sums its entry's local sources in ascending p, and writes the sum
-//      to the CSR entry and its mirror when every source of the entry lies in
-//      this block, else to the entry's partial-sum slot.
+//      lane l sums its entry's local sources, and writes the sum to the CSR entry and
+//      its mirror when every source of the entry lies in this block, else to the
+//      entry's partial-sum slot.
 // k_shared_sum: one warp per group of 32 shared entries: the partial sums in
 //   ascending block (coalesced [j][lane]), written to the entry and its mirror.
 // Each entry's summation order is fixed by the plan, so the values are bitwise
-// reproducible; no atomics, no element matrix leaves the SM.
+// reproducible; no atomics, no element matrix leaves the SM.  Both kernels are
+// launched with programmatic dependent launch: what they read of the plan overlaps
+// the tail of the kernel before.
+//
+// What bounds it on GB300 (P1 128^3, FP64, one assembly 949 -> 709 us; FP32 at 64^3
+// 75 -> 61 us, both with k_shared_sum).  One element per thread and scalar
+// double-words took 46 warp instructions per element at 57 % issue.  The packed
+// pairs with grid-split coordinates take 27, and left latency as the bound:
+//   - random vertex and coefficient loads need an L1 line each while in flight,
+//     and the blocks' shared memory leaves few lines: nodes staged by cp.async 833 ->
+//     743 us, coefficients by cp.async 782 -> 745 us;
+//   - occupancy: three CTAs of 256 threads at 80 registers 789 us, two at 128
+//     registers 889 us, four at 64 registers (spills) 880 us;
+//   - the map rows' outputs staged beside the sources, uniform loop bounds in the
+//     sums: 750 -> 727 us.
+// About half of the issue slots are used; the rest is the latency of the block's phases,
+// the scattered 8-byte writes of the sums (~30 us) and k_shared_sum (~130 us).
 struct BlockArgs {
   const int32_t* bgrp;
   const int32_t* bsrc0;
   const int32_t* bgoff;
   const uint16_t* bsrc;
   const int2* bout;
-  void* partial;  // 8-byte slots: float2 (double-word), double, or a float in the low half
+  void* partial;  // 8-byte slots: a double, or a float in the low half
+  const int32_t* bnode;        // kStageNodes per block: its unique nodes, the last repeated
+  const int32_t* bnode_n;      // their number, or -1 (more than kStageNodes)
+  const uchar4* elem_local;    // per Morton position, the vertices' places among them
 };
 
-__device__ __forceinline__ void partial_put(void* pp, int32_t q, float v) { static_cast<float2*>(pp)[q].x = v; }
-__device__ __forceinline__ void partial_put(void* pp, int32_t q, ff v)
-{
-  static_cast<float2*>(pp)[q] = make_float2(v.hi, v.lo);
-}
-__device__ __forceinline__ void partial_put(void* pp, int32_t q, double v) { static_cast<double*>(pp)[q] = v; }
-template <typename T> __device__ __forceinline__ T partial_get(const void* pp, int32_t q);
-template <> __device__ __forceinline__ float partial_get<float>(const void* pp, int32_t q)
-{
-  return __ldg(static_cast<const float2*>(pp) + q).x;
-}
-template <> __device__ __forceinline__ ff partial_get<ff>(const void* pp, int32_t q)
-{
-  const float2 v = __ldg(static_cast<const float2*>(pp) + q);
-  return ff{v.x, v.y};
-}
-template <> __device__ __forceinline__ double partial_get<double>(const void* pp, int32_t q)
-{
-  return __ldg(static_cast<const double*>(pp) + q);
-}
-
-// Block-map staging in shared memory: the block's local sources (up to
-// kStageSrc, the first groups' rows) and group offsets (up to kStageGroups + 1),
-// copied with cp.async while the element matrices are computed.
+// Block-map staging in shared memory: the block's local sources (kStageSrc) and its
+// groups' outputs and offsets (kStageGroups), copied with cp.async while the element
+// matrices are computed.  A block of 512 elements of a volume mesh has about 5,500
+// sources in 33 groups; one with more than the stage holds copies the first of them
+// and reads its map from global memory.
 constexpr int kStageSrc = 6144;
-constexpr int kStageGroups = 96;
-// dynamic shared memory of a block: its element matrices (BE x NU entries, then
-// the zero of the padding sources), the staged sources and group offsets
-template <typename T, int BE, int NU>
-__host__ __device__ constexpr size_t block_em_bytes()
-{
-  return ((sizeof(T) * (BE * NU + 1) + 15) / 16) * 16;
-}
-template <typename T, int BE, int NU>
+constexpr int kStageGroups = 40;
+// The block's element matrices in shared memory: entry u of local element l at
+// u kElemBlock + l -- consecutive elements in consecutive words, so a warp's stores
+// are conflict-free -- then the zero of the padding sources.  Double-words keep
+// their low parts in a second array of kEmStride floats.
+constexpr int kEmStride = 10 * kElemBlock + 4;
+template <int MODE>
+constexpr size_t kEmBytes = (MODE == kF32 ? sizeof(float) : sizeof(double)) * kEmStride;
+// dynamic shared memory of a block: its element matrices, the staged sources, node
+// records and ids, and group offsets
+constexpr size_t kNodeStageBytes = kStageNodes * (2 * sizeof(float4) + sizeof(float) + sizeof(int32_t));
+template <int MODE>
 __host__ __device__ constexpr size_t block_smem_bytes()
 {
-  return block_em_bytes<T, BE, NU>() + 2 * kStageSrc + 4 * (kStageGroups + 1);
+  return kEmBytes<MODE> + 2 * kStageSrc + 256 * kStageGroups + (MODE == kF64 ? 0 : kNodeStageBytes) +
+         4 * (kStageGroups + 1);
 }
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
 {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
                "l"(gmem));
+}
+// The double c[e] of an array of n, copied asynchronously into the 16-byte slot
+// `smem` as the aligned 16 bytes that hold it (read back with coef_slot).  The bypassing copy
+// takes no L1 line: random 8-byte loads would each hold one while in flight, and the
+// blocks' shared memory leaves few.  Where those 16 bytes reach past the array
+// (an end of an array that is odd in length or off the 16-byte grid) the value is stored.
+__device__ __forceinline__ void coef_fetch(double* smem, const double* c, int64_t e, int64_t n)
+{
+  const int odd = (int)((reinterpret_cast<uintptr_t>(c + e) >> 3) & 1);
+  const int64_t e0 = e - odd;
+  if (e0 >= 0 && e0 + 1 < n) cp_async16(smem, c + e0);
+  else smem[odd] = __ldg(c + e);
+}
+__device__ __forceinline__ double coef_slot(const double* smem, const double* c, int64_t e)
+{
+  return smem[(reinterpret_cast<uintptr_t>(c + e) >> 3) & 1];
 }
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem)
 {
@@ -865,136 +1143,227 @@ __device__ __forceinline__ void cp_async4(void* smem, const void* gmem)
 // group offsets, each up to the stage's size.
 template <int THREADS>
 __device__ __forceinline__ void stage_block_map(const BlockArgs& bm, int32_t g0, int32_t g1, int32_t src0,
-                                                int32_t src1, uint16_t* s_src, int32_t* s_goff)
+                                                int32_t src1, uint16_t* s_src, int2* s_out, int32_t* s_goff)
 {
   const int32_t n_src = min(src1 - src0, kStageSrc), n_goff = min(g1 - g0, kStageGroups) + 1;
+  const int32_t n_out = 32 * min(g1 - g0, kStageGroups);
   for (int i = threadIdx.x; i < n_src / 8; i += THREADS) cp_async16(s_src + 8 * i, bm.bsrc + src0 + 8 * i);
+  for (int i = threadIdx.x; i < n_out / 2; i += THREADS) cp_async16(s_out + 2 * i, bm.bout + 32 * (int64_t)g0 + 2 * i);
   for (int i = threadIdx.x; i < n_goff; i += THREADS) cp_async4(s_goff + i, bm.bgoff + g0 + i);
   asm volatile("cp.async.commit_group;\n" ::);
 }
 
-// Phase 2 of the block assembly: each warp takes groups of 32 of the block's
-// runs; lane l sums its run's sources from the element matrices em in shared
-// memory (4 at a time, ascending p) and writes a complete entry to its CSR
-// position and mirror, a shared entry's partial to its slot.  Rows past the
-// stage come from global memory.
-template <int MODE, int THREADS>
-__device__ __forceinline__ void block_sums(const BlockArgs& bm, int32_t g0, int32_t g1, int32_t src0,
-                                           const uint16_t* s_src, const int32_t* s_goff,
-                                           const typename Arith<MODE>::T* em,
-                                           typename Arith<MODE>::Out* __restrict__ values)
+// One run's sum by one lane, four sources per step, from the byte offsets `src`
+// (row j at src[32 j]) of the block's entries; rows past L read the zero entry.  The
+// rows j and j + 1 go to two accumulators as a packed pair, combined at the end.
+__device__ __forceinline__ uint32_t src_row(const uint16_t* src, int32_t j, int32_t L)
 {
-  using A = Arith<MODE>;
-  using T = typename A::T;
-  const int lane = threadIdx.x & 31;
-  for (int32_t g = g0 + (threadIdx.x >> 5); g < g1; g += THREADS / 32) {
-    const int2 out = bm.bout[32 * g + lane];  // used after the sum: its latency overlaps it
-    const int32_t gi = g - g0;
-    const int32_t o = gi < kStageGroups ? s_goff[gi] : bm.bgoff[g];
-    const int32_t o1 = gi + 1 <= kStageGroups ? s_goff[gi + 1] : bm.bgoff[g + 1];
-    const int32_t L = (o1 - o) >> 5;
-    T v = A::zero();
-    if (o1 - src0 <= kStageSrc) {
-      const uint16_t* s = s_src + (o - src0) + lane;
-      int32_t j = 0;
-      for (; j + 4 <= L; j += 4) {
-        const uint32_t i0 = s[32 * j], i1 = s[32 * j + 32], i2 = s[32 * j + 64], i3 = s[32 * j + 96];
-        const T x0 = em[i0], x1 = em[i1], x2 = em[i2], x3 = em[i3];
-        A::sum_into(v, x0);
-        A::sum_into(v, x1);
-        A::sum_into(v, x2);
-        A::sum_into(v, x3);
-      }
-      for (; j < L; ++j) A::sum_into(v, em[s[32 * j]]);
-    } else {
-      // past the stage (rare): the rows from global memory, 4 in flight
-      const uint16_t* s = bm.bsrc + o + lane;
-      int32_t j = 0;
-      for (; j + 4 <= L; j += 4) {
-        const uint32_t i0 = __ldg(s + 32 * j), i1 = __ldg(s + 32 * j + 32), i2 = __ldg(s + 32 * j + 64),
-                       i3 = __ldg(s + 32 * j + 96);
-        A::sum_into(v, em[i0]);
-        A::sum_into(v, em[i1]);
-        A::sum_into(v, em[i2]);
-        A::sum_into(v, em[i3]);
-      }
-      for (; j < L; ++j) A::sum_into(v, em[__ldg(s + 32 * j)]);
+  return j < L ? src[32 * j] : 4u * 10u * kElemBlock;
+}
+__device__ __forceinline__ float em_at(const unsigned char* em, uint32_t off)
+{
+  return *reinterpret_cast<const float*>(em + off);
+}
+template <int MODE>
+__device__ __forceinline__ typename Arith<MODE>::Out run_sum(const unsigned char* em, const uint16_t* src, int32_t L)
+{
+  if constexpr (MODE == kDW) {
+    // error-free sums of the high parts, the low parts and errors collected
+    const unsigned char* em_lo = em + 4 * kEmStride;
+    ff2 s{f2_make(0.0f, 0.0f), f2_make(0.0f, 0.0f)};
+    for (int32_t j = 0; j < L; j += 4) {
+      const uint32_t i0 = src_row(src, j, L), i1 = src_row(src, j + 1, L), i2 = src_row(src, j + 2, L),
+                     i3 = src_row(src, j + 3, L);
+      const ff2 x{f2_make(em_at(em, i0), em_at(em, i1)), f2_make(em_at(em_lo, i0), em_at(em_lo, i1))};
+      const ff2 y{f2_make(em_at(em, i2), em_at(em, i3)), f2_make(em_at(em_lo, i2), em_at(em_lo, i3))};
+      const ff2 t = f2_two_sum(s.hi, x.hi), u = f2_two_sum(t.hi, y.hi);
+      s.hi = u.hi;
+      s.lo = s.lo + ((t.lo + x.lo) + (u.lo + y.lo));
     }
-    if (out.x >= 0) {
-      const typename A::Out r = A::out(v);
-      values[out.x] = r;
-      if (out.y != out.x) values[out.y] = r;
-    } else if (out.x != kNoOutput) {
-      partial_put(bm.partial, -1 - out.x, v);
+    const float2 h = f2_get(s.hi), l = f2_get(s.lo);
+    const ff t = two_sum(h.x, h.y);
+    return (double)t.hi + (double)__fadd_rn(t.lo, __fadd_rn(l.x, l.y));
+  } else if constexpr (MODE == kF32) {
+    f2 s = f2_make(0.0f, 0.0f);
+    for (int32_t j = 0; j < L; j += 4) {
+      const uint32_t i0 = src_row(src, j, L), i1 = src_row(src, j + 1, L), i2 = src_row(src, j + 2, L),
+                     i3 = src_row(src, j + 3, L);
+      s = (s + f2_make(em_at(em, i0), em_at(em, i1))) + f2_make(em_at(em, i2), em_at(em, i3));
     }
+    const float2 h = f2_get(s);
+    return h.x + h.y;
+  } else {
+    double s = 0.0;
+    for (int32_t j = 0; j < L; ++j) s += *reinterpret_cast<const double*>(em + 2 * src[32 * j]);
+    return s;
   }
 }
 
-// P1: one CTA per block of kElemBlock elements.  THREADS per CTA: 512 (one
-// element each, two CTAs per SM) for the double-word and FP64 arithmetic, 256
-// (two elements each, four CTAs per SM) for FP32 -- measured on GB300 at P1
-// 128^3 (the double-word loop over two elements spills).
+// Phase 2 of the block assembly: each warp takes groups of 32 of the block's
+// runs; lane l sums its run's sources from the element matrices em in shared
+// memory and writes a complete entry to its CSR position and mirror, a shared
+// entry's partial to its slot.  A block whose map exceeds the stage (rare) reads it
+// from global memory.  Loop bounds go through shuffles, which makes them uniform
+// for the compiler: no divergence handling around the loops.
 template <int MODE, int THREADS>
-__global__ void __launch_bounds__(THREADS, 2048 / THREADS / 2)
+__device__ __forceinline__ void block_sums_from(const BlockArgs& bm, int32_t g0, int32_t g1, int32_t src0,
+                                                const uint16_t* src, const int2* out_of, const int32_t* goff,
+                                                const unsigned char* em, typename Arith<MODE>::Out* __restrict__ values)
+{
+  using Out = typename Arith<MODE>::Out;
+  const int lane = threadIdx.x & 31;
+  const int n = g1 - g0;
+  for (int gi = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); gi < n; gi += THREADS / 32) {
+    const int2 out = out_of[32 * gi + lane];
+    const int32_t o = goff[gi];
+    const int32_t L = __shfl_sync(0xffffffffu, (goff[gi + 1] - o) >> 5, 0);
+    const Out r = run_sum<MODE>(em, src + (o - src0) + lane, L);
+    // a partial takes an 8-byte slot in every precision
+    Out* at = out.x >= 0 ? values + out.x
+                         : reinterpret_cast<Out*>(static_cast<double*>(bm.partial) + (-1 - (int64_t)out.x));
+    if (out.x != kNoOutput) *at = r;
+    if (out.x >= 0 && out.y != out.x) values[out.y] = r;
+  }
+}
+template <int MODE, int THREADS>
+__device__ __forceinline__ void block_sums(const BlockArgs& bm, int32_t g0, int32_t g1, int32_t src0, int32_t src1,
+                                           const uint16_t* s_src, const int2* s_out, const int32_t* s_goff,
+                                           const unsigned char* em, typename Arith<MODE>::Out* __restrict__ values)
+{
+  if (src1 - src0 <= kStageSrc && g1 - g0 <= kStageGroups)
+    block_sums_from<MODE, THREADS>(bm, g0, g1, src0, s_src, s_out, s_goff, em, values);
+  else
+    block_sums_from<MODE, THREADS>(bm, g0, g1, 0, bm.bsrc, bm.bout + 32 * (int64_t)g0, bm.bgoff + g0, em, values);
+}
+
+// P1: one CTA per block of kElemBlock elements.  Double-word and FP32: 256 threads,
+// two elements each as packed pairs; native FP64: 512 threads, one element each.
+// SPLIT: the node records are split on grids (edges_dw; FP32 reads either form).
+template <int MODE> constexpr int kBlockThreads = MODE == kF64 ? 512 : 256;
+template <int MODE, bool SPLIT>
+__global__ void __launch_bounds__(kBlockThreads<MODE>, MODE == kF32 ? 4 : (MODE == kDW ? 3 : 2))
     k_block_asm(ElemArgs a, BlockArgs bm, typename Arith<MODE>::Out* __restrict__ values)
 {
   using A = Arith<MODE>;
   using T = typename A::T;
-  constexpr int NU = 10;
+  constexpr int NU = 10, THREADS = kBlockThreads<MODE>;
   extern __shared__ __align__(16) unsigned char smem[];
-  T* em = reinterpret_cast<T*>(smem);  // the block's element matrices, then a zero (padding source)
-  uint16_t* s_src = reinterpret_cast<uint16_t*>(smem + block_em_bytes<T, kElemBlock, NU>());
-  int32_t* s_goff = reinterpret_cast<int32_t*>(s_src + kStageSrc);
-  __shared__ T tab[7 * NU];
-  const int32_t g0 = bm.bgrp[blockIdx.x], g1 = bm.bgrp[blockIdx.x + 1];
-  const int32_t src0 = bm.bsrc0[blockIdx.x], src1 = bm.bsrc0[blockIdx.x + 1];
-  stage_block_map<THREADS>(bm, g0, g1, src0, src1, s_src, s_goff);
+  uint16_t* s_src = reinterpret_cast<uint16_t*>(smem + kEmBytes<MODE>);
+  int2* s_out = reinterpret_cast<int2*>(s_src + kStageSrc);
+  float4* s_a = reinterpret_cast<float4*>(s_out + 32 * kStageGroups);
+  float4* s_b = s_a + kStageNodes;
+  float* s_z = reinterpret_cast<float*>(s_b + kStageNodes);
+  int32_t* s_id = reinterpret_cast<int32_t*>(s_z + kStageNodes);
+  int32_t* s_goff = MODE == kF64 ? reinterpret_cast<int32_t*>(s_a) : s_id + kStageNodes;
+  __shared__ T mass[NU];
+  pdl_trigger();
   const int64_t p0 = (int64_t)blockIdx.x * kElemBlock;
   const int64_t E = a.n_elem;
-  for (int i = threadIdx.x; i < 7 * NU; i += THREADS) tab[i] = A::from(a.tables[i]);
-  if (threadIdx.x == 0) em[kElemBlock * NU] = A::zero();
-  __syncthreads();
-#pragma unroll 1
-  for (int i = 0; i < kElemBlock / THREADS; ++i) {
-    const int lp = i * THREADS + threadIdx.x;
+  if constexpr (MODE == kF64) {
+    const int32_t g0 = bm.bgrp[blockIdx.x], g1 = bm.bgrp[blockIdx.x + 1];
+    const int32_t src0 = bm.bsrc0[blockIdx.x], src1 = bm.bsrc0[blockIdx.x + 1];
+    stage_block_map<THREADS>(bm, g0, g1, src0, src1, s_src, s_out, s_goff);
+    pdl_wait();
+    double* em = reinterpret_cast<double*>(smem);
+    if (threadIdx.x < NU) mass[threadIdx.x] = a.tables[6 * NU + threadIdx.x];
+    if (threadIdx.x == 0) em[NU * kElemBlock] = 0.0;
+    __syncthreads();
+    const int lp = threadIdx.x;
     if (p0 + lp < E) {
-      T K[NU];
-      p1_element<MODE>(a, tab, elem_nodes(a, p0 + lp), elem_coef(a, p0 + lp), K);
+      double K[NU];
+      p1_element_f64(a, mass, elem_nodes(a, p0 + lp), elem_coef(a, p0 + lp), K);
 #pragma unroll
-      for (int u = 0; u < NU; ++u) em[lp * NU + u] = K[u];
+      for (int u = 0; u < NU; ++u) em[u * kElemBlock + lp] = K[u];
     }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    block_sums<MODE, THREADS>(bm, g0, g1, src0, src1, s_src, s_out, s_goff, smem, values);
+  } else {
+    // asynchronous copies in the order of need: the records of the block's unique
+    // nodes, the pair's coefficients, the block map.  A warp's coefficient slots lie in
+    // the shared rows that only its own elements' entries overwrite.
+    float* em = reinterpret_cast<float*>(smem);
+    const int lane = threadIdx.x & 31, lp = threadIdx.x + (threadIdx.x & ~31);
+    // past the last element the pair repeats it (no source refers to the copies)
+    const int64_t p1 = min(p0 + lp, E - 1), p2 = min(p0 + lp + 32, E - 1);
+    const int32_t id = bm.bnode[(int64_t)blockIdx.x * kStageNodes + threadIdx.x];
+    const int64_t e1 = a.elem_order[p1], e2 = a.elem_order[p2];
+    const bool staged = bm.bnode_n[blockIdx.x] >= 0;
+    const int32_t g0 = bm.bgrp[blockIdx.x], g1 = bm.bgrp[blockIdx.x + 1];
+    const int32_t src0 = bm.bsrc0[blockIdx.x], src1 = bm.bsrc0[blockIdx.x + 1];
+    cp_async16(s_a + threadIdx.x, a.geo.rec + 2 * (int64_t)id);
+    cp_async16(s_b + threadIdx.x, a.geo.rec + 2 * (int64_t)id + 1);
+    if (MODE == kDW) cp_async4(s_z + threadIdx.x, a.geo.loz + id);
+    s_id[threadIdx.x] = id;
+    asm volatile("cp.async.commit_group;\n" ::);
+    // up to here only the plan was read; the coefficients, the partial sums and the
+    // values belong to the kernels before this one until they are complete
+    pdl_wait();
+    double* slot1 = reinterpret_cast<double*>(em + (lane >> 4) * kElemBlock + (lp - lane) + 4 * (lane & 15));
+    double* slot2 = slot1 + kElemBlock;  // two rows on
+    if (a.coeff) {
+      coef_fetch(slot1, a.coeff, e1, E);
+      coef_fetch(slot2, a.coeff, e2, E);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+    stage_block_map<THREADS>(bm, g0, g1, src0, src1, s_src, s_out, s_goff);
+    if (threadIdx.x < (MODE == kDW ? 2 : 1)) em[threadIdx.x * kEmStride + NU * kElemBlock] = 0.0f;
+    if (!a.stiff && threadIdx.x < NU) mass[threadIdx.x] = A::from(a.tables[6 * NU + threadIdx.x]);
+    typename Pair<MODE>::T J[3][3];
+    int4 n0, n1;
+    if (staged) {
+      const uchar4 l0 = __ldg(bm.elem_local + p1), l1 = __ldg(bm.elem_local + p2);
+      n0 = make_int4(l0.x, l0.y, l0.z, l0.w);
+      n1 = make_int4(l1.x, l1.y, l1.z, l1.w);
+      asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+      __syncthreads();
+      pair_edges<SPLIT>(StagedNodes{s_a, s_b, s_z}, n0, n1, J);
+    } else {
+      n0 = elem_nodes(a, p1);
+      n1 = elem_nodes(a, p2);
+      __syncthreads();  // mass
+      pair_edges<SPLIT>(GlobalNodes{a.geo}, n0, n1, J);
+    }
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    const double c0 = a.coeff ? coef_slot(slot1, a.coeff, e1) : a.cconst;
+    const double c1 = a.coeff ? coef_slot(slot2, a.coeff, e2) : a.cconst;
+    __syncwarp();  // before the entries overwrite the slots
+    const auto node = [&](int e) {
+      const int4 n = e ? n1 : n0;
+      return staged ? make_int4(s_id[n.x], s_id[n.y], s_id[n.z], s_id[n.w]) : n;
+    };
+    if constexpr (MODE == kDW) p1_pair_dw(a, mass, J, node, c0, c1, lp, em, em + kEmStride);
+    else p1_pair_f32(a, mass, J, node, c0, c1, lp, em);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    block_sums<MODE, THREADS>(bm, g0, g1, src0, src1, s_src, s_out, s_goff, smem, values);
   }
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  __syncthreads();
-  block_sums<MODE, THREADS>(bm, g0, g1, src0, s_src, s_goff, em, values);
 }
 
-template <int MODE>
+template <typename V>
 __global__ void __launch_bounds__(256) k_shared_sum(int64_t n_groups, const int32_t* __restrict__ sgoff,
-                                                    const int2* __restrict__ sout, const void* __restrict__ partial,
-                                                    typename Arith<MODE>::Out* __restrict__ values)
+                                                    const int2* __restrict__ sout, const double* partial, V* values)
 {
-  using A = Arith<MODE>;
-  using T = typename A::T;
+  pdl_trigger();
   const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (g >= n_groups) return;
+  const bool live = g < n_groups;
   const int lane = threadIdx.x & 31;
-  const int2 out = sout[32 * g + lane];
-  const int32_t o = sgoff[g], L = (sgoff[g + 1] - o) >> 5;
-  T v = A::zero();
+  const int2 out = live ? sout[32 * g + lane] : make_int2(kNoOutput, 0);
+  const int32_t o = live ? sgoff[g] : 0, L = live ? (sgoff[g + 1] - o) >> 5 : 0;
+  pdl_wait();  // every CTA waits, so that this kernel's end implies the one before's
+  V v = V(0);
   // 8 partials in flight, summed in ascending j
   for (int32_t j = 0; j < L; j += 8) {
-    T x[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = j + i < L ? partial_get<T>(partial, o + 32 * (j + i) + lane) : A::zero();
+    V x[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      if (j + i < L) A::sum_into(v, x[i]);
+      x[i] = j + i < L ? *reinterpret_cast<const V*>(partial + o + 32 * (j + i) + lane) : V(0);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v += x[i];
   }
   if (out.x >= 0) {
-    const typename A::Out r = A::out(v);
-    values[out.x] = r;
-    if (out.y != out.x) values[out.y] = r;
+    values[out.x] = v;
+    if (out.y != out.x) values[out.y] = v;
   }
 }
 
@@ -1012,24 +1381,23 @@ static mg_status allow_smem(K kernel, size_t bytes, std::once_flag (&once)[64])
   return MG_OK;
 }
 
-template <int MODE>
+template <int MODE, bool SPLIT>
 static mg_status launch_block_t(mg_plan* p, const ElemArgs& a, void* d_values, cudaStream_t st)
 {
   using Out = typename Arith<MODE>::Out;
-  using T = typename Arith<MODE>::T;
-  const BlockArgs bm{p->d_bgrp, p->d_bsrc0, p->d_bgoff, p->d_bsrc, p->d_bout, p->d_partial};
+  const BlockArgs bm{p->d_bgrp,    p->d_bsrc0, p->d_bgoff,   p->d_bsrc,      p->d_bout,
+                     p->d_partial, p->d_bnode, p->d_bnode_n, p->d_elem_local};
   static std::once_flag once[64];
   if (a.n_elem > 0) {
-    constexpr size_t smem = block_smem_bytes<T, kElemBlock, 10>();
-    constexpr int threads = MODE == kF32 ? 256 : 512;
-    MG_TRY(allow_smem(k_block_asm<MODE, threads>, smem, once));
-    k_block_asm<MODE, threads><<<(unsigned)p->n_blocks, threads, smem, st>>>(a, bm, static_cast<Out*>(d_values));
+    constexpr size_t smem = block_smem_bytes<MODE>();
+    MG_TRY(allow_smem(k_block_asm<MODE, SPLIT>, smem, once));
+    MG_CUDA(launch_smem(true, k_block_asm<MODE, SPLIT>, (int)p->n_blocks, kBlockThreads<MODE>, smem, st, a, bm,
+                        static_cast<Out*>(d_values)));
   }
-  MG_CUDA(cudaGetLastError());
   if (p->n_sgroups > 0)
-    k_shared_sum<MODE><<<(unsigned)((p->n_sgroups + 7) / 8), 256, 0, st>>>(p->n_sgroups, p->d_sgoff, p->d_sout,
-                                                                         p->d_partial, static_cast<Out*>(d_values));
-  MG_CUDA(cudaGetLastError());
+    MG_CUDA(launch_pdl(k_shared_sum<Out>, (int)((p->n_sgroups + 7) / 8), 256, st, p->n_sgroups,
+                       (const int32_t*)p->d_sgoff, (const int2*)p->d_sout, (const double*)p->d_partial,
+                       static_cast<Out*>(d_values)));
   return MG_OK;
 }
 
@@ -1082,12 +1450,15 @@ static mg_status launch_assemble_gather(mg_plan* p, int op, const double* d_coef
   a.cconst = op == MG_OP_STIFF_CONST ? c : 1.0;
   a.tables = d_tab;
   a.wsum = t->wsum;
+  a.w_hi = (float)t->wsum;
+  a.w_lo = (float)(t->wsum - (double)a.w_hi);
   a.stiff = (op == MG_OP_STIFF_KAPPA || op == MG_OP_STIFF_CONST);
   a.em = p->d_em;
   a.flags = p->d_counters + 4;
   if (uses_block_map(m->order)) {
-    if (prec == MG_F32) return launch_block_t<kF32>(p, a, d_values, st);
-    return prec == MG_F64_NATIVE ? launch_block_t<kF64>(p, a, d_values, st) : launch_block_t<kDW>(p, a, d_values, st);
+    if (prec == MG_F32) return launch_block_t<kF32, false>(p, a, d_values, st);
+    if (prec == MG_F64_NATIVE) return launch_block_t<kF64, false>(p, a, d_values, st);
+    return m->grid_split ? launch_block_t<kDW, true>(p, a, d_values, st) : launch_block_t<kDW, false>(p, a, d_values, st);
   }
   if (prec == MG_F32) return launch_gather_t<kF32>(p, a, d_values, st);
   return prec == MG_F64_NATIVE ? launch_gather_t<kF64>(p, a, d_values, st) : launch_gather_t<kDW>(p, a, d_values, st);

@@ -84,8 +84,12 @@ struct mg_mesh {
   std::vector<int32_t> tri_geo;     //   and their geoIds (2nd tag)
   // device copies
   double4_32a* d_xyz = nullptr;      // (x, y, z, 0)
-  // x = hi + mid + lo exactly (three floats per coordinate), packed so that
-  // one 32-byte sector holds a node's (hi.xyz, mid.xyz, lo.x, lo.y); lo.z apart
+  // x = hi + mid + lo (three floats per coordinate), packed so that one 32-byte
+  // sector holds a node's (hi.xyz, mid.xyz, lo.x, lo.y); lo.z apart.  grid_split:
+  // hi and mid are multiples of per-axis units, so that differences of the hi and
+  // of the mid parts are exact (build_node_records); else each part is the
+  // remainder rounded to a float, and the sum is exact
+  bool grid_split = false;
   float4* d_node_rec = nullptr;  // 2 float4 per node
   float* d_lo_z = nullptr;
   int4* d_conn = nullptr;        // vertex node ids
@@ -132,8 +136,15 @@ struct mg_plan {
   int32_t* d_bgrp = nullptr;        // n_blocks + 1
   int32_t* d_bsrc0 = nullptr;       // n_blocks + 1: bgoff[bgrp[b]] (block b's first local source)
   int32_t* d_bgoff = nullptr;       // n_bgroups + 1
-  uint16_t* d_bsrc = nullptr;       // n_bsrc
+  uint16_t* d_bsrc = nullptr;       // n_bsrc (on the device: byte offsets 4 (u kElemBlock + local element))
   int2* d_bout = nullptr;           // 32 n_bgroups
+  // the blocks' unique nodes (build_block_nodes): block b's at bnode[b kStageNodes],
+  // ascending, bnode_n[b] of them and the last one repeated (-1: more than
+  // kStageNodes, its first nodes only), and per Morton position the places of its four
+  // vertices among them
+  int32_t* d_bnode = nullptr;
+  int32_t* d_bnode_n = nullptr;     // n_blocks
+  uchar4* d_elem_local = nullptr;   // n_elem
   int32_t* d_sgoff = nullptr;       // n_sgroups + 1
   int2* d_sout = nullptr;           // 32 n_sgroups
   void* d_partial = nullptr;        // n_partial slots of 8 bytes (zero at padding)
@@ -251,6 +262,9 @@ constexpr int kGatherRowBlock = 256;
 // the one-pass P1 assembly: elements per block (one CTA) and the empty-lane
 // output of its block map
 constexpr int kElemBlock = 512;
+// nodes of a block staged in shared memory by the element kernels (8-bit local
+// vertex numbers); a block of 512 elements of a volume mesh has 150 to 200
+constexpr int kStageNodes = 256;
 inline int elems_per_block(int) { return kElemBlock; }
 constexpr int32_t kNoOutput = INT32_MIN;
 // the assembly of an element order runs through the block map (one pass, P1)
@@ -262,7 +276,11 @@ inline bool uses_block_map(int order) { return order == 1; }
 // p nu + u, ascending p): see mg_plan::d_bgrp
 mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int32_t* uslot, const int32_t* umirror,
                           const uint32_t* src, cudaStream_t st);
+mg_status build_block_nodes(mg_plan* p, cudaStream_t st);     // the blocks' unique nodes
 mg_status build_edges_device(mg_mesh* m, cudaStream_t st);    // edges on the GPU (mg_pattern.cu)
+// the device coordinates and node records (d_xyz, d_node_rec, d_lo_z, grid_split)
+// from the host coordinates; needs d_conn (mg_pattern.cu)
+mg_status build_node_records(mg_mesh* m);
 mg_status ensure_edges(mg_mesh* m);
 mg_status launch_assemble(mg_plan* p, int op, const double* d_coeff, double c, int quad, int prec,
                           void* d_values, cudaStream_t st);

@@ -272,37 +272,17 @@ mg_status mesh_device(mg_mesh* m)
   if (m->on_device) return check_device(m->device, "the mesh");
   MG_CUDA(cudaGetDevice(&m->device));
   const int64_t N = m->n_nodes, E = m->n_elem;
-  std::vector<double4_32a> x64(N);
-  std::vector<float4> rec(2 * N);
-  std::vector<float> loz(N);
-#pragma omp parallel for
-  for (int64_t i = 0; i < N; ++i) {
-    double c[3] = {m->xyz[3 * i], m->xyz[3 * i + 1], m->xyz[3 * i + 2]};
-    float h[3], md[3], l[3];
-    for (int k = 0; k < 3; ++k) {  // each remainder is exact in double
-      h[k] = (float)c[k];
-      const double r1 = c[k] - (double)h[k];
-      md[k] = (float)r1;
-      l[k] = (float)(r1 - (double)md[k]);
-    }
-    x64[i] = make_double4_32a(c[0], c[1], c[2], 0.0);
-    rec[2 * i] = make_float4(h[0], h[1], h[2], md[0]);
-    rec[2 * i + 1] = make_float4(md[1], md[2], l[0], l[1]);
-    loz[i] = l[2];
-  }
   MG_CUDA(cudaMalloc(&m->d_xyz, sizeof(double4_32a) * std::max<int64_t>(N, 1)));
   MG_CUDA(cudaMalloc(&m->d_node_rec, 2 * sizeof(float4) * std::max<int64_t>(N, 1)));
   MG_CUDA(cudaMalloc(&m->d_lo_z, sizeof(float) * std::max<int64_t>(N, 1)));
   MG_CUDA(cudaMalloc(&m->d_conn, sizeof(int4) * std::max<int64_t>(E, 1)));
   MG_CUDA(cudaMalloc(&m->d_dofs, sizeof(int32_t) * std::max<int64_t>(E * m->nb, 1)));
-  MG_CUDA(cudaMemcpy(m->d_xyz, x64.data(), sizeof(double4_32a) * N, cudaMemcpyHostToDevice));
-  MG_CUDA(cudaMemcpy(m->d_node_rec, rec.data(), 2 * sizeof(float4) * N, cudaMemcpyHostToDevice));
-  MG_CUDA(cudaMemcpy(m->d_lo_z, loz.data(), sizeof(float) * N, cudaMemcpyHostToDevice));
   MG_CUDA(cudaMemcpy(m->d_conn, m->conn.data(), sizeof(int4) * E, cudaMemcpyHostToDevice));
   if (m->order == 1)  // P1 dofs = the connectivity, already on the device
     MG_CUDA(cudaMemcpy(m->d_dofs, m->d_conn, sizeof(int32_t) * E * 4, cudaMemcpyDeviceToDevice));
   else
     MG_CUDA(cudaMemcpy(m->d_dofs, m->dofs.data(), sizeof(int32_t) * E * m->nb, cudaMemcpyHostToDevice));
+  MG_TRY(build_node_records(m));
   m->on_device = true;
   return MG_OK;
 }

@@ -18,6 +18,8 @@
 // The pattern is copied to the host (the export calls and the boundary-multiplier
 // build read it there) and, for the device plan build, kept on the device.
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 #include <vector>
 
 #include <cub/cub.cuh>
@@ -25,6 +27,184 @@
 #include "mg_internal.h"
 
 namespace mg {
+
+// ------------------------------------------------------------ node records --
+// The device coordinates and the three-float node records x = hi + mid + lo.
+// Where the mesh allows, the parts are split on per-axis grids: with |x| <= 2^e on
+// the axis, hi is a multiple of 2^(e-23) and mid of 2^(e-47), so that the
+// differences of two nodes' hi and mid parts are exact floats, and lo carries the
+// rest to 2^(e-72).  An edge vector then keeps an absolute error of 2^(e-70), a
+// relative 2^-50 of every gradient as long as no element is thinner than 2^-20 of
+// the largest coordinate; thinner elements, and coordinates whose lower parts
+// would leave the normal floats, take the general split (each part the remainder
+// rounded to a float, exact), whose differences cost error-free sums.
+
+// stats: per axis the largest |x| (bits of a double), then the smallest altitude
+// over 2^emax (bits of a float)
+__global__ void __launch_bounds__(256) k_node_xyz(int64_t N, const double* __restrict__ raw, double4_32a* __restrict__ xyz,
+                                                  unsigned long long* __restrict__ stats)
+{
+  __shared__ unsigned long long mx[3];
+  if (threadIdx.x < 3) mx[threadIdx.x] = 0ull;
+  __syncthreads();
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < N) {
+    const double x = raw[3 * i], y = raw[3 * i + 1], z = raw[3 * i + 2];
+    xyz[i] = make_double4_32a(x, y, z, 0.0);
+    atomicMax(&mx[0], (unsigned long long)__double_as_longlong(fabs(x)));
+    atomicMax(&mx[1], (unsigned long long)__double_as_longlong(fabs(y)));
+    atomicMax(&mx[2], (unsigned long long)__double_as_longlong(fabs(z)));
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) atomicMax(&stats[threadIdx.x], mx[threadIdx.x]);
+}
+
+// e with 2^(e-1) <= |x| < 2^e from the bits of a normal double (-1074 for smaller)
+__host__ __device__ __forceinline__ int grid_exponent(unsigned long long bits)
+{
+  const int ex = (int)((bits >> 52) & 0x7ff);
+  return ex == 0 ? -1074 : ex - 1022;
+}
+
+// 2^k as a double, |k| <= 1022
+__host__ __device__ __forceinline__ double pow2(int k)
+{
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)(k + 1023) << 52);
+#else
+  return std::ldexp(1.0, k);
+#endif
+}
+
+// The smallest altitude det / |C_a| of the elements, in units of 2^emax: edge
+// differences in FP64, the rest in FP32 (only its size against 2^-20 matters).
+__global__ void __launch_bounds__(256) k_min_altitude(int64_t E, const int4* __restrict__ conn,
+                                                      const double4_32a* __restrict__ xyz, double scale,
+                                                      uint32_t* __restrict__ min_alt)
+{
+  __shared__ uint32_t mn;
+  if (threadIdx.x == 0) mn = 0x7f800000u;
+  __syncthreads();
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e < E) {
+    const int4 n = conn[e];
+    const double4_32a p = xyz[n.x], q[3] = {xyz[n.y], xyz[n.z], xyz[n.w]};
+    float d[3][3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      d[k][0] = (float)((q[k].x - p.x) * scale);
+      d[k][1] = (float)((q[k].y - p.y) * scale);
+      d[k][2] = (float)((q[k].z - p.z) * scale);
+    }
+    float c[4][3], big = 0.0f;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) c[3][r] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float *a = d[(k + 1) % 3], *b = d[(k + 2) % 3];
+      c[k][0] = a[1] * b[2] - a[2] * b[1];
+      c[k][1] = a[2] * b[0] - a[0] * b[2];
+      c[k][2] = a[0] * b[1] - a[1] * b[0];
+#pragma unroll
+      for (int r = 0; r < 3; ++r) c[3][r] -= c[k][r];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) big = fmaxf(big, c[k][0] * c[k][0] + c[k][1] * c[k][1] + c[k][2] * c[k][2]);
+    const float det = d[0][0] * c[0][0] + d[0][1] * c[0][1] + d[0][2] * c[0][2];
+    const float alt = fabsf(det) * rsqrtf(big);
+    atomicMin(&mn, alt > 0.0f ? __float_as_uint(alt) : 0u);  // NaN counts as zero
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMin(min_alt, mn);
+}
+
+struct SplitGrid {
+  int on;
+  int e[3];  // per axis
+};
+
+__device__ __forceinline__ void split3(double x, const SplitGrid& g, int k, float& h, float& m, float& l)
+{
+  if (g.on) {
+    const double hd = rint(x * pow2(23 - g.e[k])) * pow2(g.e[k] - 23);
+    const double r1 = x - hd;
+    const double md = rint(r1 * pow2(47 - g.e[k])) * pow2(g.e[k] - 47);
+    h = (float)hd;
+    m = (float)md;
+    l = (float)(r1 - md);
+  } else {  // each remainder is exact in double
+    h = (float)x;
+    const double r1 = x - (double)h;
+    m = (float)r1;
+    l = (float)(r1 - (double)m);
+  }
+}
+
+__global__ void __launch_bounds__(256) k_node_split(int64_t N, const double4_32a* __restrict__ xyz, SplitGrid g,
+                                                    float4* __restrict__ rec, float* __restrict__ loz)
+{
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const double4_32a p = xyz[i];
+  float h[3], m[3], l[3];
+  split3(p.x, g, 0, h[0], m[0], l[0]);
+  split3(p.y, g, 1, h[1], m[1], l[1]);
+  split3(p.z, g, 2, h[2], m[2], l[2]);
+  rec[2 * i] = make_float4(h[0], h[1], h[2], m[0]);
+  rec[2 * i + 1] = make_float4(m[1], m[2], l[0], l[1]);
+  loz[i] = l[2];
+}
+
+mg_status build_node_records(mg_mesh* m)
+{
+  const int64_t N = m->n_nodes, E = m->n_elem;
+  m->grid_split = false;
+  if (N == 0) return MG_OK;
+  double* raw = nullptr;
+  MG_CUDA(cudaMalloc(&raw, sizeof(double) * (3 * N + 4)));
+  unsigned long long* stats = reinterpret_cast<unsigned long long*>(raw + 3 * N);
+  uint32_t* min_alt = reinterpret_cast<uint32_t*>(stats + 3);
+  const cudaStream_t st = cudaStreamLegacy;
+  const uint32_t inf = 0x7f800000u;
+  unsigned long long h[3] = {0, 0, 0};
+  uint32_t halt = 0;
+  SplitGrid g{};
+  const unsigned nb = (unsigned)((N + 255) / 256), eb = (unsigned)((E + 255) / 256);
+  cudaError_t e = cudaMemcpyAsync(raw, m->xyz.data(), sizeof(double) * 3 * N, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(stats, 0, 4 * sizeof(double), st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(min_alt, &inf, sizeof(inf), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) {
+    k_node_xyz<<<nb, 256, 0, st>>>(N, raw, m->d_xyz, stats);
+    e = cudaMemcpyAsync(h, stats, sizeof(h), cudaMemcpyDeviceToHost, st);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) {
+    int emax = -1074;
+    bool fits = true;
+    for (int k = 0; k < 3; ++k) {
+      g.e[k] = grid_exponent(h[k]);
+      emax = std::max(emax, g.e[k]);
+      if (g.e[k] < -50 || g.e[k] > 100) fits = false;
+    }
+    if (fits && eb > 0) {
+      k_min_altitude<<<eb, 256, 0, st>>>(E, m->d_conn, m->d_xyz, pow2(-emax), min_alt);
+      e = cudaMemcpyAsync(&halt, min_alt, sizeof(halt), cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+      float alt;
+      std::memcpy(&alt, &halt, sizeof(alt));
+      g.on = alt >= 0x1p-20f;
+    }
+  }
+  if (e == cudaSuccess) {
+    k_node_split<<<nb, 256, 0, st>>>(N, m->d_xyz, g, m->d_node_rec, m->d_lo_z);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  }
+  cudaFree(raw);
+  if (e != cudaSuccess) return cuda_error(e, "node records");
+  m->grid_split = g.on != 0;
+  return MG_OK;
+}
 
 // one thread per (element, test basis j): the element's nb couplings of row dofs[j]
 __global__ void __launch_bounds__(256) k_pattern_keys(int64_t n_elem, int nb, const int32_t* __restrict__ dofs,

@@ -210,6 +210,9 @@ static void free_plan(mg_plan* p)
   cudaFree(p->d_bgoff);
   cudaFree(p->d_bsrc);
   cudaFree(p->d_bout);
+  cudaFree(p->d_bnode);
+  cudaFree(p->d_bnode_n);
+  cudaFree(p->d_elem_local);
   cudaFree(p->d_sgoff);
   cudaFree(p->d_sout);
   cudaFree(p->d_partial);
@@ -464,7 +467,16 @@ mg_status mg_plan_export_block_map(mg_plan* p, int32_t* h_elem_order, int32_t* h
   if (h_bgrp) MG_CUDA(cudaMemcpy(h_bgrp, p->d_bgrp, sizeof(int32_t) * (p->n_blocks + 1), cudaMemcpyDeviceToHost));
   if (h_goff) MG_CUDA(cudaMemcpy(h_goff, p->d_bgoff, sizeof(int32_t) * (G + 1), cudaMemcpyDeviceToHost));
   if (h_src && p->n_bsrc)
+  {
     MG_CUDA(cudaMemcpy(h_src, p->d_bsrc, sizeof(uint16_t) * p->n_bsrc, cudaMemcpyDeviceToHost));
+    // the kernels' byte offsets (4 per entry, entry-major) as element * nunique + entry
+    const int nu = nunique(p->mesh->order), be = kElemBlock;
+#pragma omp parallel for
+    for (int64_t i = 0; i < p->n_bsrc; ++i) {
+      const int s = h_src[i] / 4;
+      h_src[i] = (uint16_t)(s < nu * be ? (s % be) * nu + s / be : s);
+    }
+  }
   if (h_out && G) MG_CUDA(cudaMemcpy(h_out, p->d_bout, sizeof(int2) * 32 * G, cudaMemcpyDeviceToHost));
   if (h_sgoff) MG_CUDA(cudaMemcpy(h_sgoff, p->d_sgoff, sizeof(int32_t) * (G3 + 1), cudaMemcpyDeviceToHost));
   if (h_sout && G3) MG_CUDA(cudaMemcpy(h_sout, p->d_sout, sizeof(int2) * 32 * G3, cudaMemcpyDeviceToHost));

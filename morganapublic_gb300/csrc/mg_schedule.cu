@@ -464,7 +464,8 @@ __global__ void k_sgroup_out(int64_t G3, int64_t S, const int32_t* __restrict__ 
   sout[i] = i < S ? make_int2(uslot[sh_t[i]], umirror[sh_t[i]]) : make_int2(kNoOutput, kNoOutput);
 }
 
-// one thread per (group, lane): the run's local sources [j][lane] and its output
+// one thread per (group, lane): the run's local sources [j][lane], stored as the
+// kernels' byte offset 4 (u be + l) of entry u of local element l, and its output
 __global__ void k_bfill(int64_t G, int nu, int be, const int32_t* __restrict__ grun0, const int32_t* __restrict__ gcnt,
                         const uint32_t* __restrict__ perm, const uint32_t* __restrict__ skey,
                         const int32_t* __restrict__ rt, const int32_t* __restrict__ rj,
@@ -479,7 +480,7 @@ __global__ void k_bfill(int64_t G, int nu, int be, const int32_t* __restrict__ g
   const int64_t g = i >> 5;
   const int lane = (int)(i & 31);
   const int32_t o = bgoff[g], L = (bgoff[g + 1] - o) >> 5;
-  const uint16_t pad = (uint16_t)(be * nu);
+  const uint16_t pad = (uint16_t)(4 * be * nu);
   if (lane >= gcnt[g]) {
     bout[i] = make_int2(kNoOutput, 0);
     for (int32_t j = 0; j < L; ++j) bsrc[o + 32 * j + lane] = pad;
@@ -489,7 +490,10 @@ __global__ void k_bfill(int64_t G, int nu, int be, const int32_t* __restrict__ g
   const uint32_t ri = perm[sr];
   const uint32_t base = (skey[sr] >> 6) * (uint32_t)be * (uint32_t)nu;
   const int32_t t = rt[ri], k0 = rstart[ri], len = rlen[ri];
-  for (int32_t j = 0; j < L; ++j) bsrc[o + 32 * j + lane] = j < len ? (uint16_t)(src[k0 + j] - base) : pad;
+  for (int32_t j = 0; j < L; ++j) {
+    const uint32_t i0 = j < len ? src[k0 + j] - base : 0;
+    bsrc[o + 32 * j + lane] = j < len ? (uint16_t)(4 * ((i0 % (uint32_t)nu) * (uint32_t)be + i0 / (uint32_t)nu)) : pad;
+  }
   if (nrun[t] == 1) {
     bout[i] = make_int2(uslot[t], umirror[t]);
   } else {
@@ -615,6 +619,7 @@ mg_status build_slot_map(mg_plan* p, cudaStream_t st)
   if (hbad) return set_error(MG_ERR_INVALID_ARG, "slot map: an element coupling is missing from the plan's pattern");
   if (uses_block_map(m->order)) {
     // one-pass assembly: the per-entry lists become the block map
+    MG_TRY(build_block_nodes(p, st));
     MG_TRY(build_block_map(p, U, useg, uslot, umirror, src, st));
     p->n_upper = U;
     p->n_slot_contrib = C;
@@ -676,6 +681,83 @@ mg_status build_slot_map(mg_plan* p, cudaStream_t st)
 }
 
 
+// ----------------------------------------------------------- block nodes --
+// One CTA per block of kElemBlock elements: its 4 kElemBlock vertex ids sorted with
+// their positions, the first of each run an entry of the block's node list, and
+// the run's rank the local number of its vertices.
+__global__ void __launch_bounds__(256) k_block_nodes(int64_t E, const int32_t* __restrict__ dofs_m,
+                                                     int32_t* __restrict__ bnode, int32_t* __restrict__ bnode_n,
+                                                     uchar4* __restrict__ elem_local)
+{
+  constexpr int ITEMS = 4 * kElemBlock / 256;
+  using Sort = cub::BlockRadixSort<uint32_t, 256, ITEMS, uint16_t>;
+  using Scan = cub::BlockScan<int, 256>;
+  __shared__ union {
+    typename Sort::TempStorage sort;
+    typename Scan::TempStorage scan;
+    uint8_t local[4 * kElemBlock];
+  } sh;
+  __shared__ uint32_t last[256];
+  const int64_t q0 = (int64_t)blockIdx.x * 4 * kElemBlock;
+  const int t = threadIdx.x;
+  uint32_t key[ITEMS];
+  uint16_t pos[ITEMS];
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const int q = t * ITEMS + i;
+    key[i] = q0 + q < 4 * E ? (uint32_t)dofs_m[q0 + q] : 0xffffffffu;
+    pos[i] = (uint16_t)q;
+  }
+  Sort(sh.sort).Sort(key, pos);
+  last[t] = key[ITEMS - 1];
+  __syncthreads();
+  int head[ITEMS], rank[ITEMS], total = 0;
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const bool first = i == 0 && t == 0;
+    const uint32_t prev = i > 0 ? key[i > 0 ? i - 1 : 0] : (t > 0 ? last[t > 0 ? t - 1 : 0] : 0u);
+    head[i] = key[i] != 0xffffffffu && (first || prev != key[i]) ? 1 : 0;
+  }
+  Scan(sh.scan).InclusiveSum(head, rank, total);
+  __syncthreads();
+  const bool fits = total <= kStageNodes;
+  if (t == 0) bnode_n[blockIdx.x] = fits ? total : -1;
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    if (head[i] && rank[i] <= kStageNodes) {
+      int32_t* out = bnode + (int64_t)blockIdx.x * kStageNodes;
+      out[rank[i] - 1] = (int32_t)key[i];
+      if (rank[i] == total)  // the last one fills the list, so every slot names a node
+        for (int k = total; k < kStageNodes; ++k) out[k] = (int32_t)key[i];
+    }
+    sh.local[pos[i]] = (uint8_t)(fits ? rank[i] - 1 : 0);
+  }
+  __syncthreads();
+  for (int l = t; l < kElemBlock; l += 256) {
+    const int64_t p = (int64_t)blockIdx.x * kElemBlock + l;
+    if (p < E)
+      elem_local[p] = make_uchar4(sh.local[4 * l], sh.local[4 * l + 1], sh.local[4 * l + 2], sh.local[4 * l + 3]);
+  }
+}
+
+mg_status build_block_nodes(mg_plan* p, cudaStream_t st)
+{
+  const int64_t E = p->mesh->n_elem, nblk = std::max<int64_t>(1, (E + kElemBlock - 1) / kElemBlock);
+  SchedBuffers B;
+  int32_t *bnode, *bnode_n;
+  uchar4* local;
+  MG_TRY(B.alloc(&bnode, nblk * kStageNodes));
+  MG_TRY(B.alloc(&bnode_n, nblk));
+  MG_TRY(B.alloc(&local, E));
+  k_block_nodes<<<(unsigned)nblk, 256, 0, st>>>(E, p->d_dofs_morton, bnode, bnode_n, local);
+  MG_CUDA(cudaGetLastError());
+  p->d_bnode = bnode;
+  p->d_bnode_n = bnode_n;
+  p->d_elem_local = local;
+  for (void* q : {(void*)bnode, (void*)bnode_n, (void*)local}) B.keep(q);
+  return MG_OK;
+}
+
 // ------------------------------------------------------------- block map --
 // The one-pass P1 assembly's layout (see mg_plan::d_bgrp) from the slot map's
 // per-entry source lists (p nu + u, ascending p):
@@ -692,7 +774,7 @@ mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int3
                           const uint32_t* src, cudaStream_t st)
 {
   const int nu = nunique(p->mesh->order), be = elems_per_block(p->mesh->order);
-  if (be * nu >= UINT16_MAX) return set_error(MG_ERR_SIZE, "block map: a block's entries above 16 bits");
+  if (4 * be * nu >= UINT16_MAX) return set_error(MG_ERR_SIZE, "block map: a block's entries above 16 bits");
   const int64_t E = p->mesh->n_elem;
   const int64_t nblk = std::max<int64_t>(1, (E + be - 1) / be);
   const int64_t nseg = nblk;

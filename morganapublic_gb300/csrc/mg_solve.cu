@@ -33,39 +33,12 @@
 
 #include "mg_ff.cuh"
 #include "mg_internal.h"
+#include "mg_launch.cuh"
 
 namespace mg {
 
 constexpr int kSolveThreads = 256;
 constexpr int kMaxSolveBlocks = 2048;  // bound of the per-CTA partial arrays
-
-// Programmatic dependent launch: wait for the preceding kernel's memory (a no-op
-// when there is no programmatic dependency), and let the next kernel be
-// scheduled once every CTA of this one has started.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_k(bool pdl, void (*kernel)(KArgs...), int grid, int block, cudaStream_t st,
-                            Args&&... args)
-{
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t st, Args&&... args)
-{
-  return launch_k(true, kernel, grid, block, st, std::forward<Args>(args)...);
-}
 
 struct CgScalars {
   double rz, alpha, beta, rr, bb, tol2, pq, rz_prev;
