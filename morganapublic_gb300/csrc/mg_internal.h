@@ -66,6 +66,13 @@ int quad_rule(int quad, std::vector<double>* Y, std::vector<double>* W);
 void basis_values(int order, const double* Y, double* v);
 void basis_grads(int order, const double* Y, double* gx, double* gy, double* gz);
 
+// Row ranges of the resident CG's CTAs: CTA c owns the rows d_rows[c] .. d_rows[c + 1],
+// at most max_rows (ctas = 0: not built).
+struct RowPartition {
+  int32_t* d_rows = nullptr;
+  int ctas = 0, max_rows = 0;
+};
+
 }  // namespace mg
 
 // ---------------------------------------------------------------- handles --
@@ -168,6 +175,7 @@ struct mg_plan {
   void* d_work = nullptr;
   size_t work_bytes = 0;
   double* h_pinned = nullptr;  // small pinned scalars
+  mg::RowPartition cg_part[2];  // resident CG in FP64 and FP32 (built by the first solve)
   // temporary buffers of the host-buffer entry points
   void* d_tmp_values = nullptr;
   size_t tmp_values_bytes = 0;

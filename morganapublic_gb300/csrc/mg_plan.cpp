@@ -224,6 +224,7 @@ static void free_plan(mg_plan* p)
   cudaFree(p->d_counters);
   for (double* t : p->d_tables) cudaFree(t);
   cudaFree(p->d_work);
+  for (RowPartition& rp : p->cg_part) cudaFree(rp.d_rows);
   cudaFree(p->d_tmp_values);
   cudaFree(p->d_tmp_coeff);
   if (p->h_pinned) cudaFreeHost(p->h_pinned);
@@ -318,6 +319,7 @@ mg_status plan_work(mg_plan* p, size_t bytes, void** ptr)
 {
   if (p->work_bytes < bytes) {
     cudaFree(p->d_work);
+  for (RowPartition& rp : p->cg_part) cudaFree(rp.d_rows);
     p->d_work = nullptr;
     p->work_bytes = 0;
     MG_CUDA(cudaMalloc(&p->d_work, bytes));

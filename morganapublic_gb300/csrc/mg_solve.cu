@@ -28,6 +28,7 @@
 #include <cmath>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -445,6 +446,328 @@ __global__ void __launch_bounds__(kSolveThreads) k_cg_dir(int64_t n, const V* __
     p[i] = z[i] + beta * p[i];
 }
 
+// ------------------------------------------------------- resident CG --
+// The same iteration as K1..K3 in one cooperative kernel: each CTA (one per SM) owns a
+// range of rows and, where they are few enough, keeps their x, r, p, q and D^-1 in shared
+// memory, so an iteration streams the matrix and exchanges p.  The dot products go
+// through CTA 0: it adds the CTAs' partial sums in a fixed order and publishes the
+// total, so all take the same alpha, beta and stopping decision, and a solve is
+// bitwise reproducible.
+//
+// A value is published as two 64-bit words, each half of the double with the sum's
+// epoch: a word is current when its epoch is, with no fence and no reset.  Two
+// sets alternate: a CTA writes its words of the sum after next only when it has the
+// next one's total, which CTA 0 publishes after reading all partials of both.
+// Every wait is bounded (kSpinLimit polls): a CTA that gives up records done = 9
+// and returns, the others follow.
+//
+// What bounds it (GB300, P1 64^3, FP64): the FP64 pipe, 22 operations a row or 10 us of
+// an iteration, then the exchanges (~2 us each; every CTA polling every
+// other's partials or flags took 3 and 4 us: the polls queue at a few L2 lines).
+// K1..K3 took 39.6 us an iteration there and 24 us at any small size.
+template <typename V> constexpr int kResidentThreads = sizeof(V) == 8 ? 512 : 768;
+constexpr int kResidentIters = 512;  // iterations per launch (the host looks in between)
+constexpr int kSpinLimit = 1 << 21;
+constexpr int kMaxResidentCtas = 1024;
+
+// Exchange buffer: 2 sets of 4 words (2 values) per CTA, 2 sets of totals on a line of
+// their own, and the barrier's counter.
+struct GatherBuf {
+  unsigned long long* words;   // [set][cta][4]
+  unsigned long long* totals;  // [set][16]
+  unsigned int* count;
+};
+constexpr size_t kGatherBytes = sizeof(unsigned long long) * (8 * kMaxResidentCtas + 32) + 128;
+
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v)
+{
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ ulonglong2 ld_relaxed2(const unsigned long long* p)
+{
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void publish(unsigned long long* w, double v, unsigned int epoch)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v), e = (unsigned long long)epoch << 32;
+  st_relaxed(w, e | (b >> 32));
+  st_relaxed(w + 1, e | (b & 0xffffffffull));
+}
+// Waits for NV values published at w; false when the wait ran out.
+template <int NV>
+__device__ __forceinline__ bool receive(const unsigned long long* w, unsigned int epoch, double (&v)[NV])
+{
+  for (int spin = 0; spin < kSpinLimit; ++spin) {
+    ulonglong2 x[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) x[k] = ld_relaxed2(w + 2 * k);
+    bool current = true;
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      current = current && (unsigned int)(x[k].x >> 32) == epoch && (unsigned int)(x[k].y >> 32) == epoch;
+    if (current) {
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        v[k] = __longlong_as_double((long long)((x[k].x << 32) | (x[k].y & 0xffffffffull)));
+      return true;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = 0.0;
+  return false;
+}
+
+// Sum over all threads of all CTAs of NV values, the same in every thread (false
+// after a wait that ran out).  red: NV * blockDim.x + 8 values of shared memory; gat:
+// NV * gridDim.x + NV + 1 doubles; at least 128 threads.  Per CTA: the threads' values by
+// 128 threads in ascending stride, a shuffle tree, four warps' results in order; CTA 0's
+// thread c waits for CTA c's partials, its warp k adds the k-th ones in a fixed order.
+template <typename V, int NV>
+__device__ __forceinline__ bool grid_sum(const typename Dot<V>::A (&v)[NV], typename Dot<V>::A* red, double* gat,
+                                         const GatherBuf& gb, unsigned int epoch, double (&total)[NV])
+{
+  using D = Dot<V>;
+  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, C = gridDim.x;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) red[k * T + tid] = v[k];
+  __syncthreads();
+  if (tid < 128) {
+    typename D::A a[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      a[k] = red[k * T + tid];
+      for (int i = tid + 128; i < T; i += 128) a[k] = D::add(a[k], red[k * T + i]);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) a[k] = D::add(a[k], D::shfl(a[k], off));
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) red[NV * T + 4 * k + (tid >> 5)] = a[k];
+  }
+  __syncthreads();
+  unsigned long long* set = gb.words + (size_t)(epoch & 1u) * 4 * kMaxResidentCtas;
+  unsigned long long* result = gb.totals + (epoch & 1u) * 16;
+  if (tid < NV) {  // thread k publishes value k
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) s += D::to_double(red[NV * T + 4 * tid + w]);
+    publish(set + 4 * blockIdx.x + 2 * tid, s, epoch);
+  }
+  bool ok = true;
+  if (blockIdx.x == 0) {
+    for (int c = tid; c < C; c += T) {
+      double p[NV];
+      ok = receive<NV>(set + 4 * c, epoch, p) && ok;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) gat[k * C + c] = p[k];
+    }
+    ok = __syncthreads_and(ok) != 0;
+    if (tid < 32 * NV) {
+      const int k = tid >> 5;
+      double a = 0.0;
+      for (int c = lane; c < C; c += 32) a += gat[k * C + c];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+      if (lane == 0) {
+        gat[NV * C + k] = a;
+        if (ok) publish(result + 2 * k, a, epoch);
+      }
+    }
+  } else if (tid == 0) {
+    double p[NV];
+    ok = receive<NV>(result, epoch, p);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) gat[NV * C + k] = p[k];
+  }
+  ok = __syncthreads_and(ok) != 0;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) total[k] = gat[NV * C + k];
+  return ok;
+}
+
+// All CTAs' global writes before the barrier are seen by all CTAs' plain loads after it:
+// one thread's fence releases the CTA's writes, and after the wait drops its stale L1
+// lines.  `target`: the arrivals of all CTAs so far and at this barrier.
+__device__ __forceinline__ bool grid_barrier(const GatherBuf& gb, unsigned int target)
+{
+  __syncthreads();
+  bool ok = true;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(gb.count) : "memory");
+    int spin = 0;
+    for (; spin < kSpinLimit; ++spin) {
+      unsigned int f;
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(gb.count) : "memory");
+      if ((int)(f - target) >= 0) break;
+    }
+    ok = spin < kSpinLimit;
+    __threadfence();
+  }
+  return __syncthreads_and(ok) != 0;
+}
+
+// U entries of one lane of a group of G, and their products with p
+template <typename V, int G, int U, typename I>
+__device__ __forceinline__ void load_entries(const I* __restrict__ ci, const V* __restrict__ val, int row, int b0, int s1,
+                                             int (&c)[U], V (&v)[U])
+{
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int k = b0 + u * G;
+    c[u] = k < s1 ? column<I>(ci, k, row) : -1;
+    v[u] = k < s1 ? __ldg(val + k) : V(0);
+  }
+}
+template <typename V, int U>
+__device__ __forceinline__ void gather_entries(const V* p, const int (&c)[U], const V (&v)[U], V& sa, V& sb)
+{
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const V xv = c[u] >= 0 ? p[c[u]] : V(0);
+    // one chain in FP64: its pipe is busy with the other warps meanwhile, and a second
+    // accumulator costs an addition per row
+    if (sizeof(V) == 4 && (u & 1)) sb = fma(v[u], xv, sb);
+    else sa = fma(v[u], xv, sa);
+  }
+}
+
+// Up to `iters` iterations from the state of k_cg_start (or of an earlier launch).
+// p is read by plain loads (its values change within the kernel).
+template <typename V, int G, int U, typename I>
+__global__ void __launch_bounds__(kResidentThreads<V>, 1)
+    k_cg_resident(const int32_t* __restrict__ part, int max_rows, const int32_t* __restrict__ rp,
+                  const I* __restrict__ ci, const V* __restrict__ val, V* dinv, V* x, V* r, V* z, V* p, V* q_out,
+                  int in_smem, GatherBuf gb, unsigned int epoch, int iters, CgScalars* s)
+{
+  using D = Dot<V>;
+  extern __shared__ __align__(16) unsigned char smem[];
+  double* gat = reinterpret_cast<double*>(smem);
+  typename D::A* red = reinterpret_cast<typename D::A*>(gat + 2 * gridDim.x + 2);
+  int32_t* srp = reinterpret_cast<int32_t*>(red + 2 * blockDim.x + 8);  // the rows' starts
+  if (s->done) return;
+  const int r0 = part[blockIdx.x], rows = part[blockIdx.x + 1] - r0;
+  const int tid = threadIdx.x, T = blockDim.x;
+  // the rows' vectors: in shared memory, or where they are
+  V *sx = x + r0, *sr = r + r0, *sd = dinv + r0, *sp = p + r0, *sq = q_out + r0;
+  if (in_smem) {
+    V* v = reinterpret_cast<V*>(srp + (max_rows + 2) / 2 * 2);
+    sx = v, sr = v + max_rows, sd = v + 2 * max_rows, sp = v + 3 * max_rows, sq = v + 4 * max_rows;
+    for (int i = tid; i < rows; i += T) {
+      sx[i] = x[r0 + i];
+      sr[i] = r[r0 + i];
+      sp[i] = p[r0 + i];
+      sd[i] = dinv[r0 + i];
+    }
+  }
+  for (int i = tid; i <= rows; i += T) srp[i] = rp[r0 + i];
+  double rz = s->rz, rz_prev = s->rz_prev, rr = s->rr, beta = s->beta, alpha = s->alpha, pq = s->pq;
+  const double target = s->tol2 * s->bb, anchor = s->delta2 * s->rr_anchor;
+  const int maxit = s->maxit;
+  int iter = s->iter, done = 0;
+  unsigned int arrivals = 0;  // at the barriers so far (the counter starts at zero)
+  __syncthreads();
+  for (int it = 0; it < iters; ++it) {
+    // q = A p, p . q: the next row's first entries load while this row's gathers are
+    // in flight
+    typename D::A acc[1] = {D::zero()};
+    {
+      const int lane = tid & (G - 1), step = T / G;
+      int c[U];
+      V v[U];
+      int base = tid / G, s0 = 0, s1 = 0;
+      if (base < rows) {
+        s0 = srp[base] + lane, s1 = srp[base + 1];
+        load_entries<V, G, U, I>(ci, val, r0 + base, s0, s1, c, v);
+      }
+      while (base < rows) {
+        const int next = base + step;
+        int n0 = 0, n1 = 0;
+        int cn[U];
+        V vn[U];
+        if (next < rows) n0 = srp[next] + lane, n1 = srp[next + 1];
+        load_entries<V, G, U, I>(ci, val, r0 + next, n0, n1, cn, vn);
+        V sa = V(0), sb = V(0);
+        gather_entries<V, U>(p, c, v, sa, sb);
+        for (int b0 = s0 + G * U; b0 < s1; b0 += G * U) {
+          load_entries<V, G, U, I>(ci, val, r0 + base, b0, s1, c, v);
+          gather_entries<V, U>(p, c, v, sa, sb);
+        }
+        V q = sizeof(V) == 4 ? sa + sb : sa;
+#pragma unroll
+        for (int off = G / 2; off > 0; off >>= 1) q += __shfl_xor_sync(group_mask<G>(), q, off, G);
+        if (lane == 0) {
+          sq[base] = q;
+          D::mac(acc[0], sp[base], q);
+        }
+        base = next, s0 = n0, s1 = n1;
+#pragma unroll
+        for (int u = 0; u < U; ++u) c[u] = cn[u], v[u] = vn[u];
+      }
+    }
+    double tot[1];
+    if (!grid_sum<V, 1>(acc, red, gat, gb, ++epoch, tot)) { done = 9; break; }
+    pq = tot[0];
+    alpha = rz / pq;
+    if (!(pq > 0.0) || !isfinite(alpha)) { done = 2; break; }  // A not SPD on the Krylov space
+    // x += alpha p, r -= alpha q, z = D^-1 r, r . z, r . r
+    const V al = (V)alpha;
+    typename D::A acc2[2] = {D::zero(), D::zero()};
+    for (int i = tid; i < rows; i += T) {
+      sx[i] += al * sp[i];
+      const V ri = sr[i] - al * sq[i];
+      sr[i] = ri;
+      const V zi = sd[i] * ri;
+      sq[i] = zi;
+      D::mac(acc2[0], ri, zi);
+      D::mac(acc2[1], ri, ri);
+    }
+    double tot2[2];
+    if (!grid_sum<V, 2>(acc2, red, gat, gb, ++epoch, tot2)) { done = 9; break; }
+    rz_prev = rz;
+    beta = tot2[0] / rz;
+    rz = tot2[0];
+    rr = tot2[1];
+    ++iter;
+    if (rr <= target) done = 1;
+    else if (iter >= maxit) done = 3;
+    else if (rr <= anchor) done = 5;  // the host re-anchors, then forms the direction
+    if (done) break;
+    // p = z + beta p
+    const V be = (V)beta;
+    for (int i = tid; i < rows; i += T) {
+      const V pi = sq[i] + be * sp[i];
+      sp[i] = pi;
+      p[r0 + i] = pi;
+    }
+    if (!grid_barrier(gb, arrivals += gridDim.x)) { done = 9; break; }
+  }
+  for (int i = tid; i < rows; i += T) {
+    if (in_smem) {
+      x[r0 + i] = sx[i];
+      r[r0 + i] = sr[i];
+    }
+    z[r0 + i] = sd[i] * sr[i];
+  }
+  if (tid == 0 && (blockIdx.x == 0 || done == 9)) {
+    if (blockIdx.x == 0) {
+      s->rz = rz;
+      s->rz_prev = rz_prev;
+      s->rr = rr;
+      s->beta = beta;
+      s->alpha = alpha;
+      s->pq = pq;
+      s->iter = iter;
+    }
+    s->done = done;
+  }
+}
+
 // Start of a solve: r = b - A x (or r = b when x is zero), z = D^-1 r, p = z,
 // D^-1 from the diagonal, partials of r.z, r.r, b.b.
 template <typename V, int G>
@@ -673,13 +996,14 @@ struct CgWork {
   V *r, *z, *p, *q, *dinv;
   double* partials;  // 3 * kMaxSolveBlocks
   CgScalars* s;
+  GatherBuf gather;
 };
 
 template <typename V>
 static size_t cg_work_bytes(int64_t n)
 {
   const size_t vec = ((size_t)n * sizeof(V) + 255) / 256 * 256;
-  return 5 * vec + 3 * kMaxSolveBlocks * sizeof(double) + 256;
+  return 5 * vec + 3 * kMaxSolveBlocks * sizeof(double) + kGatherBytes + 256;
 }
 
 template <typename V>
@@ -692,6 +1016,10 @@ static CgWork<V> cg_work_carve(void* base, int64_t n)
   c += 256;
   w.partials = (double*)c;
   c += 3 * kMaxSolveBlocks * sizeof(double);
+  w.gather.words = (unsigned long long*)c;
+  w.gather.totals = w.gather.words + 8 * kMaxResidentCtas;
+  w.gather.count = (unsigned int*)(w.gather.totals + 32);
+  c += kGatherBytes;
   w.r = (V*)c; c += vec;
   w.z = (V*)c; c += vec;
   w.p = (V*)c; c += vec;
@@ -706,10 +1034,110 @@ constexpr double kMinAnchorRatio = 1e-3;
 // Iterations per replay of the captured CG graph between two host checks.
 constexpr int kGraphIters = 16;
 
+// Shape of the resident CG.  The vectors go to shared memory only while that leaves most
+// of the SM's 256 KB to L1, which the matrix stream and the gathers of p need (measured:
+// 213 KB of vectors at P2 48^3 left 15 KB of lines, 95 ms a solve).
+constexpr size_t kResidentVectors = 112 * 1024;
+// ... and only for systems that stay in L2: streaming from HBM one CTA per SM has too few
+// loads in flight (P2 48^3 in FP32, 222 MB: 103 us an iteration against 81 us with the
+// three kernels; P2 36^3, 94 MB: 44.2 against 45.3; P1 64^3 in FP64, 53 MB: 23.6 against 39.6).
+constexpr int64_t kResidentBytes = 100ll << 20;
+template <typename V>
+static size_t resident_smem(int ctas, int threads, int max_rows, bool vectors)
+{
+  return (2 * ctas + 2) * sizeof(double) + sizeof(typename Dot<V>::A) * (2 * threads + 8) +
+         sizeof(int32_t) * (size_t)((max_rows + 2) / 2 * 2) + (vectors ? 5 * sizeof(V) * (size_t)max_rows : 0);
+}
+// Threads per CTA: the passes over the rows evenly filled.
+template <typename V>
+static int resident_threads(int max_rows, int G)
+{
+  const int64_t units = (int64_t)max_rows * G, most = kResidentThreads<V>;
+  const int64_t passes = std::max<int64_t>(1, (units + most - 1) / most);
+  const int64_t t = ((units + passes - 1) / passes + 31) / 32 * 32;
+  return (int)std::min(most, std::max<int64_t>(t, 128));
+}
+// The plan's row partition for vectors of type V: as many CTAs as SMs, at least 256 rows
+// each on average, with equal shares of the rows' cost: FP64 the FMA slots of the row's
+// passes (U entries each) and 8 of the vector updates; FP32 its entries and 12.
+template <typename V>
+static mg_status resident_partition(mg_plan* p, const RowPartition** out)
+{
+  std::lock_guard<std::mutex> lock(p->upload_mu);
+  RowPartition& rp = p->cg_part[sizeof(V) == 8 ? 0 : 1];
+  *out = &rp;
+  if (rp.ctas != 0) return MG_OK;
+  const int64_t n = p->ndof;
+  const int ctas = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)sm_count(), (n + 255) / 256, (int64_t)kMaxResidentCtas}));
+  const auto cost = [&](int64_t r) -> int64_t {
+    const int64_t len = p->rowptr[r + 1] - p->rowptr[r];
+    constexpr int U = CgShape<V>::U;
+    return sizeof(V) == 8 ? U * std::max<int64_t>(1, (len + U - 1) / U) + 8 : len + 12;
+  };
+  int64_t total = 0;
+  for (int64_t r = 0; r < n; ++r) total += cost(r);
+  std::vector<int32_t> part(ctas + 1, (int32_t)n);
+  part[0] = 0;
+  int64_t sum = 0;
+  int c = 1;
+  for (int64_t r = 0; r < n && c < ctas; ++r) {
+    sum += cost(r);
+    while (c < ctas && sum * ctas >= total * c) part[c++] = (int32_t)(r + 1);
+  }
+  int max_rows = 0;
+  for (int k = 0; k < ctas; ++k) max_rows = std::max(max_rows, part[k + 1] - part[k]);
+  int32_t* d = nullptr;
+  MG_CUDA(cudaMalloc(&d, sizeof(int32_t) * part.size()));
+  const cudaError_t e = cudaMemcpy(d, part.data(), sizeof(int32_t) * part.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaFree(d);
+    return cuda_error(e, "CG row partition");
+  }
+  rp.d_rows = d;
+  rp.max_rows = max_rows;
+  rp.ctas = ctas;
+  return MG_OK;
+}
+
+template <typename V, int G, int U, typename I>
+static mg_status resident_launch(mg_plan* p, const RowPartition* part, const V* vals, V* x, CgWork<V>& w, int threads, size_t smem,
+                                 bool in_smem, unsigned int epoch, cudaStream_t st)
+{
+  const auto kernel = k_cg_resident<V, G, U, I>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)part->ctas);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const I* ci;
+  if constexpr (sizeof(I) == 2) ci = p->d_coloff;
+  else ci = p->d_colind;
+  MG_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const int32_t*)part->d_rows, part->max_rows, (const int32_t*)p->d_rowptr, ci,
+                             vals, w.dinv, x, w.r, w.z, w.p, w.q, in_smem ? 1 : 0, w.gather, epoch, kResidentIters, w.s));
+  return MG_OK;
+}
+// Whether all CTAs of the kernel can be resident at once (else the caller takes the
+// three-kernel iteration).
+template <typename V, int G, int U, typename I>
+static mg_status resident_fits(int ctas, int threads, size_t smem, bool* fits)
+{
+  const auto kernel = k_cg_resident<V, G, U, I>;
+  MG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0;
+  MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+  *fits = (int64_t)per_sm * sm_count() >= ctas;
+  return MG_OK;
+}
+
 // Runs CG on A (vals) from the state set up by k_cg_start until `done`.
 template <typename V>
 static mg_status cg_iterate(mg_plan* p, const V* vals, V* x, CgWork<V>& w, int G, int nb, int maxit,
-                            cudaStream_t st, CgScalars* h_s)
+                            cudaStream_t st, CgScalars* h_s, unsigned int* epoch)
 {
   const int64_t n = p->ndof;
   const int vb = vec_blocks<V>(n);
@@ -718,6 +1146,40 @@ static mg_status cg_iterate(mg_plan* p, const V* vals, V* x, CgWork<V>& w, int G
   bool use_graph = true;
   cudaStreamCaptureStatus cs;
   MG_CUDA(cudaStreamIsCapturing(st, &cs));
+  const RowPartition* part = nullptr;
+  MG_TRY(resident_partition<V>(p, &part));
+  constexpr int U = CgShape<V>::U;
+  const int threads = resident_threads<V>(part->max_rows, G);
+  const bool in_smem = resident_smem<V>(part->ctas, threads, part->max_rows, true) <= kResidentVectors;
+  const size_t smem = resident_smem<V>(part->ctas, threads, part->max_rows, in_smem);
+  const int64_t bytes = p->nnz * (int64_t)(sizeof(V) + (p->d_coloff ? 2 : 4)) + 6 * n * (int64_t)sizeof(V);
+  bool resident = bytes <= kResidentBytes && smem <= kResidentVectors && cs == cudaStreamCaptureStatusNone;
+  const auto on_kernel = [&](auto&& f) -> mg_status {  // f(lanes per row, index type) of this system
+    if constexpr (sizeof(V) == 8) {
+      return p->d_coloff ? f(std::integral_constant<int, 1>(), int16_t()) : f(std::integral_constant<int, 1>(), int32_t());
+    } else {
+      MG_DISPATCH_G(G, return p->d_coloff ? f(std::integral_constant<int, g>(), int16_t())
+                                          : f(std::integral_constant<int, g>(), int32_t()))
+    }
+    return MG_OK;
+  };
+  if (resident)
+    MG_TRY(on_kernel([&](auto g, auto i) {
+      return resident_fits<V, decltype(g)::value, U, decltype(i)>(part->ctas, threads, smem, &resident);
+    }));
+  if (resident) {
+    for (;;) {
+      MG_CUDA(cudaMemsetAsync(w.gather.count, 0, sizeof(unsigned int), st));
+      MG_TRY(on_kernel([&](auto g, auto i) {
+        return resident_launch<V, decltype(g)::value, U, decltype(i)>(p, part, vals, x, w, threads, smem, in_smem, *epoch, st);
+      }));
+      *epoch += 2 * kResidentIters;
+      MG_CUDA(cudaMemcpyAsync(h_s, w.s, sizeof(CgScalars), cudaMemcpyDeviceToHost, st));
+      MG_CUDA(cudaStreamSynchronize(st));
+      if (h_s->done == 9) return set_error(MG_ERR_CUDA, "CG: a wait between the kernel's CTAs ran out");
+      if (h_s->done) return MG_OK;
+    }
+  }
   if (cs != cudaStreamCaptureStatusNone || st == nullptr) use_graph = false;  // no nested capture; legacy stream cannot capture
   constexpr bool pdl = CgShape<V>::pdl;
   auto body = [&]() {
@@ -769,6 +1231,7 @@ static mg_status cg_start(mg_plan* p, const V* vals, const V* b, const V* x, int
   init.tol2 = tol * tol;
   init.maxit = maxit;
   MG_CUDA(cudaMemcpyAsync(w.s, &init, sizeof(CgScalars), cudaMemcpyHostToDevice, st));
+  MG_CUDA(cudaMemsetAsync(w.gather.words, 0, kGatherBytes, st));  // no epoch is current
   const int64_t n = p->ndof;
   MG_DISPATCH_G(G, (k_cg_start<V, g><<<nb, kSolveThreads, 0, st>>>(n, p->d_rowptr, p->d_colind, vals, p->d_diag, b,
                                                                      x, zero_x, jacobi, w.r, w.z, w.p, w.dinv,
@@ -910,7 +1373,8 @@ mg_status mg_cg_solve(mg_plan* p, const double* d_values, const double* d_b, dou
   MG_CUDA(cudaEventRecord(e0, st));
   CgScalars* hs = reinterpret_cast<CgScalars*>(p->h_pinned);
   mg_status s = cg_start<double>(p, d_values, d_b, d_x, 0, precond == MG_PREC_JACOBI, rtol, maxit, w, G, nb, st);
-  if (s == MG_OK) s = cg_iterate<double>(p, d_values, d_x, w, G, nb, maxit, st, hs);
+  unsigned int epoch = 0;
+  if (s == MG_OK) s = cg_iterate<double>(p, d_values, d_x, w, G, nb, maxit, st, hs, &epoch);
   MG_CUDA(cudaEventRecord(e1, st));
   MG_CUDA(cudaEventSynchronize(e1));
   float ms = 0.f;
@@ -961,6 +1425,7 @@ mg_status mg_cg_refined(mg_plan* p, const double* d_values64, const float* d_val
   MG_CUDA(cudaEventCreate(&e1));
   MG_CUDA(cudaEventRecord(e0, st));
   int anchors = 0, inner = 0;
+  unsigned int epoch = 0;
   bool converged = false;
   double relres = INFINITY, bb64 = 1.0;
   mg_status s = MG_OK;
@@ -997,7 +1462,7 @@ mg_status mg_cg_refined(mg_plan* p, const double* d_values64, const float* d_val
       MG_CUDA(cudaMemcpyAsync(w.s, hs, sizeof(CgScalars), cudaMemcpyHostToDevice, st));
     }
     while (s == MG_OK) {
-      s = cg_iterate<float>(p, d_values32, x32, w, G, nb, max_inner, st, hs);
+      s = cg_iterate<float>(p, d_values32, x32, w, G, nb, max_inner, st, hs, &epoch);
       if (s != MG_OK) break;
       inner = hs->iter;
       const int why = hs->done;
