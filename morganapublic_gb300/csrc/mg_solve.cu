@@ -110,6 +110,10 @@ static int row_group(const mg_plan* p)
   return row_group<V>(p->ndof, p->nnz);
 }
 
+// FP32 rows are streamed where the columns are 32-bit (16-bit offsets need each entry's
+// row) and rows are long.
+static bool stream_rows(const mg_plan* p) { return !p->d_coloff && p->nnz > 16 * p->ndof; }
+
 // CTAs covering every row once (G lanes per row), for the standalone SpMV.
 static int spmv_full_grid(int64_t rows, int G)
 {
@@ -215,6 +219,60 @@ __device__ __forceinline__ V row_dot(int64_t row, const int32_t* __restrict__ rp
 #pragma unroll
   for (int off = G / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(group_mask<G>(), sum, off, G);
   return sum;
+}
+
+// 16 rows by one warp, their entries streamed: each lane loads every 32nd entry of the
+// rows (coalesced, kStreamBatch in flight before the gathers of x) and writes the
+// products to the warp's window of shared memory, then two lanes sum each row's
+// products from there with compensation (error-free sums of the rounded products: as
+// accurate as a chain of FMAs in several accumulators, and as fast as plain sums here).
+// Returns row (row0 + lane / 2)'s sum, in both of its lanes.
+// Bound by the gathers of x and the L1 data path (76 % of its wavefronts; with a few
+// lanes per row every load touches several rows' lines).  GB300, P2 37 x 51 x 43 in
+// FP32: 39.0 -> 35.9 us at 8 CTAs per SM (42.7 at 6).  Whole warps per row (32 lanes,
+// eight rows reduced together) measured 63 us.
+constexpr int kStreamRows = 16, kStreamWindow = 512, kStreamBatch = 8;
+__device__ __forceinline__ float rows_dot_stream(int64_t row0, int64_t n, const int32_t* __restrict__ rp,
+                                                 const int32_t* __restrict__ ci, const float* __restrict__ val,
+                                                 const float* __restrict__ x, float* window)
+{
+  const int lane = threadIdx.x & 31;
+  const int64_t row = row0 + (lane >> 1);
+  const int lo = __ldg(rp + min(row, n)), hi = __ldg(rp + min(row + 1, n));
+  const int s0 = __shfl_sync(0xffffffffu, lo, 0), s1 = __shfl_sync(0xffffffffu, hi, 31);
+  ff sum{0.0f, 0.0f};
+  for (int w0 = s0; w0 < s1; w0 += kStreamWindow) {
+    const int w1 = min(w0 + kStreamWindow, s1);
+    for (int e0 = w0; e0 < w1; e0 += 32 * kStreamBatch) {
+      int c[kStreamBatch];
+      float v[kStreamBatch];
+#pragma unroll
+      for (int u = 0; u < kStreamBatch; ++u) {
+        const int e = e0 + 32 * u + lane;
+        c[u] = e < w1 ? __ldg(ci + e) : -1;
+        v[u] = e < w1 ? __ldg(val + e) : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < kStreamBatch; ++u)
+        if (c[u] >= 0) window[e0 - w0 + 32 * u + lane] = __fmul_rn(v[u], __ldg(x + c[u]));
+    }
+    __syncwarp();
+    const int i1 = min(hi, w1) - w0;
+    for (int i = max(lo, w0) - w0 + (lane & 1); i < i1; i += 8) {
+      float q[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) q[u] = i + 2 * u < i1 ? window[i + 2 * u] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const ff t = two_sum(sum.hi, q[u]);
+        sum.hi = t.hi;
+        sum.lo = __fadd_rn(sum.lo, t.lo);
+      }
+    }
+    __syncwarp();
+  }
+  const ff t = two_sum(sum.hi, __shfl_xor_sync(0xffffffffu, sum.hi, 1));
+  return __fadd_rn(t.hi, __fadd_rn(t.lo, __fadd_rn(sum.lo, __shfl_xor_sync(0xffffffffu, sum.lo, 1))));
 }
 
 // Dot-product accumulation: FP64 for FP64 vectors; for FP32 vectors a
@@ -345,6 +403,22 @@ __global__ void __launch_bounds__(kSolveThreads) k_spmv(int64_t n, const int32_t
   }
 }
 
+// y = A x by streamed rows (rows_dot_stream), one warp per 16 rows
+__global__ void __launch_bounds__(kSolveThreads, 8)
+    k_spmv_stream(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                  const float* __restrict__ val, const float* __restrict__ x, float* __restrict__ y)
+{
+  __shared__ float window[kSolveThreads / 32][kStreamWindow];
+  pdl_wait();
+  pdl_trigger();
+  const int64_t row0 = (blockIdx.x * (int64_t)(kSolveThreads / 32) + (threadIdx.x >> 5)) * kStreamRows;
+  if (row0 >= n) return;
+  const float s = rows_dot_stream(row0, n, rp, ci, val, x, window[threadIdx.x >> 5]);
+  const int lane = threadIdx.x & 31;
+  const int64_t row = row0 + (lane >> 1);
+  if ((lane & 1) == 0 && row < n) y[row] = s;
+}
+
 // K1: q = A p, alpha = rz / (p . q)
 template <typename V, int G, typename I>
 __global__ void __launch_bounds__(kSolveThreads) k_cg_spmv(int64_t n, const int32_t* __restrict__ rp,
@@ -380,6 +454,45 @@ __global__ void __launch_bounds__(kSolveThreads) k_cg_spmv(int64_t n, const int3
   }
 }
 
+// K1 by streamed rows (rows_dot_stream), FP32 (P2 48^3, mixed solve: 49.6 -> 47.5 ms)
+constexpr int kCgStreamCtas = 6;  // per SM: 40 registers; 8 spill (60.8 ms a solve), 5: 48.9 ms
+__global__ void __launch_bounds__(kSolveThreads, kCgStreamCtas)
+    k_cg_spmv_stream(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                     const float* __restrict__ val, const float* __restrict__ p, float* __restrict__ q, double* partials,
+                     CgScalars* s)
+{
+  using D = Dot<float>;
+  __shared__ float window[kSolveThreads / 32][kStreamWindow];
+  __shared__ D::A sh[32];
+  __shared__ double shd[32];
+  pdl_wait();
+  pdl_trigger();
+  if (s->done) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t step = (int64_t)gridDim.x * (kSolveThreads / 32) * kStreamRows;
+  D::A acc = D::zero();
+  for (int64_t row0 = (blockIdx.x * (int64_t)(kSolveThreads / 32) + (threadIdx.x >> 5)) * kStreamRows; row0 < n;
+       row0 += step) {
+    const float v = rows_dot_stream(row0, n, rp, ci, val, p, window[threadIdx.x >> 5]);
+    const int64_t row = row0 + (lane >> 1);
+    if ((lane & 1) == 0 && row < n) {
+      q[row] = v;
+      D::mac(acc, p[row], v);
+    }
+  }
+  const double b = block_sum<float>(acc, sh);
+  if (threadIdx.x == 0) partials[blockIdx.x] = b;
+  if (last_block(&s->ticket[0])) {
+    const double pq = reduce_partials(partials, gridDim.x, shd);
+    if (threadIdx.x == 0) {
+      s->pq = pq;
+      s->alpha = s->rz / pq;
+      if (!(pq > 0.0) || !isfinite(s->alpha)) s->done = 2;
+      s->ticket[0] = 0;
+    }
+  }
+}
+
 // K2: x += alpha p; r -= alpha q; z = D^-1 r; rz, rr, beta, convergence
 template <typename V>
 __global__ void __launch_bounds__(kSolveThreads) k_cg_update(int64_t n, V* __restrict__ x, V* __restrict__ r,
@@ -395,8 +508,34 @@ __global__ void __launch_bounds__(kSolveThreads) k_cg_update(int64_t n, V* __res
   if (s->done) return;
   const V alpha = (V)s->alpha;
   typename D::A prz = D::zero(), prr = D::zero();
+  int64_t i0 = 0;
+  if constexpr (sizeof(V) == 4) {
+    // FP32: the vectors are the solver's own (16-byte aligned), four entries per step
+    // (P2 48^3: update 15.3 -> 12.6 us, direction 6.5 -> 4.9 us)
+    const int64_t n4 = n / 4;
+    i0 = 4 * n4;
+    for (int64_t i = blockIdx.x * (int64_t)kSolveThreads + threadIdx.x; i < n4;
+         i += (int64_t)gridDim.x * kSolveThreads) {
+      const float4 pv = reinterpret_cast<const float4*>(p)[i], qv = reinterpret_cast<const float4*>(q)[i];
+      const float4 dv = reinterpret_cast<const float4*>(dinv)[i];
+      float4 xv = reinterpret_cast<float4*>(x)[i], rv = reinterpret_cast<float4*>(r)[i], zv;
+      float *xp = &xv.x, *rp = &rv.x, *zp = &zv.x;
+      const float *pp = &pv.x, *qp = &qv.x, *dp = &dv.x;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        xp[k] += alpha * pp[k];
+        rp[k] -= alpha * qp[k];
+        zp[k] = dp[k] * rp[k];
+        D::mac(prz, rp[k], zp[k]);
+        D::mac(prr, rp[k], rp[k]);
+      }
+      reinterpret_cast<float4*>(x)[i] = xv;
+      reinterpret_cast<float4*>(r)[i] = rv;
+      reinterpret_cast<float4*>(z)[i] = zv;
+    }
+  }
 #pragma unroll 4
-  for (int64_t i = blockIdx.x * (int64_t)kSolveThreads + threadIdx.x; i < n;
+  for (int64_t i = i0 + blockIdx.x * (int64_t)kSolveThreads + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * kSolveThreads) {
     x[i] += alpha * p[i];
     const V ri = r[i] - alpha * q[i];
@@ -440,8 +579,20 @@ __global__ void __launch_bounds__(kSolveThreads) k_cg_dir(int64_t n, const V* __
   pdl_trigger();
   if (s->done) return;
   const V beta = (V)s->beta;
+  int64_t i0 = 0;
+  if constexpr (sizeof(V) == 4) {
+    const int64_t n4 = n / 4;
+    i0 = 4 * n4;
+    for (int64_t i = blockIdx.x * (int64_t)kSolveThreads + threadIdx.x; i < n4;
+         i += (int64_t)gridDim.x * kSolveThreads) {
+      const float4 zv = reinterpret_cast<const float4*>(z)[i];
+      float4 pv = reinterpret_cast<float4*>(p)[i];
+      pv = make_float4(zv.x + beta * pv.x, zv.y + beta * pv.y, zv.z + beta * pv.z, zv.w + beta * pv.w);
+      reinterpret_cast<float4*>(p)[i] = pv;
+    }
+  }
 #pragma unroll 4
-  for (int64_t i = blockIdx.x * (int64_t)kSolveThreads + threadIdx.x; i < n;
+  for (int64_t i = i0 + blockIdx.x * (int64_t)kSolveThreads + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * kSolveThreads)
     p[i] = z[i] + beta * p[i];
 }
@@ -957,6 +1108,10 @@ mg_status launch_spmv(mg_plan* p, int prec, const void* vals, const void* x, voi
       if (G == 1) launch_pdl(k_spmv<double, 1, kF64Entries, int32_t>, nb, kSolveThreads, st, n, rp, c, v, xx, yy);
       else launch_pdl(k_spmv<double, 2, kF64PairEntries, int32_t>, nb, kSolveThreads, st, n, rp, c, v, xx, yy);
     }
+  } else if (stream_rows(p)) {
+    const int64_t warps = (p->ndof + kStreamRows - 1) / kStreamRows, per = kSolveThreads / 32;
+    launch_pdl(k_spmv_stream, (int)((warps + per - 1) / per), kSolveThreads, st, p->ndof, (const int32_t*)p->d_rowptr,
+               (const int32_t*)p->d_colind, (const float*)vals, (const float*)x, (float*)y);
   } else {
     const int G = row_group<float>(p), nb = row_blocks<float>(p, G);
     if (p->d_coloff) {
@@ -1183,7 +1338,15 @@ static mg_status cg_iterate(mg_plan* p, const V* vals, V* x, CgWork<V>& w, int G
   if (cs != cudaStreamCaptureStatusNone || st == nullptr) use_graph = false;  // no nested capture; legacy stream cannot capture
   constexpr bool pdl = CgShape<V>::pdl;
   auto body = [&]() {
-    if (p->d_coloff) {
+    if constexpr (sizeof(V) == 4) {
+      if (stream_rows(p))
+        launch_k(pdl, k_cg_spmv_stream, row_blocks((n + kStreamRows - 1) / kStreamRows, 32, kCgStreamCtas), kSolveThreads, st, n,
+                 (const int32_t*)p->d_rowptr, (const int32_t*)p->d_colind, vals, (const float*)w.p, w.q, w.partials,
+                 w.s);
+    }
+    if (sizeof(V) == 4 && stream_rows(p)) {
+      // launched above
+    } else if (p->d_coloff) {
       MG_DISPATCH_G(G, (launch_k(pdl, k_cg_spmv<V, g, int16_t>, nb, kSolveThreads, st, n,
                                  (const int32_t*)p->d_rowptr, (const int16_t*)p->d_coloff, vals, (const V*)w.p, w.q,
                                  w.partials, w.s)));
