@@ -40,6 +40,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 #include "mg_ff.cuh"
 #include "mg_internal.h"
@@ -67,13 +68,8 @@ __device__ __forceinline__ bool dw_scale_ok(float hi)
 __device__ __forceinline__ bool dw_scale_ok(ff v) { return dw_scale_ok(v.hi); }
 
 template <int MODE> struct Arith;
-// sum_into(s, x): s += x for the phase-2 sums.  The double-word form defers
-// renormalisation: the high words are added error-free (two_sum), the low
-// words and errors collect in s.lo, which may exceed half an ulp of s.hi (the
-// final hi + lo is formed in FP64 when the value is written).
 template <> struct Arith<kF32> {
   using T = float;
-  __device__ static void sum_into(T& s, T x) { s += x; }
   using Out = float;
   // double -> float by integer operations (the conversion instruction runs on
   // the FP64 pipe): hi + lo of the double-word split, rounded once
@@ -83,28 +79,18 @@ template <> struct Arith<kF32> {
     return __fadd_rn(t.hi, t.lo);
   }
   __device__ static T zero() { return 0.0f; }
-  __device__ static Out out(T v) { return v; }
 };
 template <> struct Arith<kDW> {
   using T = ff;
-  __device__ static void sum_into(T& s, T x)
-  {
-    const ff t = two_sum(s.hi, x.hi);
-    s.hi = t.hi;
-    s.lo = __fadd_rn(s.lo, __fadd_rn(t.lo, x.lo));
-  }
   using Out = double;
   __device__ static T from(double x) { return ff_from_double_bits(x); }
   __device__ static T zero() { return ff{0.0f, 0.0f}; }
-  __device__ static Out out(T v) { return ff_to_double_int(v); }
 };
 template <> struct Arith<kF64> {
   using T = double;
-  __device__ static void sum_into(T& s, T x) { s += x; }
   using Out = double;
   __device__ static T from(double x) { return x; }
   __device__ static T zero() { return 0.0; }
-  __device__ static Out out(T v) { return v; }
 };
 
 // ---------------------------------------------------------------- geometry --
@@ -183,12 +169,7 @@ constexpr float kCancelTol = 16.0f;
 template <typename T>
 __device__ __forceinline__ float hi_of(const T& v);
 template <>
-__device__ __forceinline__ float hi_of<float>(const float& v) { return v; }
-template <>
 __device__ __forceinline__ float hi_of<ff>(const ff& v) { return v.hi; }
-
-template <>
-__device__ __forceinline__ float hi_of<double>(const double& v) { return (float)v; }
 
 // P1 stiffness needs the gradient of every vertex: the columns C_0..C_3 of the
 // cofactor matrix (gradients times det).  C_1..C_3 come from the edge vectors at
@@ -427,7 +408,7 @@ __device__ __forceinline__ ff metric_dot<ff>(const ff g[6], const ff* tab, int N
 // ------------------------------------------------------------ assembly --
 // P1: the one-pass block assembly (k_block_asm, k_shared_sum, below).
 // P2, two passes, each element computed once:
-//   k_elem_mat     one thread per element, along the plan's Morton order p: the
+//   k_elem_mat_pair  two elements per thread, along the plan's Morton order p: the
 //                  unique entries u of its (symmetric) element matrix into the
 //                  plan's element-matrix array em;
 //   k_slot_gather  one thread per diagonal or upper CSR entry: the sum of the em
@@ -436,49 +417,15 @@ __device__ __forceinline__ ff metric_dot<ff>(const ff g[6], const ff* tab, int N
 //                  entry and to its mirror -- a fixed order, so the values are
 //                  bitwise reproducible, with no atomics.
 
-// Geometry of an element from the mesh's absolute node records, in the mode's
-// arithmetic; returns whether the determinant cancels (det_cancels).
-//  FP32          edges (hi_k - hi_0) + (mid_k - mid_0), to a float ulp of the
-//                edge;
-//  double-word   edges dw_diff3 of the three floats: the exact FP64 difference
-//                of the mesh coordinates (the reference's x_k - x_0) to ~2^-47;
-//  FP64          from the FP64 coordinates.
-template <int MODE>
-__device__ __forceinline__ bool geometry_abs_lazy(const GeoPtrs& g, int4 n, Cof<typename Arith<MODE>::T>& f)
+// Geometry of an element from the mesh's FP64 coordinates.
+__device__ __forceinline__ void geometry_f64(const GeoPtrs& g, int4 n, Cof<double>& f)
 {
-  using T = typename Arith<MODE>::T;
-  T J[3][3];
-  if constexpr (MODE == kF64) {
-    const double4_32a x0 = g.xyz[n.x];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const double4_32a xk = g.xyz[k == 0 ? n.y : (k == 1 ? n.z : n.w)];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) J[r][k] = comp(xk, r) - comp(x0, r);
-    }
-    cofactors<double>(J, f);
-    return false;
-  } else {
-    const float4 a0 = g.rec[2 * (int64_t)n.x], b0 = g.rec[2 * (int64_t)n.x + 1];
-    const float lz0 = MODE == kDW ? g.loz[n.x] : 0.0f;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const int64_t id = k == 0 ? n.y : (k == 1 ? n.z : n.w);
-      const float4 ak = g.rec[2 * id], bk = g.rec[2 * id + 1];
-      const float lzk = MODE == kDW ? g.loz[id] : 0.0f;
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        if constexpr (MODE == kF32)
-          J[r][k] = (rec_hi(ak, r) - rec_hi(a0, r)) + (rec_mid(ak, bk, r) - rec_mid(a0, b0, r));
-        else
-          J[r][k] = dw_diff3(rec_hi(ak, r), rec_hi(a0, r), rec_mid(ak, bk, r), rec_mid(a0, b0, r), rec_lo(bk, lzk, r),
-                             rec_lo(b0, lz0, r));
-      }
-    }
-    if constexpr (MODE == kDW) dw_cofactors(J, f);
-    else cofactors<T>(J, f);
-    return det_cancels<T>(J, f);
-  }
+  Fetch<kF64> D;
+  D.x[0] = g.xyz[n.x];
+  D.x[1] = g.xyz[n.y];
+  D.x[2] = g.xyz[n.z];
+  D.x[3] = g.xyz[n.w];
+  geometry(D, f);
 }
 
 // Near-degenerate elements: the FP64 geometry from the mesh's FP64 coordinates,
@@ -564,7 +511,7 @@ struct ElemArgs {
   GeoPtrs geo;
   const double* coeff;        // per element in the caller's order, or null
   double cconst;              // used when coeff is null
-  const double* tables;       // unique-entry tables: stiff[6][nu] then mass[nu]
+  const double* tables;       // unique-entry tables: stiff[6][nu], mass[nu], P2: bary[kBaryTerms]
   double wsum;
   float w_hi, w_lo;           // wsum as a double-word
   int stiff;
@@ -593,7 +540,7 @@ __device__ __forceinline__ int4 elem_nodes(const ElemArgs& a, int64_t p)
 __device__ __forceinline__ void p1_element_f64(const ElemArgs& a, const double* mass, int4 n, double coef, double K[10])
 {
   Cof<double> f;
-  geometry_abs_lazy<kF64>(a.geo, n, f);
+  geometry_f64(a.geo, n, f);
   if (coef_not_finite(coef)) atomicOr(a.flags, 1u);
   if (a.stiff) {
     // the rare elements (p1_class) go out of line, entered only when a lane of
@@ -730,61 +677,75 @@ __device__ __forceinline__ void em_pair(float* em, int u, int lp, f2 v)
   em[u * kElemBlock + lp + 32] = x.y;
 }
 
+// Cofactor columns C[k][r] = cofactor (r, k) of J and the determinant of a pair; per lane
+// whether the determinant cancels.
+struct PairGeo {
+  ff2 C[3][3];
+  ff2 det;
+  bool degen0, degen1;
+};
+__device__ __forceinline__ void pair_cofactors(const ff2 (&J)[3][3], PairGeo& f)
+{
+  f2 nJ[3][3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) nJ[r][k] = -J[r][k].hi;
+#define MG_COF(r, k, r1, k1, r2, k2) \
+  f.C[k][r] = ff2_cross(J[r1][k1], J[r2][k2], J[r1][k2], J[r2][k1], nJ[r1][k1], nJ[r1][k2], nJ[r2][k1])
+  MG_COF(0, 0, 1, 1, 2, 2);
+  MG_COF(0, 1, 1, 2, 2, 0);
+  MG_COF(0, 2, 1, 0, 2, 1);
+  MG_COF(1, 0, 2, 1, 0, 2);
+  MG_COF(1, 1, 2, 2, 0, 0);
+  MG_COF(1, 2, 2, 0, 0, 1);
+  MG_COF(2, 0, 0, 1, 1, 2);
+  MG_COF(2, 1, 0, 2, 1, 0);
+  MG_COF(2, 2, 0, 0, 1, 1);
+#undef MG_COF
+  const ff2 c0[3] = {f.C[0][0], f.C[1][0], f.C[2][0]};
+  const ff2 d = ff2_dot3(J[0], c0, nJ[0]);
+  f.det = f2_fast_two_sum(d.hi, d.lo);
+  const float2 dh = f2_get(f.det.hi), t0 = f2_get(J[0][0].hi * c0[0].hi), t1 = f2_get(J[0][1].hi * c0[1].hi),
+               t2 = f2_get(J[0][2].hi * c0[2].hi);
+  f.degen0 = cancels(t0.x, t1.x, t2.x, dh.x);
+  f.degen1 = cancels(t0.y, t1.y, t2.y, dh.y);
+}
+// n / det: quotient digits q1 + q2 + q3, the remainder of each by FMAs; |det| in 2^-100 .. 2^100
+__device__ __forceinline__ ff2 pair_quotient(f2 nh, f2 nl, ff2 det)
+{
+  const f2 rb = f2_rcp(det.hi), nd = -det.hi;
+  const f2 q1 = nh * rb;
+  const f2 r1 = fma2(nd, q1, nh) + fma2(-det.lo, q1, nl);
+  const f2 q2 = r1 * rb;
+  const f2 q3 = fma2(nd, q2, r1) * rb;
+  return f2_fast_two_sum(q1, q2 + q3);
+}
+
 // From the pair's edges J and coefficients; node(e): the global vertex ids of
 // element e of the pair (for the rare paths).
 template <typename Node>
 __device__ __forceinline__ void p1_pair_dw(const ElemArgs& a, const ff* mass, const ff2 (&J)[3][3], Node node, double coef0,
                                            double coef1, int lp, float* em_hi, float* em_lo)
 {
-  ff2 C[3][3];  // C[k]: cofactor column k of J (C[k][r] = cofactor (r, k))
-  ff2 det;
-  bool degen0, degen1;
-  {
-    f2 nJ[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) nJ[r][k] = -J[r][k].hi;
-#define MG_COF(r, k, r1, k1, r2, k2) \
-  C[k][r] = ff2_cross(J[r1][k1], J[r2][k2], J[r1][k2], J[r2][k1], nJ[r1][k1], nJ[r1][k2], nJ[r2][k1])
-    MG_COF(0, 0, 1, 1, 2, 2);
-    MG_COF(0, 1, 1, 2, 2, 0);
-    MG_COF(0, 2, 1, 0, 2, 1);
-    MG_COF(1, 0, 2, 1, 0, 2);
-    MG_COF(1, 1, 2, 2, 0, 0);
-    MG_COF(1, 2, 2, 0, 0, 1);
-    MG_COF(2, 0, 0, 1, 1, 2);
-    MG_COF(2, 1, 0, 2, 1, 0);
-    MG_COF(2, 2, 0, 0, 1, 1);
-#undef MG_COF
-    const ff2 c0[3] = {C[0][0], C[1][0], C[2][0]};
-    const ff2 d = ff2_dot3(J[0], c0, nJ[0]);
-    det = f2_fast_two_sum(d.hi, d.lo);
-    const float2 dh = f2_get(det.hi), t0 = f2_get(J[0][0].hi * c0[0].hi), t1 = f2_get(J[0][1].hi * c0[1].hi),
-                 t2 = f2_get(J[0][2].hi * c0[2].hi);
-    degen0 = cancels(t0.x, t1.x, t2.x, dh.x);
-    degen1 = cancels(t0.y, t1.y, t2.y, dh.y);
-    if (a.stiff) {
-      degen0 |= det_extreme(dh.x);
-      degen1 |= det_extreme(dh.y);
-    }
+  PairGeo f;
+  pair_cofactors(J, f);
+  const ff2 (&C)[3][3] = f.C;
+  ff2& det = f.det;
+  bool &degen0 = f.degen0, &degen1 = f.degen1;
+  if (a.stiff) {
+    const float2 dh = f2_get(det.hi);
+    degen0 |= det_extreme(dh.x);
+    degen1 |= det_extreme(dh.y);
   }
   if (coef_not_finite(coef0) || coef_not_finite(coef1)) atomicOr(a.flags, 1u);
   const ff2 coef = ff2_make(ff_from_double_bits(coef0), ff_from_double_bits(coef1));
   if (a.stiff) {
-    // s = coef w / det: quotient digits q1 + q2 + q3, the remainder of each by FMAs
-    ff2 s;
-    {
-      const f2 wh = f2_make(a.w_hi, a.w_hi), wl = f2_make(a.w_lo, a.w_lo);
-      const f2 nh = coef.hi * wh;
-      const f2 nl = fma2(coef.lo, wh, coef.hi * wl) - fma2(-coef.hi, wh, nh);
-      const f2 rb = f2_rcp(det.hi), nd = -det.hi;
-      const f2 q1 = nh * rb;
-      const f2 r1 = fma2(nd, q1, nh) + fma2(-det.lo, q1, nl);
-      const f2 q2 = r1 * rb;
-      const f2 q3 = fma2(nd, q2, r1) * rb;
-      s = f2_fast_two_sum(q1, q2 + q3);
-    }
+    // s = coef w / det
+    const f2 wh = f2_make(a.w_hi, a.w_hi), wl = f2_make(a.w_lo, a.w_lo);
+    const f2 nh = coef.hi * wh;
+    const f2 nl = fma2(coef.lo, wh, coef.hi * wl) - fma2(-coef.hi, wh, nh);
+    const ff2 s = pair_quotient(nh, nl, det);
     ff2 K[10];
     {
       const f2 ns = -s.hi;
@@ -861,17 +822,16 @@ __device__ __forceinline__ void p1_pair_dw(const ElemArgs& a, const ff* mass, co
   }
 }
 
-template <typename Node>
-__device__ __forceinline__ void p1_pair_f32(const ElemArgs& a, const float* mass, const f2 (&J)[3][3], Node node,
-                                            double coef0, double coef1, int lp, float* em)
+// FP32: C[0] from the face opposite vertex 0, (x3 - x1) x (x2 - x1), then the cofactor
+// columns of J; the determinant; per lane whether it cancels.
+__device__ __forceinline__ void pair_gradients(const f2 (&J)[3][3], f2 (&C)[4][3], f2& det, bool& degen0, bool& degen1)
 {
-  f2 C[3][3];  // cofactor columns
   f2 nJ[3][3];
 #pragma unroll
   for (int r = 0; r < 3; ++r)
 #pragma unroll
     for (int k = 0; k < 3; ++k) nJ[r][k] = -J[r][k];
-#define MG_COF(r, k, r1, k1, r2, k2) C[k][r] = f2_cross(J[r1][k1], J[r2][k2], J[r1][k2], J[r2][k1], nJ[r1][k2])
+#define MG_COF(r, k, r1, k1, r2, k2) C[k + 1][r] = f2_cross(J[r1][k1], J[r2][k2], J[r1][k2], J[r2][k1], nJ[r1][k2])
   MG_COF(0, 0, 1, 1, 2, 2);
   MG_COF(0, 1, 1, 2, 2, 0);
   MG_COF(0, 2, 1, 0, 2, 1);
@@ -882,47 +842,50 @@ __device__ __forceinline__ void p1_pair_f32(const ElemArgs& a, const float* mass
   MG_COF(2, 1, 0, 2, 1, 0);
   MG_COF(2, 2, 0, 0, 1, 1);
 #undef MG_COF
-  f2 det = fma2(J[0][2], C[2][0], fma2(J[0][1], C[1][0], J[0][0] * C[0][0]));
+  f2 e2[3], e3[3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    e2[r] = J[r][1] - J[r][0];
+    e3[r] = J[r][2] - J[r][0];
+  }
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    const int r1 = (r + 1) % 3, r2 = (r + 2) % 3;
+    C[0][r] = f2_cross(e3[r1], e2[r2], e3[r2], e2[r1], -e3[r2]);
+  }
+  det = fma2(J[0][2], C[3][0], fma2(J[0][1], C[2][0], J[0][0] * C[1][0]));
+  const float2 dh = f2_get(det), t0 = f2_get(J[0][0] * C[1][0]), t1 = f2_get(J[0][1] * C[2][0]),
+               t2 = f2_get(J[0][2] * C[3][0]);
+  degen0 = cancels(t0.x, t1.x, t2.x, dh.x);
+  degen1 = cancels(t0.y, t1.y, t2.y, dh.y);
+}
+
+template <typename Node>
+__device__ __forceinline__ void p1_pair_f32(const ElemArgs& a, const float* mass, const f2 (&J)[3][3], Node node,
+                                            double coef0, double coef1, int lp, float* em)
+{
+  f2 C[4][3];
+  f2 det;
   bool degen0, degen1;
-  {
-    const float2 dh = f2_get(det), t0 = f2_get(J[0][0] * C[0][0]), t1 = f2_get(J[0][1] * C[1][0]),
-                 t2 = f2_get(J[0][2] * C[2][0]);
-    degen0 = cancels(t0.x, t1.x, t2.x, dh.x);
-    degen1 = cancels(t0.y, t1.y, t2.y, dh.y);
-    if (a.stiff) {
-      degen0 |= det_extreme(dh.x);
-      degen1 |= det_extreme(dh.y);
-    }
+  pair_gradients(J, C, det, degen0, degen1);
+  if (a.stiff) {
+    const float2 dh = f2_get(det);
+    degen0 |= det_extreme(dh.x);
+    degen1 |= det_extreme(dh.y);
   }
   if (coef_not_finite(coef0) || coef_not_finite(coef1)) atomicOr(a.flags, 1u);
   const f2 coef = f2_make(Arith<kF32>::from(coef0), Arith<kF32>::from(coef1));
   if (a.stiff) {
-    // C_0 from the face opposite vertex 0, (x3 - x1) x (x2 - x1)
-    f2 C0[3];
-    {
-      f2 e2[3], e3[3];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        e2[r] = J[r][1] - J[r][0];
-        e3[r] = J[r][2] - J[r][0];
-      }
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        const int r1 = (r + 1) % 3, r2 = (r + 2) % 3;
-        C0[r] = f2_cross(e3[r1], e2[r2], e3[r2], e2[r1], -e3[r2]);
-      }
-    }
     // s = coef w / det, one correction of the quotient estimate
     const f2 nu = coef * f2_make(a.w_hi, a.w_hi), rb = f2_rcp(det), q = nu * rb;
     const f2 s = fma2(fma2(-det, q, nu), rb, q);
-    const f2* G[4] = {C0, C[0], C[1], C[2]};
     f2 diag[4];
     int u = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = i; j < 4; ++j, ++u) {
-        const f2 k = s * fma2(G[i][2], G[j][2], fma2(G[i][1], G[j][1], G[i][0] * G[j][0]));
+        const f2 k = s * fma2(C[i][2], C[j][2], fma2(C[i][1], C[j][1], C[i][0] * C[j][0]));
         if (j == i) diag[i] = k;
         em_pair(em, u, lp, k);
       }
@@ -949,52 +912,312 @@ __device__ __forceinline__ void p1_pair_f32(const ElemArgs& a, const float* mass
   }
 }
 
-// The element pass of the two-pass P2 assembly: one thread per element along
-// the plan's Morton order p, its 55 entries to em[u * E + p] (entry-major: the
-// stores of one u coalesce across the warp), the metric contraction reading the
-// tables from shared memory.
-template <int MODE>
-__global__ void __launch_bounds__(256, 1) k_elem_mat(ElemArgs a)
+// ------------------------------------------------- P2 elements, two per thread --
+// The stiffness in barycentric form: with G_ab = s C_a . C_b (C_0 = -(C_1 + C_2 + C_3),
+// C_a / det the gradient of lambda_a) and the P2 gradients (4 lambda_i - 1) grad
+// lambda_i and 4 (lambda_a grad lambda_b + lambda_b grad lambda_a), entry
+//   (vertex i, vertex j)              one term   G_ij
+//   (vertex i, edge (a, b))           two terms  G_ib, G_ia
+//   (edge (a, b), edge (c, d))        four terms G_bd, G_bc, G_ad, G_ac
+//   (edge (a, b) with itself)         three      G_bb, G_ab, G_aa
+// with coefficients summed over the card (RefTables::bary, in this order): 136 products
+// per element, where the contraction of the six metric coefficients C_a . C_b with
+// tables T^{ab} takes 330.
+constexpr int kBaryTerms = 10 + 24 * 2 + 15 * 4 + 6 * 3;
+// vertex s of local edge e: (0,1) (1,2) (2,0) (0,3) (1,3) (2,3)
+__host__ __device__ constexpr int p2_edge(int e, int s) { return (int)((0x323130022110ull >> (8 * e + 4 * s)) & 0xf); }
+// place of G_ab among the ten
+__host__ __device__ constexpr int g_index(int a, int b)
+{
+  return a <= b ? a * 4 - a * (a - 1) / 2 + (b - a) : b * 4 - b * (b - 1) / 2 + (a - b);
+}
+
+// sum_k g[i_k] t[k], N terms (i0 .. i3 the indices): double-word as in metric_dot,
+// packed; table entries as (hi, hi, lo, lo)
+template <int N>
+__device__ __forceinline__ ff2 bary_sum(const ff2 (&g)[10], const f2 (&ng)[10], const float4* t, int i0, int i1, int i2, int i3)
+{
+  const int id[4] = {i0, i1, i2, i3};
+  f2 hi, lo;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const float4 tk = t[k];
+    const f2 th = f2_make(tk.x, tk.y), tl = f2_make(tk.z, tk.w);
+    const ff2 gk = g[id[k]];
+    const f2 q = gk.hi * th, qe = fma2(ng[id[k]], th, q);
+    if (k == 0) {
+      hi = q;
+      lo = fma2(gk.hi, tl, gk.lo * th) - qe;
+    } else {
+      const ff2 s = f2_two_sum(hi, q);
+      hi = s.hi;
+      lo = lo + fma2(gk.hi, tl, fma2(gk.lo, th, s.lo - qe));
+    }
+  }
+  return f2_fast_two_sum(hi, lo);
+}
+template <int N>
+__device__ __forceinline__ f2 bary_sum(const f2 (&g)[10], const f2 (&)[10], const float2* t, int i0, int i1, int i2, int i3)
+{
+  const int id[4] = {i0, i1, i2, i3};
+  f2 v = g[i0] * f2_make(t[0].x, t[0].y);
+#pragma unroll
+  for (int k = 1; k < N; ++k) v = fma2(g[id[k]], f2_make(t[k].x, t[k].y), v);
+  return v;
+}
+// entry u of elements p0 and p1 into the element-matrix array
+__device__ __forceinline__ void em_pair_put(void* em, int64_t E, int u, int64_t p0, int64_t p1, ff2 v)
+{
+  const float2 h = f2_get(v.hi), l = f2_get(v.lo);
+  em_put(em, u * E + p0, ff{h.x, l.x});
+  em_put(em, u * E + p1, ff{h.y, l.y});
+}
+__device__ __forceinline__ void em_pair_put(void* em, int64_t E, int u, int64_t p0, int64_t p1, f2 v)
+{
+  const float2 x = f2_get(v);
+  em_put(em, u * E + p0, x.x);
+  em_put(em, u * E + p1, x.y);
+}
+template <typename T2, typename Tab>
+__device__ __forceinline__ void p2_stiffness(const T2 (&g)[10], const f2 (&ng)[10], const Tab* t, void* em, int64_t E,
+                                             int64_t p0, int64_t p1)
+{
+  int u = 0;
+#pragma unroll
+  for (int i = 0; i < 10; ++i)
+#pragma unroll
+    for (int j = i; j < 10; ++j, ++u) {
+      T2 v;
+      if (j < 4) {
+        v = bary_sum<1>(g, ng, t, g_index(i, j), 0, 0, 0);
+        t += 1;
+      } else if (i < 4) {
+        const int a = p2_edge(j - 4, 0), b = p2_edge(j - 4, 1);
+        v = bary_sum<2>(g, ng, t, g_index(i, b), g_index(i, a), 0, 0);
+        t += 2;
+      } else if (i != j) {
+        const int a = p2_edge(i - 4, 0), b = p2_edge(i - 4, 1), c = p2_edge(j - 4, 0), d = p2_edge(j - 4, 1);
+        v = bary_sum<4>(g, ng, t, g_index(b, d), g_index(b, c), g_index(a, d), g_index(a, c));
+        t += 4;
+      } else {
+        const int a = p2_edge(i - 4, 0), b = p2_edge(i - 4, 1);
+        v = bary_sum<3>(g, ng, t, g_index(b, b), g_index(a, b), g_index(a, a), 0);
+        t += 3;
+      }
+      em_pair_put(em, E, u, p0, p1, v);
+    }
+}
+
+__device__ __forceinline__ ff2 ff2_mul(ff2 a, ff2 b)
+{
+  const f2 p = a.hi * b.hi;
+  const f2 lo = fma2(a.hi, b.lo, a.lo * b.hi) - fma2(-a.hi, b.hi, p);
+  return f2_fast_two_sum(p, lo);
+}
+// -(a + b + c), the high parts summed error-free
+__device__ __forceinline__ ff2 ff2_neg_sum(ff2 a, ff2 b, ff2 c)
+{
+  const ff2 x = f2_two_sum(a.hi, b.hi), y = f2_two_sum(x.hi, c.hi);
+  return -f2_fast_two_sum(y.hi, (a.lo + b.lo) + (c.lo + (x.lo + y.lo)));
+}
+
+// The element pass of the two-pass P2 assembly: two elements per thread (Morton
+// positions 32 apart: a warp covers 64) as packed pairs, the 55 entries of each to
+// em[u * E + p] (entry-major: the stores of one u coalesce across the warp).
+// Bound by the element-matrix stores and instruction issue; GB300, P2 48^3, FP64: scalar
+// double-words with the six-coefficient contraction 125 us, this form 69 us.
+template <int MODE, bool SPLIT>
+__global__ void __launch_bounds__(128, 4) k_elem_mat_pair(ElemArgs a)
 {
   using A = Arith<MODE>;
-  using T = typename A::T;
+  using Tab = typename std::conditional<MODE == kDW, float4, float2>::type;
   constexpr int NU = 55;
-  __shared__ T tab[7 * NU];
-  for (int i = threadIdx.x; i < 7 * NU; i += blockDim.x) tab[i] = A::from(a.tables[i]);
-  __syncthreads();
-  const int64_t E = a.n_elem;
-  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  __shared__ Tab tab[kBaryTerms > NU ? kBaryTerms : NU];
   {
-    if (p >= E) return;
-    const double coef_d = a.coeff ? __ldg(a.coeff + a.elem_order[p]) : a.cconst;
-    const int32_t* dp = a.dofs_m + p * 10;
-    const int4 n = make_int4(dp[0], dp[1], dp[2], dp[3]);
-    Cof<T> f;
-    const bool degenerate = geometry_abs_lazy<MODE>(a.geo, n, f);
-    if (coef_not_finite(coef_d)) atomicOr(a.flags, 1u);
-    const T coef = A::from(coef_d);
-    if constexpr (MODE != kF64) {
-      if (__any_sync(__activemask(), degenerate)) {
-        if (degenerate) f = abs_geometry_fp64<T>(a.geo.xyz, n);
+    const double* t = a.stiff ? a.tables + 7 * NU : a.tables + 6 * NU;
+    for (int i = threadIdx.x; i < (a.stiff ? kBaryTerms : NU); i += blockDim.x) {
+      if constexpr (MODE == kDW) {
+        const ff v = ff_from_double_bits(t[i]);
+        tab[i] = make_float4(v.hi, v.hi, v.lo, v.lo);
+      } else {
+        const float v = A::from(t[i]);
+        tab[i] = make_float2(v, v);
       }
     }
+  }
+  __syncthreads();
+  const int64_t E = a.n_elem;
+  const int lane = threadIdx.x & 31;
+  const int64_t first = (blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5)) * 64;
+  if (first >= E) return;
+  // past the last element the pair repeats it (the same values stored again)
+  const int64_t p0 = min(first + lane, E - 1), p1 = min(first + 32 + lane, E - 1);
+  const double c0 = a.coeff ? __ldg(a.coeff + a.elem_order[p0]) : a.cconst;
+  const double c1 = a.coeff ? __ldg(a.coeff + a.elem_order[p1]) : a.cconst;
+  const auto vertices = [&](int64_t p) {
+    const int2* d = reinterpret_cast<const int2*>(a.dofs_m + p * 10);
+    const int2 x = __ldg(d), y = __ldg(d + 1);
+    return make_int4(x.x, x.y, y.x, y.y);
+  };
+  const int4 n0 = vertices(p0), n1 = vertices(p1);
+  typename Pair<MODE>::T J[3][3];
+  pair_edges<SPLIT>(GlobalNodes{a.geo}, n0, n1, J);
+  if (coef_not_finite(c0) || coef_not_finite(c1)) atomicOr(a.flags, 1u);
+  if constexpr (MODE == kDW) {
+    PairGeo f;
+    pair_cofactors(J, f);
+    if (f.degen0 || f.degen1) {  // rare: the FP64 geometry of that lane
+      const Cof<ff> x = abs_geometry_fp64<ff>(a.geo.xyz, f.degen0 ? n0 : n1), y = abs_geometry_fp64<ff>(a.geo.xyz, f.degen1 ? n1 : n0);
+      const auto pick = [&](ff2 v, ff vx, ff vy) {
+        const float2 h = f2_get(v.hi), l = f2_get(v.lo);
+        return ff2_make(f.degen0 ? vx : ff{h.x, l.x}, f.degen1 ? vy : ff{h.y, l.y});
+      };
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int r = 0; r < 3; ++r) f.C[k][r] = pick(f.C[k][r], x.c[r][k], y.c[r][k]);
+      f.det = pick(f.det, x.det, y.det);
+    }
+    const ff2 coef = ff2_make(ff_from_double_bits(c0), ff_from_double_bits(c1));
     if (a.stiff) {
-      T g[6];
-      const T sc = coef / f.det;
-      metric<T>(f, sc, g);
-      if constexpr (MODE == kDW)
-        if (!dw_scale_ok(sc) || !dw_scale_ok(g[0])) atomicOr(a.flags, 2u);
-#pragma unroll 5
-      for (int u = 0; u < NU; ++u) em_put(a.em, u * E + p, metric_dot<T>(g, tab, NU, u));
+      ff2 s = pair_quotient(coef.hi, coef.lo, f.det);
+      const float2 dh = f2_get(f.det.hi);
+      if (det_extreme(dh.x) || det_extreme(dh.y)) {  // outside the estimate's range
+        const float2 dl = f2_get(f.det.lo), ch = f2_get(coef.hi), cl = f2_get(coef.lo);
+        s = ff2_make(ff_div(ff{ch.x, cl.x}, ff{dh.x, dl.x}), ff_div(ff{ch.y, cl.y}, ff{dh.y, dl.y}));
+      }
+      ff2 g[10];
+      f2 nC[3][3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int r = 0; r < 3; ++r) nC[k][r] = -f.C[k][r].hi;
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int l = k; l < 3; ++l) {
+          const ff2 d = ff2_dot3(f.C[k], f.C[l], nC[k]);
+          g[g_index(k + 1, l + 1)] = ff2_mul(s, f2_fast_two_sum(d.hi, d.lo));
+        }
+      // G_0b from the zero sum of the gradients
+#pragma unroll
+      for (int b = 1; b < 4; ++b) g[g_index(0, b)] = ff2_neg_sum(g[g_index(1, b)], g[g_index(2, b)], g[g_index(3, b)]);
+      g[0] = ff2_neg_sum(g[1], g[2], g[3]);
+      const float2 sh = f2_get(s.hi), gh = f2_get(g[g_index(1, 1)].hi);
+      if (!dw_scale_ok(sh.x) || !dw_scale_ok(gh.x) || !dw_scale_ok(sh.y) || !dw_scale_ok(gh.y)) atomicOr(a.flags, 2u);
+      f2 ng[10];
+#pragma unroll
+      for (int i = 0; i < 10; ++i) ng[i] = -g[i].hi;
+      p2_stiffness(g, ng, tab, a.em, E, p0, p1);
     } else {
-      const T sc = coef * f.det;
-      if constexpr (MODE == kDW)
-        if (!dw_scale_ok(sc)) atomicOr(a.flags, 2u);
+      const ff2 sc = ff2_mul(coef, f.det);
+      const float2 sh = f2_get(sc.hi);
+      if (!dw_scale_ok(sh.x) || !dw_scale_ok(sh.y)) atomicOr(a.flags, 2u);
+      const f2 ns = -sc.hi;
 #pragma unroll 5
-      for (int u = 0; u < NU; ++u) em_put(a.em, u * E + p, sc * tab[6 * NU + u]);
+      for (int u = 0; u < NU; ++u) {
+        const float4 t = tab[u];
+        const f2 th = f2_make(t.x, t.y), tl = f2_make(t.z, t.w), q = sc.hi * th;
+        em_pair_put(a.em, E, u, p0, p1, f2_fast_two_sum(q, fma2(sc.hi, tl, sc.lo * th) - fma2(ns, th, q)));
+      }
+    }
+  } else {
+    f2 C[4][3];  // C_0 from the face opposite vertex 0, then the cofactor columns
+    f2 det;
+    bool degen0, degen1;
+    pair_gradients(J, C, det, degen0, degen1);
+    if (degen0 || degen1) {
+      const Cof<float> x = abs_geometry_fp64<float>(a.geo.xyz, degen0 ? n0 : n1), y = abs_geometry_fp64<float>(a.geo.xyz, degen1 ? n1 : n0);
+      const auto pick = [&](f2 v, float vx, float vy) {
+        const float2 h = f2_get(v);
+        return f2_make(degen0 ? vx : h.x, degen1 ? vy : h.y);
+      };
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int r = 0; r < 3; ++r) C[k + 1][r] = pick(C[k + 1][r], x.c[r][k], y.c[r][k]);
+      det = pick(det, x.det, y.det);
+    }
+    const f2 coef = f2_make(A::from(c0), A::from(c1));
+    if (a.stiff) {
+      const float2 dh = f2_get(det), ch = f2_get(coef);
+      const f2 s = f2_make(ch.x / dh.x, ch.y / dh.y);
+      f2 g[10];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int l = k; l < 4; ++l)
+          g[g_index(k, l)] = s * fma2(C[k][2], C[l][2], fma2(C[k][1], C[l][1], C[k][0] * C[l][0]));
+      p2_stiffness(g, g, tab, a.em, E, p0, p1);
+    } else {
+      const f2 sc = coef * det;
+#pragma unroll 5
+      for (int u = 0; u < NU; ++u) em_pair_put(a.em, E, u, p0, p1, sc * f2_make(tab[u].x, tab[u].y));
     }
   }
 }
+
+// The P2 element pass in native FP64: one thread per element, the six metric
+// coefficients contracted with the tables T^{ab} in shared memory.
+__global__ void __launch_bounds__(256, 1) k_elem_mat_f64(ElemArgs a)
+{
+  constexpr int NU = 55;
+  __shared__ double tab[7 * NU];
+  for (int i = threadIdx.x; i < 7 * NU; i += blockDim.x) tab[i] = a.tables[i];
+  __syncthreads();
+  const int64_t E = a.n_elem;
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (p >= E) return;
+  const double coef = a.coeff ? __ldg(a.coeff + a.elem_order[p]) : a.cconst;
+  const int32_t* dp = a.dofs_m + p * 10;
+  Cof<double> f;
+  geometry_f64(a.geo, make_int4(dp[0], dp[1], dp[2], dp[3]), f);
+  if (coef_not_finite(coef)) atomicOr(a.flags, 1u);
+  if (a.stiff) {
+    double g[6];
+    metric<double>(f, coef / f.det, g);
+#pragma unroll 5
+    for (int u = 0; u < NU; ++u) em_put(a.em, u * E + p, metric_dot<double>(g, tab, NU, u));
+  } else {
+    const double sc = coef * f.det;
+#pragma unroll 5
+    for (int u = 0; u < NU; ++u) em_put(a.em, u * E + p, sc * tab[6 * NU + u]);
+  }
+}
+
+// The sum of an entry's sources, two at a time: double-words in two packed accumulators
+// (the high parts error-free, the low parts and errors collected) and written as
+// one FP64 sum of the two parts; floats packed; FP64 in order.
+template <int MODE> struct SourceSum;
+template <> struct SourceSum<kDW> {
+  ff2 s{f2_make(0.0f, 0.0f), f2_make(0.0f, 0.0f)};
+  __device__ __forceinline__ void add(ff a, ff b)
+  {
+    const ff2 t = f2_two_sum(s.hi, f2_make(a.hi, b.hi));
+    s.hi = t.hi;
+    s.lo = s.lo + (t.lo + f2_make(a.lo, b.lo));
+  }
+  __device__ __forceinline__ double result() const
+  {
+    const float2 h = f2_get(s.hi), l = f2_get(s.lo);
+    const ff t = two_sum(h.x, h.y);
+    return (double)t.hi + (double)__fadd_rn(t.lo, __fadd_rn(l.x, l.y));
+  }
+};
+template <> struct SourceSum<kF32> {
+  f2 s = f2_make(0.0f, 0.0f);
+  __device__ __forceinline__ void add(float a, float b) { s = s + f2_make(a, b); }
+  __device__ __forceinline__ float result() const
+  {
+    const float2 h = f2_get(s);
+    return h.x + h.y;
+  }
+};
+template <> struct SourceSum<kF64> {
+  double s = 0.0;
+  __device__ __forceinline__ void add(double a, double b) { s = (s + a) + b; }
+  __device__ __forceinline__ double result() const { return s; }
+};
 
 // One warp per group of 32 diagonal or upper CSR entries (the slot map's
 // layout): lane l sums the sources src[o + 32 j + l] of its entry, j < L, in the
@@ -1003,6 +1226,9 @@ __global__ void __launch_bounds__(256, 1) k_elem_mat(ElemArgs a)
 // next K sources (one coalesced line per j) and the output positions load while
 // the current element-matrix values are in flight.  Padding sources
 // (kPadSource) read the zero entry `zero` past the element matrices.
+// Bound by L2: every source is a sector of its own (59 M sectors read at P2 48^3, 7.4
+// TB/s); element-major element matrices and a grid pipelined over groups measured no
+// better (256 and 448 us against 248).
 template <int MODE, int K>
 __global__ void __launch_bounds__(256) k_slot_gather(int64_t n_groups, int64_t n_upper, const int32_t* __restrict__ goff,
                                                      const int32_t* __restrict__ uslot,
@@ -1023,7 +1249,7 @@ __global__ void __launch_bounds__(256) k_slot_gather(int64_t n_groups, int64_t n
   uint32_t nxt[K];
 #pragma unroll
   for (int i = 0; i < K; ++i) nxt[i] = i < L ? __ldg(s + 32 * i) : kPadSource;
-  T v = A::zero();
+  SourceSum<MODE> sum;
   for (int32_t j = 0; j < L; j += K) {
     uint32_t idx[K];
 #pragma unroll
@@ -1034,11 +1260,10 @@ __global__ void __launch_bounds__(256) k_slot_gather(int64_t n_groups, int64_t n
 #pragma unroll
     for (int i = 0; i < K; ++i) x[i] = j + i < L ? em_get<T>(em, idx[i]) : A::zero();
 #pragma unroll
-    for (int i = 0; i < K; ++i)
-      if (j + i < L) A::sum_into(v, x[i]);
+    for (int i = 0; i < K; i += 2) sum.add(x[i], x[i + 1]);
   }
   if (live) {
-    const typename A::Out r = A::out(v);
+    const typename A::Out r = sum.result();
     values[out_a] = r;
     if (out_m != out_a) values[out_m] = r;
   }
@@ -1154,8 +1379,7 @@ __device__ __forceinline__ void stage_block_map(const BlockArgs& bm, int32_t g0,
 }
 
 // One run's sum by one lane, four sources per step, from the byte offsets `src`
-// (row j at src[32 j]) of the block's entries; rows past L read the zero entry.  The
-// rows j and j + 1 go to two accumulators as a packed pair, combined at the end.
+// (row j at src[32 j]) of the block's entries; rows past L read the zero entry.
 __device__ __forceinline__ uint32_t src_row(const uint16_t* src, int32_t j, int32_t L)
 {
   return j < L ? src[32 * j] : 4u * 10u * kElemBlock;
@@ -1165,38 +1389,23 @@ __device__ __forceinline__ float em_at(const unsigned char* em, uint32_t off)
   return *reinterpret_cast<const float*>(em + off);
 }
 template <int MODE>
+__device__ __forceinline__ typename Arith<MODE>::T em_value(const unsigned char* em, uint32_t off)
+{
+  if constexpr (MODE == kDW) return ff{em_at(em, off), em_at(em + 4 * kEmStride, off)};
+  else if constexpr (MODE == kF32) return em_at(em, off);
+  else return *reinterpret_cast<const double*>(em + 2 * off);
+}
+template <int MODE>
 __device__ __forceinline__ typename Arith<MODE>::Out run_sum(const unsigned char* em, const uint16_t* src, int32_t L)
 {
-  if constexpr (MODE == kDW) {
-    // error-free sums of the high parts, the low parts and errors collected
-    const unsigned char* em_lo = em + 4 * kEmStride;
-    ff2 s{f2_make(0.0f, 0.0f), f2_make(0.0f, 0.0f)};
-    for (int32_t j = 0; j < L; j += 4) {
-      const uint32_t i0 = src_row(src, j, L), i1 = src_row(src, j + 1, L), i2 = src_row(src, j + 2, L),
-                     i3 = src_row(src, j + 3, L);
-      const ff2 x{f2_make(em_at(em, i0), em_at(em, i1)), f2_make(em_at(em_lo, i0), em_at(em_lo, i1))};
-      const ff2 y{f2_make(em_at(em, i2), em_at(em, i3)), f2_make(em_at(em_lo, i2), em_at(em_lo, i3))};
-      const ff2 t = f2_two_sum(s.hi, x.hi), u = f2_two_sum(t.hi, y.hi);
-      s.hi = u.hi;
-      s.lo = s.lo + ((t.lo + x.lo) + (u.lo + y.lo));
-    }
-    const float2 h = f2_get(s.hi), l = f2_get(s.lo);
-    const ff t = two_sum(h.x, h.y);
-    return (double)t.hi + (double)__fadd_rn(t.lo, __fadd_rn(l.x, l.y));
-  } else if constexpr (MODE == kF32) {
-    f2 s = f2_make(0.0f, 0.0f);
-    for (int32_t j = 0; j < L; j += 4) {
-      const uint32_t i0 = src_row(src, j, L), i1 = src_row(src, j + 1, L), i2 = src_row(src, j + 2, L),
-                     i3 = src_row(src, j + 3, L);
-      s = (s + f2_make(em_at(em, i0), em_at(em, i1))) + f2_make(em_at(em, i2), em_at(em, i3));
-    }
-    const float2 h = f2_get(s);
-    return h.x + h.y;
-  } else {
-    double s = 0.0;
-    for (int32_t j = 0; j < L; ++j) s += *reinterpret_cast<const double*>(em + 2 * src[32 * j]);
-    return s;
+  SourceSum<MODE> sum;
+  for (int32_t j = 0; j < L; j += 4) {
+    const uint32_t i0 = src_row(src, j, L), i1 = src_row(src, j + 1, L), i2 = src_row(src, j + 2, L),
+                   i3 = src_row(src, j + 3, L);
+    sum.add(em_value<MODE>(em, i0), em_value<MODE>(em, i1));
+    sum.add(em_value<MODE>(em, i2), em_value<MODE>(em, i3));
   }
+  return sum.result();
 }
 
 // Phase 2 of the block assembly: each warp takes groups of 32 of the block's
@@ -1420,7 +1629,11 @@ static mg_status launch_gather_t(mg_plan* p, const ElemArgs& a, void* d_values, 
 {
   constexpr int ORDER = 2;
   const int64_t E = a.n_elem;
-  if (E > 0) k_elem_mat<MODE><<<(unsigned)((E + 255) / 256), 256, 0, st>>>(a);
+  if (E > 0) {
+    if constexpr (MODE == kF64) k_elem_mat_f64<<<(unsigned)((E + 255) / 256), 256, 0, st>>>(a);
+    else if (MODE == kDW && p->mesh->grid_split) k_elem_mat_pair<MODE, true><<<(unsigned)((E + 255) / 256), 128, 0, st>>>(a);
+    else k_elem_mat_pair<MODE, false><<<(unsigned)((E + 255) / 256), 128, 0, st>>>(a);
+  }
   MG_CUDA(cudaGetLastError());
   using Out = typename Arith<MODE>::Out;
   const unsigned blocks = (unsigned)((p->n_groups + 7) / 8);  // 8 warps (groups) per CTA

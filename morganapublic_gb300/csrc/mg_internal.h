@@ -59,6 +59,7 @@ struct RefTables {
   int order = 0, quad = 0, nb = 0, nq = 0;
   std::vector<double> stiff;  // 6 * nb * nb
   std::vector<double> mass;   // nb * nb
+  std::vector<double> bary;   // P2: coefficients of the barycentric stiffness terms (k_elem_mat_pair)
   double wsum = 0.0;
 };
 mg_status build_ref_tables(int order, int quad, RefTables* t);

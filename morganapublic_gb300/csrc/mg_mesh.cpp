@@ -174,6 +174,37 @@ mg_status build_ref_tables(int order, int quad, RefTables* t)
         }
       }
   }
+  t->bary.clear();
+  if (order == 2) {
+    // barycentric moments of the card and the coefficients of the element pass's terms
+    double one[4] = {0, 0, 0, 0}, two[4][4] = {};
+    for (int q = 0; q < nq; ++q) {
+      const double* y = &Y[3 * q];
+      const double l[4] = {1.0 - y[0] - y[1] - y[2], y[0], y[1], y[2]};
+      for (int a = 0; a < 4; ++a) {
+        one[a] += W[q] * l[a];
+        for (int b = 0; b < 4; ++b) two[a][b] += W[q] * l[a] * l[b];
+      }
+    }
+    for (int i = 0; i < 10; ++i)
+      for (int j = i; j < 10; ++j) {
+        if (j < 4) {  // (4 l_i - 1)(4 l_j - 1)
+          t->bary.push_back(16.0 * two[i][j] - 4.0 * one[i] - 4.0 * one[j] + t->wsum);
+        } else if (i < 4) {  // 4 (4 l_i - 1) l_a, 4 (4 l_i - 1) l_b
+          for (int s = 0; s < 2; ++s) {
+            const int a = kEdgePts[j - 4][s];
+            t->bary.push_back(16.0 * two[i][a] - 4.0 * one[a]);
+          }
+        } else {
+          const int a = kEdgePts[i - 4][0], b = kEdgePts[i - 4][1], c = kEdgePts[j - 4][0], d = kEdgePts[j - 4][1];
+          if (i != j) {  // 16 l_a l_c, l_a l_d, l_b l_c, l_b l_d
+            for (const double m : {two[a][c], two[a][d], two[b][c], two[b][d]}) t->bary.push_back(16.0 * m);
+          } else {
+            for (const double m : {two[a][a], 2.0 * two[a][b], two[b][b]}) t->bary.push_back(16.0 * m);
+          }
+        }
+      }
+  }
   return MG_OK;
 }
 

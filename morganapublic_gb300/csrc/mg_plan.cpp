@@ -241,7 +241,8 @@ mg_status plan_tables(mg_plan* p, int quad, const RefTables** t, const double** 
     }
   RefTables rt;
   MG_TRY(build_ref_tables(p->mesh->order, quad, &rt));
-  // device layout: unique (i <= j, sym_index order) entries, stiff[6][nu] then mass[nu]
+  // device layout: unique (i <= j, sym_index order) entries, stiff[6][nu] then mass[nu];
+  // then the barycentric coefficients (P2)
   const int nb = rt.nb, nu = nb * (nb + 1) / 2;
   std::vector<double> flat(7 * nu);
   for (int i = 0; i < nb; ++i)
@@ -250,6 +251,7 @@ mg_status plan_tables(mg_plan* p, int quad, const RefTables** t, const double** 
       for (int q = 0; q < 6; ++q) flat[q * nu + u] = rt.stiff[q * nb * nb + i * nb + j];
       flat[6 * nu + u] = rt.mass[i * nb + j];
     }
+  flat.insert(flat.end(), rt.bary.begin(), rt.bary.end());
   double* d = nullptr;
   MG_CUDA(cudaMalloc(&d, sizeof(double) * flat.size()));
   MG_CUDA(cudaMemcpy(d, flat.data(), sizeof(double) * flat.size(), cudaMemcpyHostToDevice));
