@@ -296,9 +296,10 @@ mg_status mg_assemble_host(mg_plan* plan, int32_t op, const double* h_coeff, dou
    or 1 when d_field is NULL; s_e = d_elem_scale[e] or 1 when NULL), written to
    d_b (ndof doubles).  Element vectors in double-word arithmetic (FP64-accurate
    at any scale of s and f), then one FP64 sum per dof in a fixed order:
-   deterministic, no atomics.  The first call on a plan builds the dof-to-slot
-   map (4 bytes per element-vector entry), a work buffer of 8 bytes per entry
-   and the element-geometry cache (80 bytes per element) on the device, and
+   deterministic, no atomics.  The first call on a plan builds the sums' map (P1
+   meshes whose 512-element blocks hold at most 256 nodes each: about 14 bytes per
+   element, built on the GPU; others: 4 bytes per element-vector entry and a work
+   buffer of 8) and the element-geometry cache (80 bytes per element) on the device, and
    waits for them: make that first call before capturing a CUDA graph.
    Replaces: vectorBuilder<localVectorEL3d<fnEL3dA|fnEL3dB>>::buildEpetraVector
    (src/morganaFiniteElements/traitsVectorBuilder.hpp:214-274). */

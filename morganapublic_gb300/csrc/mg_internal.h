@@ -153,6 +153,7 @@ struct mg_plan {
   int32_t* d_bnode = nullptr;
   int32_t* d_bnode_n = nullptr;     // n_blocks
   uchar4* d_elem_local = nullptr;   // n_elem
+  bool nodes_staged = false;        // every block lists its nodes
   int32_t* d_sgoff = nullptr;       // n_sgroups + 1
   int2* d_sout = nullptr;           // 32 n_sgroups
   void* d_partial = nullptr;        // n_partial slots of 8 bytes (zero at padding)
@@ -164,6 +165,14 @@ struct mg_plan {
   int32_t* d_rhs_ptr = nullptr;       // ndof + 1
   int32_t* d_rhs_slot = nullptr;      // n_elem * nb
   double* d_rhs_y = nullptr;          // n_elem * nb
+  // one-pass load vector (P1, nodes_staged; build_rhs_map): per block the positions of its
+  // element-vector entries by node (byte offsets 4 (l kElemBlock + element)), their starts
+  // per node, and each node's output (the node, or -1 - its partial slot); a shared
+  // node's partials at rhs_ptr[d] .. rhs_ptr[d + 1], ascending block
+  uint16_t* d_rhs_bpos = nullptr;     // 4 kElemBlock per block
+  uint16_t* d_rhs_bstart = nullptr;   // kStageNodes + 1 per block
+  int32_t* d_rhs_bout = nullptr;      // kStageNodes per block
+  double* d_rhs_partial = nullptr;    // one per (block, node)
   // element geometry in double-word form (built on the first call that needs it:
   // load vector, adjoint), Morton order p: det[p] and cofactor k of element p at
   // cof[k * n_elem + p] (k = 3 r + c), each (hi, lo) floats
@@ -286,6 +295,7 @@ inline bool uses_block_map(int order) { return order == 1; }
 mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int32_t* uslot, const int32_t* umirror,
                           const uint32_t* src, cudaStream_t st);
 mg_status build_block_nodes(mg_plan* p, cudaStream_t st);     // the blocks' unique nodes
+mg_status build_rhs_map(mg_plan* p, cudaStream_t st);          // the one-pass load vector's map, once per plan
 mg_status build_edges_device(mg_mesh* m, cudaStream_t st);    // edges on the GPU (mg_pattern.cu)
 // the device coordinates and node records (d_xyz, d_node_rec, d_lo_z, grid_split)
 // from the host coordinates; needs d_conn (mg_pattern.cu)

@@ -219,6 +219,10 @@ static void free_plan(mg_plan* p)
   cudaFree(p->d_rhs_ptr);
   cudaFree(p->d_rhs_slot);
   cudaFree(p->d_rhs_y);
+  cudaFree(p->d_rhs_bpos);
+  cudaFree(p->d_rhs_bstart);
+  cudaFree(p->d_rhs_bout);
+  cudaFree(p->d_rhs_partial);
   cudaFree(p->d_geo_det);
   cudaFree(p->d_geo_cof);
   cudaFree(p->d_counters);
@@ -268,7 +272,7 @@ mg_status plan_tables(mg_plan* p, int quad, const RefTables** t, const double** 
 // dof's short list sorted.
 mg_status plan_rhs_map(mg_plan* p)
 {
-  if (p->d_rhs_ptr) return MG_OK;
+  if (p->d_rhs_slot) return MG_OK;
   const mg_mesh* m = p->mesh;
   const int nb = m->nb;
   const int64_t E = m->n_elem, nd = p->ndof, pairs = E * nb;
@@ -296,7 +300,7 @@ mg_status plan_rhs_map(mg_plan* p)
   }
 #pragma omp parallel for schedule(dynamic, 1024)
   for (int64_t d = 0; d < nd; ++d) std::sort(slot.begin() + ptr[d], slot.begin() + ptr[d + 1]);
-  // all three buffers or none (the map counts as built once d_rhs_ptr is set)
+  // all three buffers or none (the map counts as built once d_rhs_slot is set)
   int32_t *d_ptr = nullptr, *d_slot = nullptr;
   double* d_y = nullptr;
   mg_status st = upload(&d_ptr, ptr);

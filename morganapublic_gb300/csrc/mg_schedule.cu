@@ -687,7 +687,7 @@ mg_status build_slot_map(mg_plan* p, cudaStream_t st)
 // the run's rank the local number of its vertices.
 __global__ void __launch_bounds__(256) k_block_nodes(int64_t E, const int32_t* __restrict__ dofs_m,
                                                      int32_t* __restrict__ bnode, int32_t* __restrict__ bnode_n,
-                                                     uchar4* __restrict__ elem_local)
+                                                     uchar4* __restrict__ elem_local, uint32_t* __restrict__ unstaged)
 {
   constexpr int ITEMS = 4 * kElemBlock / 256;
   using Sort = cub::BlockRadixSort<uint32_t, 256, ITEMS, uint16_t>;
@@ -721,7 +721,10 @@ __global__ void __launch_bounds__(256) k_block_nodes(int64_t E, const int32_t* _
   Scan(sh.scan).InclusiveSum(head, rank, total);
   __syncthreads();
   const bool fits = total <= kStageNodes;
-  if (t == 0) bnode_n[blockIdx.x] = fits ? total : -1;
+  if (t == 0) {
+    bnode_n[blockIdx.x] = fits ? total : -1;
+    if (!fits) atomicOr(unstaged, 1u);
+  }
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) {
     if (head[i] && rank[i] <= kStageNodes) {
@@ -749,12 +752,131 @@ mg_status build_block_nodes(mg_plan* p, cudaStream_t st)
   MG_TRY(B.alloc(&bnode, nblk * kStageNodes));
   MG_TRY(B.alloc(&bnode_n, nblk));
   MG_TRY(B.alloc(&local, E));
-  k_block_nodes<<<(unsigned)nblk, 256, 0, st>>>(E, p->d_dofs_morton, bnode, bnode_n, local);
+  k_block_nodes<<<(unsigned)nblk, 256, 0, st>>>(E, p->d_dofs_morton, bnode, bnode_n, local, p->d_counters + 5);
   MG_CUDA(cudaGetLastError());
   p->d_bnode = bnode;
   p->d_bnode_n = bnode_n;
   p->d_elem_local = local;
   for (void* q : {(void*)bnode, (void*)bnode_n, (void*)local}) B.keep(q);
+  return MG_OK;
+}
+
+// ------------------------------------------------- one-pass load vector --
+// Per block: the positions of its 4 kElemBlock element-vector entries sorted by node
+// (as byte offsets 4 (l kElemBlock + element)), the first one of each of its nodes, and a
+// record (node, block kStageNodes + rank) per node for the global sort.
+__global__ void __launch_bounds__(256) k_rhs_runs(int64_t E, const int32_t* __restrict__ dofs_m,
+                                                  uint16_t* __restrict__ bpos, uint16_t* __restrict__ bstart,
+                                                  uint32_t* __restrict__ key, uint32_t* __restrict__ val)
+{
+  constexpr int ITEMS = 4 * kElemBlock / 256;
+  using Sort = cub::BlockRadixSort<uint32_t, 256, ITEMS, uint16_t>;
+  using Scan = cub::BlockScan<int, 256>;
+  __shared__ union {
+    typename Sort::TempStorage sort;
+    typename Scan::TempStorage scan;
+  } sh;
+  __shared__ uint32_t last[256];
+  const int64_t q0 = (int64_t)blockIdx.x * 4 * kElemBlock, r0 = (int64_t)blockIdx.x * kStageNodes;
+  const int t = threadIdx.x;
+  uint32_t k[ITEMS];
+  uint16_t pos[ITEMS];
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const int q = t * ITEMS + i;
+    k[i] = q0 + q < 4 * E ? (uint32_t)dofs_m[q0 + q] : 0xffffffffu;
+    pos[i] = (uint16_t)(4 * ((q & 3) * kElemBlock + (q >> 2)));
+  }
+  key[r0 + t] = 0xffffffffu;  // empty ranks
+  val[r0 + t] = (uint32_t)(r0 + t);
+  Sort(sh.sort).Sort(k, pos);
+  last[t] = k[ITEMS - 1];
+  __syncthreads();
+  int head[ITEMS], rank[ITEMS], total = 0;
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const bool first = i == 0 && t == 0;
+    const uint32_t prev = i > 0 ? k[i > 0 ? i - 1 : 0] : (t > 0 ? last[t > 0 ? t - 1 : 0] : 0u);
+    head[i] = k[i] != 0xffffffffu && (first || prev != k[i]) ? 1 : 0;
+  }
+  Scan(sh.scan).InclusiveSum(head, rank, total);
+  __syncthreads();  // the empty records before the nodes'
+  uint16_t* start = bstart + (int64_t)blockIdx.x * (kStageNodes + 1);
+  int valid = 0;
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const int q = t * ITEMS + i;
+    bpos[q0 + q] = pos[i];
+    if (head[i]) {
+      start[rank[i] - 1] = (uint16_t)q;
+      key[r0 + rank[i] - 1] = k[i];
+    }
+    valid += k[i] != 0xffffffffu ? 1 : 0;
+  }
+  // the entries end where the padding of the last block begins
+  __shared__ int n_valid;
+  if (t == 0) n_valid = 0;
+  __syncthreads();
+  atomicAdd(&n_valid, valid);
+  __syncthreads();
+  for (int r = total + t; r <= kStageNodes; r += 256) start[r] = (uint16_t)n_valid;
+}
+
+// ptr[d] = first record of node d, d = 0 .. nd (records sorted by node, the empty ones last)
+__global__ void k_rhs_ptr(int64_t n, const uint32_t* __restrict__ key, int64_t nd, int32_t* __restrict__ ptr)
+{
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t > n) return;
+  const int64_t lo = t == 0 ? 0 : min((int64_t)key[t - 1], nd) + 1;
+  const int64_t hi = t == n ? nd : min((int64_t)key[t], nd);
+  for (int64_t d = lo; d <= hi; ++d) ptr[d] = (int32_t)t;
+}
+
+__global__ void k_rhs_out(int64_t n, const uint32_t* __restrict__ key, const uint32_t* __restrict__ val, int64_t nd,
+                          const int32_t* __restrict__ ptr, int32_t* __restrict__ bout)
+{
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int64_t d = key[t];
+  if (d >= nd) bout[val[t]] = 0;  // no node: not written
+  else bout[val[t]] = ptr[d + 1] - ptr[d] == 1 ? (int32_t)d : (int32_t)(-1 - t);
+}
+
+mg_status build_rhs_map(mg_plan* p, cudaStream_t st)
+{
+  if (p->d_rhs_bpos) return MG_OK;
+  const int64_t E = p->mesh->n_elem, nd = p->ndof, nblk = p->n_blocks, n = nblk * kStageNodes;
+  if (n >= INT32_MAX) return set_error(MG_ERR_SIZE, "load-vector map: too many element blocks");
+  SchedBuffers B;
+  uint16_t *bpos, *bstart;
+  int32_t *bout, *ptr;
+  uint32_t *key, *key_s, *val, *val_s;
+  double* partial;
+  MG_TRY(B.alloc(&bpos, nblk * 4 * kElemBlock));
+  MG_TRY(B.alloc(&bstart, nblk * (kStageNodes + 1)));
+  MG_TRY(B.alloc(&bout, n));
+  MG_TRY(B.alloc(&ptr, nd + 1));
+  MG_TRY(B.alloc(&partial, n));
+  MG_TRY(B.alloc(&key, n));
+  MG_TRY(B.alloc(&key_s, n));
+  MG_TRY(B.alloc(&val, n));
+  MG_TRY(B.alloc(&val_s, n));
+  size_t tb = 0;
+  MG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, key, key_s, val, val_s, (int)n, 0, 32, st));
+  unsigned char* tmp;
+  MG_TRY(B.alloc(&tmp, (int64_t)std::max(tb, (size_t)1)));
+  k_rhs_runs<<<(unsigned)nblk, 256, 0, st>>>(E, p->d_dofs_morton, bpos, bstart, key, val);
+  MG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, key, key_s, val, val_s, (int)n, 0, 32, st));
+  k_rhs_ptr<<<grid_of(n + 1), 256, 0, st>>>(n, key_s, nd, ptr);
+  k_rhs_out<<<grid_of(n), 256, 0, st>>>(n, key_s, val_s, nd, ptr, bout);
+  MG_CUDA(cudaGetLastError());
+  MG_CUDA(cudaStreamSynchronize(st));
+  p->d_rhs_bstart = bstart;
+  p->d_rhs_bout = bout;
+  p->d_rhs_ptr = ptr;
+  p->d_rhs_partial = partial;
+  p->d_rhs_bpos = bpos;
+  for (void* q : {(void*)bpos, (void*)bstart, (void*)bout, (void*)ptr, (void*)partial}) B.keep(q);
   return MG_OK;
 }
 
@@ -873,7 +995,10 @@ mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int3
                                                       umirror, nrun, srank, sgoff, bgoff, bsrc, bout);
   k_bgrp<<<grid_of(nblk + 1), 256, 0, st>>>(nblk, seg_g, bgoff, bgrp, bsrc0);
   MG_CUDA(cudaGetLastError());
+  uint32_t unstaged = 0;  // from k_block_nodes
+  MG_CUDA(cudaMemcpyAsync(&unstaged, p->d_counters + 5, sizeof(unstaged), cudaMemcpyDeviceToHost, st));
   MG_CUDA(cudaStreamSynchronize(st));
+  p->nodes_staged = unstaged == 0;
   p->d_bgrp = bgrp;
   p->d_bsrc0 = bsrc0;
   p->d_bgoff = bgoff;
