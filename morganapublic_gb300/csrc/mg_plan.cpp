@@ -325,7 +325,6 @@ mg_status plan_work(mg_plan* p, size_t bytes, void** ptr)
 {
   if (p->work_bytes < bytes) {
     cudaFree(p->d_work);
-  for (RowPartition& rp : p->cg_part) cudaFree(rp.d_rows);
     p->d_work = nullptr;
     p->work_bytes = 0;
     MG_CUDA(cudaMalloc(&p->d_work, bytes));

@@ -78,3 +78,17 @@ def test_resident_mixed_precision(n, order):
     assert info.converged and info.rel_residual <= 1e-11
     assert float((rhs - b.apply(A, x)).norm() / rhs.norm()) <= 1.5e-11
     assert float((x - u).norm() / u.norm()) <= 1e-7
+
+
+def test_partition_outlives_a_larger_work_buffer():
+    # the mixed-precision solve needs a larger work buffer than the FP64 one before it
+    import torch
+    b, kappa, mask, A, u = _system(9, 1, 1.0, 5)
+    A32 = b.assemble("stiff_kappa", coeff=kappa, quad=4, prec="f32")
+    b.apply_dirichlet(A32, torch.from_numpy(mask))
+    rhs = b.apply(A, u)
+    x, _ = b.cg(A, rhs, rtol=1e-10)
+    b.cg_refined(A, A32, rhs, rtol=1e-10)
+    filler = [torch.full((64,), 2**30, dtype=torch.int32, device="cuda") for _ in range(64)]
+    y, _ = b.cg(A, rhs, rtol=1e-10)
+    assert bool((x == y).all()) and len(filler) == 64
