@@ -83,6 +83,7 @@ struct mg_mesh {
   void* edge_stream = nullptr;
   int64_t n_nodes = 0, n_elem = 0, n_edges = -1, ndof = 0;
   double min_det = 0.0;
+  double box_lo[3] = {}, box_hi[3] = {};  // of the node coordinates
   std::vector<double> xyz;          // n_nodes * 3
   std::vector<int32_t> conn;        // n_elem * 4
   std::vector<int32_t> elem_edge;   // n_elem * 6 (when built)
@@ -259,17 +260,18 @@ mg_status plan_device(mg_plan* p);  // uploads mesh + plan on first GPU use
 mg_status plan_tables(mg_plan* p, int quad, const RefTables** t, const double** d_tab);
 mg_status plan_work(mg_plan* p, size_t bytes, void** ptr);
 mg_status plan_rhs_map(mg_plan* p);  // the load-vector slot map (once per plan)
+class DeviceScratch;  // a build's temporary device memory (mg_scratch.h)
 // CSR pattern on the GPU (mg_pattern.cu); keep_device: its device arrays become
 // the plan's d_rowptr / d_colind
-mg_status build_pattern_device(mg_plan* p, cudaStream_t st, bool keep_device);
+mg_status build_pattern_device(mg_plan* p, DeviceScratch& scratch, cudaStream_t st, bool keep_device);
 // the plan's device state from its device pattern (mg_schedule.cu): the same
 // arrays plan_device makes for a host-built plan, the assembly's map included
 // (on_device)
-mg_status build_plan_device(mg_plan* p, cudaStream_t st);
+mg_status build_plan_device(mg_plan* p, DeviceScratch& scratch, cudaStream_t st);
 // the assembly's map from the plan's device pattern and Morton dofs
 // (mg_schedule.cu), once per plan: the per-entry source lists, laid out as the
 // block map (P1) or the gather's slot map (P2)
-mg_status build_slot_map(mg_plan* p, cudaStream_t st);
+mg_status build_slot_map(mg_plan* p, DeviceScratch& scratch, cudaStream_t st);
 bool slot_map_aos(int order);  // element-matrix layout: element-major (true) or entry-major
 // padding source of the gather layout; the kernel maps it to the zero entry past
 // the element matrices
@@ -293,8 +295,8 @@ inline bool uses_block_map(int order) { return order == 1; }
 // the block map from the per-entry source lists of the slot map (P1 layout,
 // p nu + u, ascending p): see mg_plan::d_bgrp
 mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int32_t* uslot, const int32_t* umirror,
-                          const uint32_t* src, cudaStream_t st);
-mg_status build_block_nodes(mg_plan* p, cudaStream_t st);     // the blocks' unique nodes
+                          const uint32_t* src, DeviceScratch& scratch, cudaStream_t st);
+mg_status build_block_nodes(mg_plan* p, DeviceScratch& scratch, cudaStream_t st);  // the blocks' unique nodes
 mg_status build_rhs_map(mg_plan* p, cudaStream_t st);          // the one-pass load vector's map, once per plan
 mg_status build_edges_device(mg_mesh* m, cudaStream_t st);    // edges on the GPU (mg_pattern.cu)
 // the device coordinates and node records (d_xyz, d_node_rec, d_lo_z, grid_split)

@@ -359,11 +359,18 @@ static mg_status finish_mesh(mg_mesh* m)
             return set_error(MG_ERR_BAD_MESH, "element " + std::to_string(e) + " repeats a node");
       }
     }
-  // finite coordinates (a NaN would also slip through the minimum below)
+  // finite coordinates (a NaN would also slip through the minimum below), and their box
   int nonfinite = 0;
-#pragma omp parallel for reduction(max : nonfinite)
-  for (int64_t i = 0; i < 3 * N; ++i)
-    if (!std::isfinite(m->xyz[i])) nonfinite = 1;
+  double lo0 = INFINITY, lo1 = INFINITY, lo2 = INFINITY, hi0 = -INFINITY, hi1 = -INFINITY, hi2 = -INFINITY;
+#pragma omp parallel for reduction(max : nonfinite, hi0, hi1, hi2) reduction(min : lo0, lo1, lo2)
+  for (int64_t i = 0; i < N; ++i) {
+    const double x = m->xyz[3 * i], y = m->xyz[3 * i + 1], z = m->xyz[3 * i + 2];
+    if (!std::isfinite(x) || !std::isfinite(y) || !std::isfinite(z)) nonfinite = 1;
+    lo0 = std::min(lo0, x), lo1 = std::min(lo1, y), lo2 = std::min(lo2, z);
+    hi0 = std::max(hi0, x), hi1 = std::max(hi1, y), hi2 = std::max(hi2, z);
+  }
+  m->box_lo[0] = lo0, m->box_lo[1] = lo1, m->box_lo[2] = lo2;
+  m->box_hi[0] = hi0, m->box_hi[1] = hi1, m->box_hi[2] = hi2;
   if (nonfinite)
     for (int64_t i = 0; i < 3 * N; ++i)
       if (!std::isfinite(m->xyz[i]))

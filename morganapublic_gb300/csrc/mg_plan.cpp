@@ -20,6 +20,7 @@
 #include <parallel/algorithm>
 
 #include "mg_internal.h"
+#include "mg_scratch.h"
 
 namespace mg {
 
@@ -109,13 +110,8 @@ static mg_status build_pattern(mg_plan* p)
 static mg_status build_elem_order(mg_plan* p)
 {
   mg_mesh* m = p->mesh;
-  const int64_t E = m->n_elem, N = m->n_nodes;
-  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (int64_t i = 0; i < N; ++i)
-    for (int k = 0; k < 3; ++k) {
-      lo[k] = std::min(lo[k], m->xyz[3 * i + k]);
-      hi[k] = std::max(hi[k], m->xyz[3 * i + k]);
-    }
+  const int64_t E = m->n_elem;
+  const double *lo = m->box_lo, *hi = m->box_hi;
   std::vector<std::pair<uint64_t, int32_t>> kv(E);
 #pragma omp parallel for
   for (int64_t e = 0; e < E; ++e) {
@@ -186,7 +182,8 @@ mg_status plan_device(mg_plan* p)
   }
   MG_TRY(upload(&p->d_counters, std::vector<uint32_t>(8, 0u)));
   MG_CUDA(cudaMallocHost(&p->h_pinned, 64 * sizeof(double)));
-  MG_TRY(build_slot_map(p, cudaStreamLegacy));
+  DeviceScratch scratch;
+  MG_TRY(build_slot_map(p, scratch, cudaStreamLegacy));
   p->on_device = true;
   return MG_OK;
 }
@@ -364,8 +361,9 @@ mg_status mg_pattern_build_device(mg_mesh* mesh, mg_plan** out, void* stream)
   *out = nullptr;
   mg_plan* p = new mg_plan();
   p->mesh = mesh;
-  mg_status s = build_pattern_device(p, (cudaStream_t)stream, true);
-  if (s == MG_OK) s = build_plan_device(p, (cudaStream_t)stream);
+  DeviceScratch scratch;
+  mg_status s = build_pattern_device(p, scratch, (cudaStream_t)stream, true);
+  if (s == MG_OK) s = build_plan_device(p, scratch, (cudaStream_t)stream);
   if (s != MG_OK) {
     free_plan(p);
     return s;

@@ -14,6 +14,7 @@
 #include <cub/cub.cuh>
 
 #include "mg_internal.h"
+#include "mg_scratch.h"
 
 namespace mg {
 
@@ -98,27 +99,6 @@ __global__ void k_diag_coloff(int64_t nd, const int32_t* __restrict__ rowptr, co
   }
 }
 
-// Device buffers of one plan build, freed on every exit path unless handed
-// to the plan.
-struct SchedBuffers {
-  std::vector<void*> ptrs;
-  template <typename T>
-  mg_status alloc(T** p, int64_t n)
-  {
-    void* q = nullptr;
-    const cudaError_t e = cudaMalloc(&q, sizeof(T) * (size_t)std::max<int64_t>(n, 1));
-    if (e != cudaSuccess) return cuda_error(e, "device plan buffer");
-    ptrs.push_back(q);
-    *p = static_cast<T*>(q);
-    return MG_OK;
-  }
-  void keep(void* q) { ptrs.erase(std::remove(ptrs.begin(), ptrs.end(), q), ptrs.end()); }
-  ~SchedBuffers()
-  {
-    for (void* q : ptrs) cudaFree(q);
-  }
-};
-
 int grid_of(int64_t n) { return (int)std::max<int64_t>(1, (n + 255) / 256); }
 
 template <typename T>
@@ -129,7 +109,7 @@ mg_status download(std::vector<T>& h, const T* d, int64_t n, cudaStream_t st)
   return MG_OK;
 }
 template <typename T>
-mg_status upload_to(SchedBuffers& B, T** d, const std::vector<T>& h, cudaStream_t st)
+mg_status upload_to(BuildBuffers& B, T** d, const std::vector<T>& h, cudaStream_t st)
 {
   MG_TRY(B.alloc(d, (int64_t)h.size()));
   if (!h.empty()) MG_CUDA(cudaMemcpyAsync(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, st));
@@ -515,12 +495,12 @@ __global__ void k_bgrp(int64_t nblk, const int32_t* __restrict__ seg_g, const in
 }
 
 template <typename In, typename Out>
-mg_status exclusive_scan(SchedBuffers& B, const In* in, Out* out, int64_t n, cudaStream_t st)
+mg_status exclusive_scan(BuildBuffers& B, const In* in, Out* out, int64_t n, cudaStream_t st)
 {
   size_t tb = 0;
   MG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, in, out, (int)n, st));
   unsigned char* tmp;
-  MG_TRY(B.alloc(&tmp, (int64_t)std::max(tb, (size_t)1)));
+  MG_TRY(B.temp(&tmp, (int64_t)std::max(tb, (size_t)1)));
   MG_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, in, out, (int)n, st));
   return MG_OK;
 }
@@ -534,11 +514,11 @@ mg_status read_back(T* h, const T* d, cudaStream_t st)
 }
 
 // 64-bit offsets narrowed to the plan's 32-bit layout, checked
-mg_status narrow_offsets(SchedBuffers& B, const int32_t* len, int64_t n, int32_t** out, int64_t* total,
+mg_status narrow_offsets(BuildBuffers& B, const int32_t* len, int64_t n, int32_t** out, int64_t* total,
                          const char* what, cudaStream_t st)
 {
   int64_t* off64;
-  MG_TRY(B.alloc(&off64, n + 1));
+  MG_TRY(B.temp(&off64, n + 1));
   MG_TRY(exclusive_scan(B, len, off64, n + 1, st));
   MG_TRY(read_back(total, off64 + n, st));
   if (*total >= INT32_MAX) return set_error(MG_ERR_SIZE, std::string(what) + " above 2^31 entries");
@@ -554,7 +534,7 @@ mg_status narrow_offsets(SchedBuffers& B, const int32_t* len, int64_t n, int32_t
 // element-matrix layout of the gather assembly: element-major for P1
 bool slot_map_aos(int order) { return order == 1; }
 
-mg_status build_slot_map(mg_plan* p, cudaStream_t st)
+mg_status build_slot_map(mg_plan* p, DeviceScratch& scratch, cudaStream_t st)
 {
   const mg_mesh* m = p->mesh;
   const int nb = m->nb;
@@ -562,20 +542,20 @@ mg_status build_slot_map(mg_plan* p, cudaStream_t st)
   if (n * nb >= INT32_MAX) return set_error(MG_ERR_SIZE, "slot map above 2^31 contributions");
   if ((int64_t)nunique(m->order) * E >= (int64_t)INT32_MAX)
     return set_error(MG_ERR_SIZE, "element matrices above 2^31 entries");
-  SchedBuffers B;
+  BuildBuffers B(scratch);
   int32_t *inc_ptr, *cur, *nup, *ncon, *up_first, *src_first;
   uint32_t *keys, *vin, *vout;
   int* bad;
-  MG_TRY(B.alloc(&inc_ptr, nd + 1));
-  MG_TRY(B.alloc(&cur, nnz));
-  MG_TRY(B.alloc(&nup, nd + 1));
-  MG_TRY(B.alloc(&ncon, nd + 1));
-  MG_TRY(B.alloc(&up_first, nd + 1));
-  MG_TRY(B.alloc(&src_first, nd + 1));
-  MG_TRY(B.alloc(&keys, n));
-  MG_TRY(B.alloc(&vin, n));
-  MG_TRY(B.alloc(&vout, n));
-  MG_TRY(B.alloc(&bad, 1));
+  MG_TRY(B.temp(&inc_ptr, nd + 1));
+  MG_TRY(B.temp(&cur, nnz));
+  MG_TRY(B.temp(&nup, nd + 1));
+  MG_TRY(B.temp(&ncon, nd + 1));
+  MG_TRY(B.temp(&up_first, nd + 1));
+  MG_TRY(B.temp(&src_first, nd + 1));
+  MG_TRY(B.temp(&keys, n));
+  MG_TRY(B.temp(&vin, n));
+  MG_TRY(B.temp(&vout, n));
+  MG_TRY(B.temp(&bad, 1));
   MG_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), st));
   int kbits = 1;
   while ((1ll << kbits) <= nd) ++kbits;
@@ -584,7 +564,7 @@ mg_status build_slot_map(mg_plan* p, cudaStream_t st)
   const uint32_t* kin = reinterpret_cast<const uint32_t*>(p->d_dofs_morton);
   MG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, kin, keys, vin, vout, (int)n, 0, kbits, st));
   MG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb2, nup, up_first, (int)(nd + 1), st));
-  MG_TRY(B.alloc(&tmp, (int64_t)std::max(tb, tb2)));
+  MG_TRY(B.temp(&tmp, (int64_t)std::max(tb, tb2)));
   tb = std::max(tb, tb2);
   k_iota32<<<grid_of(n), 256, 0, st>>>(n, vin);
   MG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, kin, keys, vin, vout, (int)n, 0, kbits, st));
@@ -602,11 +582,11 @@ mg_status build_slot_map(mg_plan* p, cudaStream_t st)
   const int64_t U = tot[0], C = tot[1];
   int32_t *useg, *uslot, *umirror, *urow;
   uint32_t* src;
-  MG_TRY(B.alloc(&useg, U + 1));
-  MG_TRY(B.alloc(&uslot, U));
-  MG_TRY(B.alloc(&umirror, U));
-  MG_TRY(B.alloc(&urow, U));
-  MG_TRY(B.alloc(&src, C));
+  MG_TRY(B.temp(&useg, U + 1));
+  MG_TRY(B.temp(&uslot, U));
+  MG_TRY(B.temp(&umirror, U));
+  MG_TRY(B.temp(&urow, U));
+  MG_TRY(B.temp(&src, C));
   k_slot_map<<<grid_of(nd), 256, 0, st>>>(nd, nb, E, slot_map_aos(m->order) ? 1 : 0, inc_ptr, vout,
                                            p->d_dofs_morton, p->d_rowptr, p->d_colind, up_first, src_first, cur, useg,
                                            uslot, umirror, urow, src, bad);
@@ -619,8 +599,8 @@ mg_status build_slot_map(mg_plan* p, cudaStream_t st)
   if (hbad) return set_error(MG_ERR_INVALID_ARG, "slot map: an element coupling is missing from the plan's pattern");
   if (uses_block_map(m->order)) {
     // one-pass assembly: the per-entry lists become the block map
-    MG_TRY(build_block_nodes(p, st));
-    MG_TRY(build_block_map(p, U, useg, uslot, umirror, src, st));
+    MG_TRY(build_block_nodes(p, scratch, st));
+    MG_TRY(build_block_map(p, U, useg, uslot, umirror, src, scratch, st));
     p->n_upper = U;
     p->n_slot_contrib = C;
     return MG_OK;
@@ -629,22 +609,22 @@ mg_status build_slot_map(mg_plan* p, cudaStream_t st)
   const int64_t G = (U + 31) / 32;
   int32_t *glen, *goff, *gslot, *gmirror, *d_ndiag;
   uint32_t *gkey, *gkey2, *gid, *perm, *gsrc;
-  MG_TRY(B.alloc(&gkey, U));
-  MG_TRY(B.alloc(&gkey2, U));
-  MG_TRY(B.alloc(&gid, U));
-  MG_TRY(B.alloc(&perm, U));
-  MG_TRY(B.alloc(&glen, G + 1));
+  MG_TRY(B.temp(&gkey, U));
+  MG_TRY(B.temp(&gkey2, U));
+  MG_TRY(B.temp(&gid, U));
+  MG_TRY(B.temp(&perm, U));
+  MG_TRY(B.temp(&glen, G + 1));
   MG_TRY(B.alloc(&goff, G + 1));
   MG_TRY(B.alloc(&gslot, U));
   MG_TRY(B.alloc(&gmirror, U));
-  MG_TRY(B.alloc(&d_ndiag, 1));
+  MG_TRY(B.temp(&d_ndiag, 1));
   MG_CUDA(cudaMemsetAsync(d_ndiag, 0, sizeof(int32_t), st));
   int gbits = 1;
   while ((1ll << gbits) <= 2 * (nd / kGatherRowBlock + 1)) ++gbits;
   size_t tb3 = 0;
   MG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb3, gkey, gkey2, gid, perm, (int)U, 0, gbits, st));
   unsigned char* tmp3;
-  MG_TRY(B.alloc(&tmp3, (int64_t)std::max(tb3, (size_t)1)));
+  MG_TRY(B.temp(&tmp3, (int64_t)std::max(tb3, (size_t)1)));
   if (U > 0) k_group_keys<<<grid_of(U), 256, 0, st>>>(U, urow, uslot, umirror, gkey, gid, d_ndiag);
   MG_CUDA(cub::DeviceRadixSort::SortPairs(tmp3, tb3, gkey, gkey2, gid, perm, (int)U, 0, gbits, st));
   int32_t ndiag = 0;
@@ -652,11 +632,11 @@ mg_status build_slot_map(mg_plan* p, cudaStream_t st)
   k_group_len<<<grid_of(G + 1), 256, 0, st>>>(G, U, perm, useg, glen);
   // group offsets summed in 64 bits, checked against the 32-bit layout
   int64_t* goff64;
-  MG_TRY(B.alloc(&goff64, G + 1));
+  MG_TRY(B.temp(&goff64, G + 1));
   size_t tb4 = 0;
   MG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb4, glen, goff64, (int)(G + 1), st));
   unsigned char* tmp4;
-  MG_TRY(B.alloc(&tmp4, (int64_t)std::max(tb4, (size_t)1)));
+  MG_TRY(B.temp(&tmp4, (int64_t)std::max(tb4, (size_t)1)));
   MG_CUDA(cub::DeviceScan::ExclusiveSum(tmp4, tb4, glen, goff64, (int)(G + 1), st));
   int64_t S = 0;
   MG_CUDA(cudaMemcpyAsync(&S, goff64 + G, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -743,10 +723,10 @@ __global__ void __launch_bounds__(256) k_block_nodes(int64_t E, const int32_t* _
   }
 }
 
-mg_status build_block_nodes(mg_plan* p, cudaStream_t st)
+mg_status build_block_nodes(mg_plan* p, DeviceScratch& scratch, cudaStream_t st)
 {
   const int64_t E = p->mesh->n_elem, nblk = std::max<int64_t>(1, (E + kElemBlock - 1) / kElemBlock);
-  SchedBuffers B;
+  BuildBuffers B(scratch);
   int32_t *bnode, *bnode_n;
   uchar4* local;
   MG_TRY(B.alloc(&bnode, nblk * kStageNodes));
@@ -847,7 +827,8 @@ mg_status build_rhs_map(mg_plan* p, cudaStream_t st)
   if (p->d_rhs_bpos) return MG_OK;
   const int64_t E = p->mesh->n_elem, nd = p->ndof, nblk = p->n_blocks, n = nblk * kStageNodes;
   if (n >= INT32_MAX) return set_error(MG_ERR_SIZE, "load-vector map: too many element blocks");
-  SchedBuffers B;
+  DeviceScratch scratch;
+  BuildBuffers B(scratch);
   uint16_t *bpos, *bstart;
   int32_t *bout, *ptr;
   uint32_t *key, *key_s, *val, *val_s;
@@ -857,14 +838,14 @@ mg_status build_rhs_map(mg_plan* p, cudaStream_t st)
   MG_TRY(B.alloc(&bout, n));
   MG_TRY(B.alloc(&ptr, nd + 1));
   MG_TRY(B.alloc(&partial, n));
-  MG_TRY(B.alloc(&key, n));
-  MG_TRY(B.alloc(&key_s, n));
-  MG_TRY(B.alloc(&val, n));
-  MG_TRY(B.alloc(&val_s, n));
+  MG_TRY(B.temp(&key, n));
+  MG_TRY(B.temp(&key_s, n));
+  MG_TRY(B.temp(&val, n));
+  MG_TRY(B.temp(&val_s, n));
   size_t tb = 0;
   MG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, key, key_s, val, val_s, (int)n, 0, 32, st));
   unsigned char* tmp;
-  MG_TRY(B.alloc(&tmp, (int64_t)std::max(tb, (size_t)1)));
+  MG_TRY(B.temp(&tmp, (int64_t)std::max(tb, (size_t)1)));
   k_rhs_runs<<<(unsigned)nblk, 256, 0, st>>>(E, p->d_dofs_morton, bpos, bstart, key, val);
   MG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, key, key_s, val, val_s, (int)n, 0, 32, st));
   k_rhs_ptr<<<grid_of(n + 1), 256, 0, st>>>(n, key_s, nd, ptr);
@@ -893,7 +874,7 @@ mg_status build_rhs_map(mg_plan* p, cudaStream_t st)
 //      run's output;
 //   5. one thread per (group, lane): the local sources and the output.
 mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int32_t* uslot, const int32_t* umirror,
-                          const uint32_t* src, cudaStream_t st)
+                          const uint32_t* src, DeviceScratch& scratch, cudaStream_t st)
 {
   const int nu = nunique(p->mesh->order), be = elems_per_block(p->mesh->order);
   if (4 * be * nu >= UINT16_MAX) return set_error(MG_ERR_SIZE, "block map: a block's entries above 16 bits");
@@ -901,12 +882,12 @@ mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int3
   const int64_t nblk = std::max<int64_t>(1, (E + be - 1) / be);
   const int64_t nseg = nblk;
   if (64 * nblk >= UINT32_MAX / 2) return set_error(MG_ERR_SIZE, "block map: too many element blocks");
-  SchedBuffers B;
+  BuildBuffers B(scratch);
   int32_t *nrun, *shared, *rfirst, *sidx;
-  MG_TRY(B.alloc(&nrun, U + 1));
-  MG_TRY(B.alloc(&shared, U + 1));
-  MG_TRY(B.alloc(&rfirst, U + 1));
-  MG_TRY(B.alloc(&sidx, U + 1));
+  MG_TRY(B.temp(&nrun, U + 1));
+  MG_TRY(B.temp(&shared, U + 1));
+  MG_TRY(B.temp(&rfirst, U + 1));
+  MG_TRY(B.temp(&sidx, U + 1));
   k_run_count<<<grid_of(U + 1), 256, 0, st>>>(U, nu, be, useg, src, nrun, shared);
   MG_CUDA(cudaGetLastError());
   MG_TRY(exclusive_scan(B, nrun, rfirst, U + 1, st));
@@ -917,14 +898,14 @@ mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int3
   // ---- runs, sorted by (block, length); the sort is stable, so CSR order within
   uint32_t *rkey, *skey, *rid, *perm;
   int32_t *rt, *rj, *rstart, *rlen;
-  MG_TRY(B.alloc(&rkey, R));
-  MG_TRY(B.alloc(&skey, R));
-  MG_TRY(B.alloc(&rid, R));
-  MG_TRY(B.alloc(&perm, R));
-  MG_TRY(B.alloc(&rt, R));
-  MG_TRY(B.alloc(&rj, R));
-  MG_TRY(B.alloc(&rstart, R));
-  MG_TRY(B.alloc(&rlen, R));
+  MG_TRY(B.temp(&rkey, R));
+  MG_TRY(B.temp(&skey, R));
+  MG_TRY(B.temp(&rid, R));
+  MG_TRY(B.temp(&perm, R));
+  MG_TRY(B.temp(&rt, R));
+  MG_TRY(B.temp(&rj, R));
+  MG_TRY(B.temp(&rstart, R));
+  MG_TRY(B.temp(&rlen, R));
   if (U > 0)
     k_run_emit<<<grid_of(U), 256, 0, st>>>(U, nu, be, useg, src, rfirst, rkey, rid, rt, rj, rstart, rlen);
   int kbits = 1;
@@ -932,13 +913,13 @@ mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int3
   size_t tb = 0;
   MG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, rkey, skey, rid, perm, (int)R, 0, kbits, st));
   unsigned char* tmp;
-  MG_TRY(B.alloc(&tmp, (int64_t)std::max(tb, (size_t)1)));
+  MG_TRY(B.temp(&tmp, (int64_t)std::max(tb, (size_t)1)));
   MG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, rkey, skey, rid, perm, (int)R, 0, kbits, st));
   // ---- groups of 32 runs per block
   int32_t *seg_ptr, *ng, *seg_g;
-  MG_TRY(B.alloc(&seg_ptr, nseg + 1));
-  MG_TRY(B.alloc(&ng, nseg + 1));
-  MG_TRY(B.alloc(&seg_g, nseg + 1));
+  MG_TRY(B.temp(&seg_ptr, nseg + 1));
+  MG_TRY(B.temp(&ng, nseg + 1));
+  MG_TRY(B.temp(&seg_g, nseg + 1));
   k_run_starts<<<grid_of((int64_t)R + 1), 256, 0, st>>>(R, skey, nseg, seg_ptr, 6);
   k_seg_groups<<<grid_of(nseg + 1), 256, 0, st>>>(nseg, seg_ptr, ng);
   MG_CUDA(cudaGetLastError());
@@ -946,9 +927,9 @@ mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int3
   int32_t G = 0;
   MG_TRY(read_back(&G, seg_g + nseg, st));
   int32_t *grun0, *gcnt, *glen, *bgoff;
-  MG_TRY(B.alloc(&grun0, G));
-  MG_TRY(B.alloc(&gcnt, G));
-  MG_TRY(B.alloc(&glen, (int64_t)G + 1));
+  MG_TRY(B.temp(&grun0, G));
+  MG_TRY(B.temp(&gcnt, G));
+  MG_TRY(B.temp(&glen, (int64_t)G + 1));
   k_seg_fill<<<grid_of(nseg), 256, 0, st>>>(nseg, seg_ptr, seg_g, grun0, gcnt);
   k_bgroup_len<<<grid_of((int64_t)G + 1), 256, 0, st>>>(G, grun0, gcnt, perm, rlen, glen);
   MG_CUDA(cudaGetLastError());
@@ -959,19 +940,19 @@ mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int3
   int32_t *sh_csr, *sh_t, *srank, *slen, *sgoff;
   uint32_t *shk, *shk2;
   int2* sout;
-  MG_TRY(B.alloc(&sh_csr, S));
-  MG_TRY(B.alloc(&sh_t, S));
-  MG_TRY(B.alloc(&srank, U));
-  MG_TRY(B.alloc(&shk, S));
-  MG_TRY(B.alloc(&shk2, S));
-  MG_TRY(B.alloc(&slen, G3 + 1));
+  MG_TRY(B.temp(&sh_csr, S));
+  MG_TRY(B.temp(&sh_t, S));
+  MG_TRY(B.temp(&srank, U));
+  MG_TRY(B.temp(&shk, S));
+  MG_TRY(B.temp(&shk2, S));
+  MG_TRY(B.temp(&slen, G3 + 1));
   MG_TRY(B.alloc(&sout, 32 * G3));
   if (U > 0) k_shared_list<<<grid_of(U), 256, 0, st>>>(U, shared, sidx, sh_csr);
   if (S > 0) k_shared_keys<<<grid_of(S), 256, 0, st>>>(S, sh_csr, nrun, shk);
   size_t tb5 = 0;
   MG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb5, shk, shk2, sh_csr, sh_t, (int)S, 0, 6, st));
   unsigned char* tmp5;
-  MG_TRY(B.alloc(&tmp5, (int64_t)std::max(tb5, (size_t)1)));
+  MG_TRY(B.temp(&tmp5, (int64_t)std::max(tb5, (size_t)1)));
   MG_CUDA(cub::DeviceRadixSort::SortPairs(tmp5, tb5, shk, shk2, sh_csr, sh_t, (int)S, 0, 6, st));
   if (S > 0) k_shared_rank<<<grid_of(S), 256, 0, st>>>(S, sh_t, srank);
   k_sgroup_len<<<grid_of(G3 + 1), 256, 0, st>>>(G3, S, sh_t, nrun, slen);
@@ -1024,7 +1005,7 @@ mg_status build_block_map(mg_plan* p, int64_t U, const int32_t* useg, const int3
 // the dofs in that order, the diagonal entries and 16-bit column offsets, the
 // status counters and the slot map -- the arrays plan_device makes for a
 // host-built plan, from the same rules.
-mg_status build_plan_device(mg_plan* p, cudaStream_t st)
+mg_status build_plan_device(mg_plan* p, DeviceScratch& scratch, cudaStream_t st)
 {
   mg_mesh* m = p->mesh;
   const int nb = m->nb;
@@ -1032,25 +1013,20 @@ mg_status build_plan_device(mg_plan* p, cudaStream_t st)
   if (!p->d_rowptr || !p->d_colind) return set_error(MG_ERR_INVALID_ARG, "device plan: pattern not on the device");
   if (nd >= INT32_MAX / 2 || E * nb >= INT32_MAX) return set_error(MG_ERR_SIZE, "device plan: sizes above 2^30");
   MG_TRY(mesh_device(m));
-  SchedBuffers B;
+  BuildBuffers B(scratch);
   // ---- elements along the Morton curve of their centroids
   Box bx;
-  for (int k = 0; k < 3; ++k) bx.lo[k] = INFINITY, bx.hi[k] = -INFINITY;
-  for (int64_t i = 0; i < N; ++i)
-    for (int k = 0; k < 3; ++k) {
-      bx.lo[k] = std::min(bx.lo[k], m->xyz[3 * i + k]);
-      bx.hi[k] = std::max(bx.hi[k], m->xyz[3 * i + k]);
-    }
+  for (int k = 0; k < 3; ++k) bx.lo[k] = m->box_lo[k], bx.hi[k] = m->box_hi[k];
   uint64_t *ka, *kb;
   int32_t *ia, *d_elem_order;
-  MG_TRY(B.alloc(&ka, E));
-  MG_TRY(B.alloc(&kb, E));
-  MG_TRY(B.alloc(&ia, E));
+  MG_TRY(B.temp(&ka, E));
+  MG_TRY(B.temp(&kb, E));
+  MG_TRY(B.temp(&ia, E));
   MG_TRY(B.alloc(&d_elem_order, E));
   size_t tb = 0;
   MG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, ka, kb, ia, d_elem_order, (int)E, 0, 64, st));
   unsigned char* tmp;
-  MG_TRY(B.alloc(&tmp, (int64_t)tb));
+  MG_TRY(B.temp(&tmp, (int64_t)tb));
   if (E > 0) {
     k_elem_keys<<<grid_of(E), 256, 0, st>>>(E, m->d_conn, m->d_xyz, bx, ka, ia);
     MG_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, ka, kb, ia, d_elem_order, (int)E, 0, 64, st));
@@ -1064,7 +1040,7 @@ mg_status build_plan_device(mg_plan* p, cudaStream_t st)
   int* d_fits;
   MG_TRY(B.alloc(&d_diag, nd));
   MG_TRY(B.alloc(&d_coloff, p->nnz));
-  MG_TRY(B.alloc(&d_fits, 1));
+  MG_TRY(B.temp(&d_fits, 1));
   const int one = 1;
   MG_CUDA(cudaMemcpyAsync(d_fits, &one, sizeof(int), cudaMemcpyHostToDevice, st));
   if (nd > 0) k_diag_coloff<<<grid_of(nd), 256, 0, st>>>(nd, p->d_rowptr, p->d_colind, d_diag, d_coloff, d_fits);
@@ -1083,7 +1059,7 @@ mg_status build_plan_device(mg_plan* p, cudaStream_t st)
   p->d_counters = d_counters;
   for (void* q : {(void*)d_diag, (void*)d_elem_order, (void*)d_dm, (void*)d_counters}) B.keep(q);
   if (p->d_coloff) B.keep(d_coloff);
-  MG_TRY(build_slot_map(p, st));
+  MG_TRY(build_slot_map(p, scratch, st));
   p->on_device = true;
   return MG_OK;
 }

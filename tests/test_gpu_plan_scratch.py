@@ -1,0 +1,32 @@
+"""Plans built on the GPU from packed coupling keys and shared scratch against
+plans built on the host: dof counts at and around powers of two (the keys' width),
+an unstructured numbering, and the arrays that outlive the scratch."""
+import numpy as np
+import pytest
+
+from morganapublic_gb300 import meshgen
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,order", [(1, 1), (3, 1), (7, 1), (8, 1), (15, 1), (1, 2), (2, 2), (7, 2), (11, 2)])
+def test_device_plan_matches_host_plan(n, order):
+    import morganapublic_gb300 as mg
+    m = meshgen.kuhn_cube(n, jitter=0.1, seed=n, permute=True)
+    mesh = mg.Mesh(m.xyz, m.conn, order=order)
+    host = mg.MatrixBuilder(mesh)
+    built = mg.MatrixBuilder(mesh, pattern_on_device=True)
+    for a, b in zip(built.pattern(), host.pattern()):
+        assert np.array_equal(a, b)
+    assert np.array_equal(built.elem_order(), host.elem_order())
+    kappa = meshgen.lognormal(len(m.conn), 1.0, n)
+    quad = 4 if order == 1 else 11
+    want = host.assemble("stiff_kappa", coeff=kappa, quad=quad)
+    # a second plan in between takes over the memory that the first one's build gave back
+    other = mg.MatrixBuilder(mesh, pattern_on_device=True)
+    got = built.assemble("stiff_kappa", coeff=kappa, quad=quad)
+    assert bool((got == want).all())
+    maps = "export_block_map" if order == 1 else "export_slot_map"
+    a, b, c = (getattr(q, maps)() for q in (built, host, other))
+    for k in b:
+        assert np.array_equal(a[k], b[k]) and np.array_equal(c[k], b[k])
