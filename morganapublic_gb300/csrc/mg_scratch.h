@@ -2,8 +2,8 @@
 // stack order from a few large allocations, all of them freed with the object.  A
 // build makes some forty temporary arrays; as an allocation each they cost 10 us
 // to make and, because freeing one waits for the device, 10 to 300 us to give back
-// (measured, 64^3 P1 plan: 0.5 ms of allocations and 2 ms of frees, now 0.3 ms
-// together).  Every user of one scratch works on one stream, so a block that is
+// (measured, 64^3 P1 plan: 0.5 ms of allocations and 2 ms of frees; the plan's build
+// as a whole 10.2 -> 7.4 ms with packed sort keys and the box from the mesh check).  Every user of one scratch works on one stream, so a block that is
 // given back may be handed out again at once: the next use is ordered after the last.
 #pragma once
 
