@@ -238,7 +238,8 @@ struct mg_lagrange {
   int2* d_faces = nullptr;  // (element, local face)
   int32_t *d_b_rowptr = nullptr, *d_b_colind = nullptr, *d_b_src_ptr = nullptr, *d_b_src = nullptr;
   int32_t *d_s_rowptr = nullptr, *d_s_colind = nullptr, *d_s_src = nullptr;
-  double* d_face_mat = nullptr;  // n_faces * nt * nb
+  double2* d_face_area = nullptr;  // n_faces: (area2, local face)
+  double* d_face_tab = nullptr;    // per card and local face: the nt x nb matrix of a face with area2 = 1
   int32_t* d_s_diag = nullptr;
   int32_t *d_m_pair_ptr = nullptr, *d_m_slot = nullptr;
   int2* d_m_pairs = nullptr;

@@ -560,7 +560,8 @@ static void free_device(mg_lagrange* lg)
   cudaFree(lg->d_s_rowptr);
   cudaFree(lg->d_s_colind);
   cudaFree(lg->d_s_src);
-  cudaFree(lg->d_face_mat);
+  cudaFree(lg->d_face_area);
+  cudaFree(lg->d_face_tab);
   cudaFree(lg->d_s_diag);
   lg->d_s_diag = nullptr;
   cudaFree(lg->d_m_pair_ptr);
@@ -576,8 +577,26 @@ static void free_device(mg_lagrange* lg)
   lg->d_faces = nullptr;
   lg->d_b_rowptr = lg->d_b_colind = lg->d_b_src_ptr = lg->d_b_src = nullptr;
   lg->d_s_rowptr = lg->d_s_colind = lg->d_s_src = nullptr;
-  lg->d_face_mat = nullptr;
+  lg->d_face_area = nullptr;
+  lg->d_face_tab = nullptr;
   lg->on_device = false;
+}
+
+// The matrices of a face with area2 = 1, for the cards in the order of kFaceCards and
+// the four local faces.
+template <int NB, int NT>
+static void unit_face_tables(std::vector<double>& t)
+{
+  const double P[3][3] = {{0.0, 0.0, 0.0}, {1.0, 0.0, 0.0}, {0.0, 1.0, 0.0}};
+  for (const int quad : kFaceCards) {
+    FaceRule rule{};
+    face_rule(quad, &rule);
+    for (int lf = 0; lf < 4; ++lf) {
+      double mat[NT * NB];
+      face_matrix<NB, NT>(P, lf, rule, mat);
+      t.insert(t.end(), mat, mat + NT * NB);
+    }
+  }
 }
 
 mg_status lagrange_device(mg_lagrange* lg)
@@ -588,7 +607,18 @@ mg_status lagrange_device(mg_lagrange* lg)
   MG_TRY(plan_device(lg->plan));
   std::vector<int2> faces(lg->n_faces);
   for (int64_t f = 0; f < lg->n_faces; ++f) faces[f] = make_int2(lg->face_elem[f], lg->face_local[f]);
+  std::vector<double> tab;
+  if (lg->nb == 4) {
+    if (lg->nt == 3) unit_face_tables<4, 3>(tab);
+    else if (lg->nt == 1) unit_face_tables<4, 1>(tab);
+    else unit_face_tables<4, 6>(tab);
+  } else {
+    if (lg->nt == 3) unit_face_tables<10, 3>(tab);
+    else if (lg->nt == 1) unit_face_tables<10, 1>(tab);
+    else unit_face_tables<10, 6>(tab);
+  }
   mg_status s = upload(&lg->d_faces, faces);
+  if (s == MG_OK) s = upload(&lg->d_face_tab, tab);
   if (s == MG_OK) s = upload(&lg->d_b_rowptr, lg->b_rowptr);
   if (s == MG_OK) s = upload(&lg->d_b_colind, lg->b_colind);
   if (s == MG_OK) s = upload(&lg->d_b_src_ptr, lg->b_src_ptr);
@@ -604,9 +634,8 @@ mg_status lagrange_device(mg_lagrange* lg)
   if (s == MG_OK && lg->mmt) s = upload(&lg->d_p_pairs, lg->p_pairs);
   if (s == MG_OK && lg->mmt) s = upload(&lg->d_p_slot, lg->p_slot);
   if (s == MG_OK) {
-    const cudaError_t e =
-        cudaMalloc(&lg->d_face_mat, sizeof(double) * std::max<int64_t>(lg->n_faces * lg->nt * lg->nb, 1));
-    if (e != cudaSuccess) s = cuda_error(e, "cudaMalloc(face matrices)");
+    const cudaError_t e = cudaMalloc(&lg->d_face_area, sizeof(double2) * std::max<int64_t>(lg->n_faces, 1));
+    if (e != cudaSuccess) s = cuda_error(e, "cudaMalloc(face areas)");
   }
   if (s != MG_OK) {
     free_device(lg);

@@ -1,42 +1,51 @@
 // Boundary multipliers on the GPU: values of B = opLA3dA, of the saddle matrix
 // [K B^T; B 0], and the products with them.
 //
-// B is assembled in two deterministic passes:
-//   k_face_matrix  one thread per boundary face: its nt x nb local matrix
-//                  (mg_lagrange.cuh) into a staging array, face-major;
-//   k_gather_sum   one thread per entry of B: the staged values it sums, in the
-//                  reference's insertion order (element, local face, face
-//                  vertex, basis), from the host-built list of the entry.
-// No atomics, so every run gives the same bits.  The work is O(boundary faces)
-// (n^2 against the volume operator's n^3) and runs in native FP64.
+// B is assembled in two deterministic passes.  A face's local matrix is its area2 =
+// |Vx ^ Vy| times a matrix of its local face and the card alone (mg_lagrange.cuh), so
+//   k_face_area    one thread per boundary face: area2, in native FP64;
+//   k_gather_sum   one thread per entry of B: the sum of area2 times the table's entry
+//                  over the faces that the entry sums, in the reference's insertion
+//                  order (element, local face, face vertex, basis), from the
+//                  host-built list of the entry.
+// No atomics, so every run gives the same bits.  (Summing each face's local matrix at
+// its quadrature points instead cost 130 to 2000 FP64 instructions per face, on a pipe
+// that starts one per warp every 16 cycles, and 8 nt nb bytes of staging per face:
+// 41 x 47 x 35, P1: 12.9 us for B's two kernels against 6.1.)
 // The saddle values are a gather from K's and B's values through a per-entry
 // source map (plus, for setMTM / setMMT, one thread per entry of B^T B or
 // B B^T summing its products); the products with the matrices use the CSR SpMV
 // kernel of mg_solve.cu.
+// The three kernels are launched with programmatic dependence: each reads the
+// plan's lists before it waits for the kernel before it.
 #include <algorithm>
 #include <climits>
 
 #include "mg_internal.h"
 #include "mg_lagrange.cuh"
+#include "mg_launch.cuh"
 
 namespace mg {
 
 namespace {
 
-constexpr int kFaceThreads = 256;
+constexpr int kFaceThreads = 256, kAreaThreads = 128, kFillItems = 4;
 
-int grid_for(int64_t n)
+int grid_for(int64_t n, int per_cta = kFaceThreads)
 {
-  const int64_t b = (n + kFaceThreads - 1) / kFaceThreads;
+  const int64_t b = (n + per_cta - 1) / per_cta;
   return (int)std::max<int64_t>(1, std::min<int64_t>(b, 65535));
 }
 
-template <int NB, int NT>
-__global__ void __launch_bounds__(kFaceThreads) k_face_matrix(int64_t n_faces, const int2* __restrict__ faces,
-                                                          const int4* __restrict__ conn,
-                                                          const double4_32a* __restrict__ xyz, FaceRule rule,
-                                                          double* __restrict__ out)
+// Bound by the latency of three dependent loads (face, element, nodes): 128 threads
+// per CTA spread a small surface's faces over more SMs.
+__global__ void __launch_bounds__(kAreaThreads) k_face_area(int64_t n_faces, const int2* __restrict__ faces,
+                                                            const int4* __restrict__ conn,
+                                                            const double4_32a* __restrict__ xyz,
+                                                            double2* __restrict__ area)
 {
+  pdl_trigger();
+  bool waited = false;
   for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f < n_faces; f += (int64_t)gridDim.x * blockDim.x) {
     const int2 fe = faces[f];
     const int4 c = conn[fe.x];
@@ -49,39 +58,73 @@ __global__ void __launch_bounds__(kFaceThreads) k_face_matrix(int64_t n_faces, c
       P[a][1] = p.y;
       P[a][2] = p.z;
     }
-    double mat[NT * NB];
-    face_matrix<NB, NT>(P, fe.y, rule, mat);
-    double* o = out + f * (NT * NB);
-#pragma unroll
-    for (int k = 0; k < NT * NB; ++k) o[k] = mat[k];
+    const double s = face_area2(P);
+    if (!waited) pdl_wait();  // an earlier gather may still read the areas
+    waited = true;
+    area[f] = make_double2(s, (double)fe.y);
   }
+  if (!waited) pdl_wait();
 }
 
-// vals[k] = sum of src_vals[src[j]] over j in [ptr[k], ptr[k+1]), in list order
+// vals[k] = sum over j in [ptr[k], ptr[k+1]), in list order, of area2 of face src[j] / nt
+// nb times the entry src[j] % (nt nb) of its local face's table.  Bound by the latency
+// of its loads: the list's are taken four at a time and before the wait.
+template <int NTB>
 __global__ void __launch_bounds__(kFaceThreads) k_gather_sum(int64_t n, const int32_t* __restrict__ ptr,
-                                                         const int32_t* __restrict__ src,
-                                                         const double* __restrict__ src_vals,
-                                                         double* __restrict__ vals)
+                                                             const int32_t* __restrict__ src,
+                                                             const double2* area, const double* __restrict__ tab,
+                                                             double* __restrict__ vals)
 {
+  pdl_trigger();
+  bool waited = false;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
     const int32_t j1 = ptr[k + 1];
-    for (int32_t j = ptr[k]; j < j1; ++j) s += src_vals[src[j]];
+    for (int32_t j = ptr[k]; j < j1; j += 4) {
+      int32_t q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = src[min(j + i, j1 - 1)];
+      if (!waited) pdl_wait();
+      waited = true;
+      double2 a[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = area[q[i] / NTB];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (j + i < j1) s += a[i].x * tab[(int)a[i].y * NTB + q[i] % NTB];
+    }
+    if (!waited) pdl_wait();  // an earlier kernel may still read vals
+    waited = true;
     vals[k] = s;
   }
+  if (!waited) pdl_wait();
 }
 
 // Saddle entry k: K's entry src (>= 0), B's entry -(src + 1), eye_lam
-// (kSrcLamDiag) or zero (kSrcZero, a B^T B entry outside K)
+// (kSrcLamDiag) or zero (kSrcZero, a B^T B entry outside K).  Bound by the latency of
+// two dependent loads: four entries per thread, and their sources read before the wait.
 __global__ void __launch_bounds__(kFaceThreads) k_saddle_fill(int64_t n, const int32_t* __restrict__ src,
-                                                          const double* __restrict__ kv,
-                                                          const double* __restrict__ bv, double eye_lam,
+                                                          const double* kv, const double* bv, double eye_lam,
                                                           double* __restrict__ out)
 {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t s = src[k];
-    out[k] = s >= 0 ? kv[s] : (s == kSrcLamDiag ? eye_lam : (s == kSrcZero ? 0.0 : bv[-(s + 1)]));
+  pdl_trigger();
+  const int64_t step = (int64_t)gridDim.x * (kFillItems * kFaceThreads);
+  bool waited = false;
+  for (int64_t k0 = blockIdx.x * (int64_t)(kFillItems * kFaceThreads) + threadIdx.x; k0 < n; k0 += step) {
+    int32_t s[kFillItems];
+    double v[kFillItems];
+#pragma unroll
+    for (int i = 0; i < kFillItems; ++i) s[i] = k0 + i * kFaceThreads < n ? src[k0 + i * kFaceThreads] : kSrcZero;
+    if (!waited) pdl_wait();
+    waited = true;
+#pragma unroll
+    for (int i = 0; i < kFillItems; ++i)
+      v[i] = s[i] >= 0 ? kv[s[i]] : (s[i] == kSrcLamDiag ? eye_lam : (s[i] == kSrcZero ? 0.0 : bv[-(s[i] + 1)]));
+#pragma unroll
+    for (int i = 0; i < kFillItems; ++i)
+      if (k0 + i * kFaceThreads < n) out[k0 + i * kFaceThreads] = v[i];
   }
+  if (!waited) pdl_wait();
 }
 
 // Product entry m (B^T B or B B^T): scale * sum of bv[k1] bv[k2] over its
@@ -134,24 +177,26 @@ mg_status mg_lagrange_assemble(mg_lagrange* lg, int32_t quad, double* d_b_values
   MG_TRY(lagrange_device(lg));
   cudaStream_t st = (cudaStream_t)stream;
   const mg_mesh* m = lg->plan->mesh;
-  const int g = grid_for(lg->n_faces);
-  const int64_t F = lg->n_faces;
-#define MG_FACE_LAUNCH(NB_, NT_) \
-  k_face_matrix<NB_, NT_><<<g, kFaceThreads, 0, st>>>(F, lg->d_faces, m->d_conn, m->d_xyz, rule, lg->d_face_mat)
-  if (lg->nb == 4) {
-    if (lg->nt == 3) MG_FACE_LAUNCH(4, 3);
-    else if (lg->nt == 1) MG_FACE_LAUNCH(4, 1);
-    else MG_FACE_LAUNCH(4, 6);
-  } else {
-    if (lg->nt == 3) MG_FACE_LAUNCH(10, 3);
-    else if (lg->nt == 1) MG_FACE_LAUNCH(10, 1);
-    else MG_FACE_LAUNCH(10, 6);
+  const int ntb = lg->nt * lg->nb;
+  const double* tab = lg->d_face_tab;
+  for (const int card : kFaceCards) {
+    if (card == quad) break;
+    tab += 4 * ntb;
   }
-#undef MG_FACE_LAUNCH
-  MG_CUDA(cudaGetLastError());
-  k_gather_sum<<<grid_for(lg->nnz_b), kFaceThreads, 0, st>>>(lg->nnz_b, lg->d_b_src_ptr, lg->d_b_src, lg->d_face_mat,
-                                                          d_b_values);
-  MG_CUDA(cudaGetLastError());
+  MG_CUDA(launch_pdl(k_face_area, grid_for(lg->n_faces, kAreaThreads), kAreaThreads, st, lg->n_faces, lg->d_faces,
+                     m->d_conn, m->d_xyz, lg->d_face_area));
+  const auto gather = [&](auto kernel) {
+    return launch_pdl(kernel, grid_for(lg->nnz_b), kFaceThreads, st, lg->nnz_b, lg->d_b_src_ptr, lg->d_b_src,
+                      lg->d_face_area, tab, d_b_values);
+  };
+  switch (ntb) {
+    case 4: MG_CUDA(gather(k_gather_sum<4>)); break;
+    case 10: MG_CUDA(gather(k_gather_sum<10>)); break;
+    case 12: MG_CUDA(gather(k_gather_sum<12>)); break;
+    case 24: MG_CUDA(gather(k_gather_sum<24>)); break;
+    case 30: MG_CUDA(gather(k_gather_sum<30>)); break;
+    default: MG_CUDA(gather(k_gather_sum<60>)); break;
+  }
   return MG_OK;
 }
 
@@ -193,9 +238,8 @@ mg_status mg_saddle_assemble(mg_lagrange* lg, const double* d_k_values, const do
     return set_error(MG_ERR_INVALID_ARG, "mg_saddle_assemble: null argument");
   MG_TRY(lagrange_device(lg));
   cudaStream_t st = (cudaStream_t)stream;
-  k_saddle_fill<<<grid_for(lg->nnz_s), kFaceThreads, 0, st>>>(lg->nnz_s, lg->d_s_src, d_k_values, d_b_values, eye_lam,
-                                                           d_values);
-  MG_CUDA(cudaGetLastError());
+  MG_CUDA(launch_pdl(k_saddle_fill, grid_for(lg->nnz_s, kFillItems * kFaceThreads), kFaceThreads, st, lg->nnz_s,
+                     lg->d_s_src, d_k_values, d_b_values, eye_lam, d_values));
   if (eye_field != 0.0 && lg->ndof > 0) {
     k_saddle_eye<<<grid_for(lg->ndof), kFaceThreads, 0, st>>>(lg->ndof, lg->d_s_diag, eye_field, d_values);
     MG_CUDA(cudaGetLastError());

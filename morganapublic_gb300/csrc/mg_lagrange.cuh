@@ -46,6 +46,8 @@ struct FaceRule {
   double x[6], y[6], w[6];
 };
 
+constexpr int kFaceCards[4] = {1, 3, 4, 6};
+
 inline bool face_rule(int quad, FaceRule* r)
 {
   auto set = [r](int q, double x, double y, double w) { r->x[q] = x; r->y[q] = y; r->w[q] = w; };
@@ -80,11 +82,8 @@ inline bool face_rule(int quad, FaceRule* r)
   return true;
 }
 
-// Local matrix of local face lf; P[a] = coordinates of face vertex a (face
-// order), mat = NT x NB, row-major (test basis, field basis); NT = 3 (P1 test),
-// 1 (P0 test) or 6 (P2 test).
-template <int NB, int NT>
-MG_HD inline void face_matrix(const double P[3][3], int lf, const FaceRule& r, double* mat)
+// |Vx ^ Vy| of the face with vertices P[a] (face order): twice its area
+MG_HD inline double face_area2(const double P[3][3])
 {
   double vx[3], vy[3];
   for (int k = 0; k < 3; ++k) {
@@ -94,7 +93,17 @@ MG_HD inline void face_matrix(const double P[3][3], int lf, const FaceRule& r, d
   const double n0 = vx[1] * vy[2] - vx[2] * vy[1];
   const double n1 = vx[2] * vy[0] - vx[0] * vy[2];
   const double n2 = vx[0] * vy[1] - vx[1] * vy[0];
-  const double area2 = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
+  return sqrt(n0 * n0 + n1 * n1 + n2 * n2);
+}
+
+// Local matrix of local face lf; P[a] = coordinates of face vertex a (face
+// order), mat = NT x NB, row-major (test basis, field basis); NT = 3 (P1 test),
+// 1 (P0 test) or 6 (P2 test).  It is area2 times the matrix of a face with area2 = 1,
+// which depends on the local face and the card only.
+template <int NB, int NT>
+MG_HD inline void face_matrix(const double P[3][3], int lf, const FaceRule& r, double* mat)
+{
+  const double area2 = face_area2(P);
   static_assert(NT == 1 || NT == 3 || NT == 6, "P0, P1 or P2 test basis");
   for (int k = 0; k < NT * NB; ++k) mat[k] = 0.0;
   for (int q = 0; q < r.nq; ++q) {
