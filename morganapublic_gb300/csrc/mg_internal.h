@@ -235,10 +235,10 @@ struct mg_lagrange {
   std::vector<int32_t> p_pair_ptr, p_slot;
   std::vector<int2> p_pairs;
   // device copies (uploaded on first GPU use)
-  int2* d_faces = nullptr;  // (element, local face)
+  int4* d_faces = nullptr;  // the face's three nodes (face order), local face
   int32_t *d_b_rowptr = nullptr, *d_b_colind = nullptr, *d_b_src_ptr = nullptr, *d_b_src = nullptr;
   int32_t *d_s_rowptr = nullptr, *d_s_colind = nullptr, *d_s_src = nullptr;
-  double2* d_face_area = nullptr;  // n_faces: (area2, local face)
+  double2* d_face_area = nullptr;  // n_faces: area2, and the local face in the low word of y
   double* d_face_tab = nullptr;    // per card and local face: the nt x nb matrix of a face with area2 = 1
   int32_t* d_s_diag = nullptr;
   int32_t *d_m_pair_ptr = nullptr, *d_m_slot = nullptr;

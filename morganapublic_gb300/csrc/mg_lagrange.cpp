@@ -605,8 +605,12 @@ mg_status lagrange_device(mg_lagrange* lg)
   std::lock_guard<std::mutex> lock(lg->upload_mu);
   if (lg->on_device) return check_device(lg->plan->mesh->device, "the multiplier handle");
   MG_TRY(plan_device(lg->plan));
-  std::vector<int2> faces(lg->n_faces);
-  for (int64_t f = 0; f < lg->n_faces; ++f) faces[f] = make_int2(lg->face_elem[f], lg->face_local[f]);
+  std::vector<int4> faces(lg->n_faces);
+  for (int64_t f = 0; f < lg->n_faces; ++f) {
+    const int32_t* c = &lg->plan->mesh->conn[4 * (int64_t)lg->face_elem[f]];
+    const int lf = lg->face_local[f];
+    faces[f] = make_int4(c[face_vertex(lf, 0)], c[face_vertex(lf, 1)], c[face_vertex(lf, 2)], lf);
+  }
   std::vector<double> tab;
   if (lg->nb == 4) {
     if (lg->nt == 3) unit_face_tables<4, 3>(tab);

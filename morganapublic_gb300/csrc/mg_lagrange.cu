@@ -11,7 +11,7 @@
 // No atomics, so every run gives the same bits.  (Summing each face's local matrix at
 // its quadrature points instead cost 130 to 2000 FP64 instructions per face, on a pipe
 // that starts one per warp every 16 cycles, and 8 nt nb bytes of staging per face:
-// 41 x 47 x 35, P1: 12.9 us for B's two kernels against 6.1.)
+// 41 x 47 x 35, P1, B and the saddle values: 27 us against 9.)
 // The saddle values are a gather from K's and B's values through a per-entry
 // source map (plus, for setMTM / setMMT, one thread per entry of B^T B or
 // B B^T summing its products); the products with the matrices use the CSR SpMV
@@ -37,23 +37,21 @@ int grid_for(int64_t n, int per_cta = kFaceThreads)
   return (int)std::max<int64_t>(1, std::min<int64_t>(b, 65535));
 }
 
-// Bound by the latency of three dependent loads (face, element, nodes): 128 threads
-// per CTA spread a small surface's faces over more SMs.
-__global__ void __launch_bounds__(kAreaThreads) k_face_area(int64_t n_faces, const int2* __restrict__ faces,
-                                                            const int4* __restrict__ conn,
+// Bound by latency: the face's node ids, its nodes and an FP64 chain; 128 threads per
+// CTA spread a small surface's faces over more SMs.
+__global__ void __launch_bounds__(kAreaThreads) k_face_area(int64_t n_faces, const int4* __restrict__ faces,
                                                             const double4_32a* __restrict__ xyz,
                                                             double2* __restrict__ area)
 {
   pdl_trigger();
   bool waited = false;
   for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f < n_faces; f += (int64_t)gridDim.x * blockDim.x) {
-    const int2 fe = faces[f];
-    const int4 c = conn[fe.x];
-    const int v[4] = {c.x, c.y, c.z, c.w};
+    const int4 c = faces[f];
+    const int v[3] = {c.x, c.y, c.z};
     double P[3][3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const double4_32a p = xyz[v[face_vertex(fe.y, a)]];
+      const double4_32a p = xyz[v[a]];
       P[a][0] = p.x;
       P[a][1] = p.y;
       P[a][2] = p.z;
@@ -61,7 +59,7 @@ __global__ void __launch_bounds__(kAreaThreads) k_face_area(int64_t n_faces, con
     const double s = face_area2(P);
     if (!waited) pdl_wait();  // an earlier gather may still read the areas
     waited = true;
-    area[f] = make_double2(s, (double)fe.y);
+    area[f] = make_double2(s, __hiloint2double(0, c.w));
   }
   if (!waited) pdl_wait();
 }
@@ -80,18 +78,18 @@ __global__ void __launch_bounds__(kFaceThreads) k_gather_sum(int64_t n, const in
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
     const int32_t j1 = ptr[k + 1];
-    for (int32_t j = ptr[k]; j < j1; j += 4) {
-      int32_t q[4];
+    for (int32_t j = ptr[k]; j < j1; j += 2) {
+      int32_t q[2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = src[min(j + i, j1 - 1)];
+      for (int i = 0; i < 2; ++i) q[i] = src[min(j + i, j1 - 1)];
       if (!waited) pdl_wait();
       waited = true;
-      double2 a[4];
+      double2 a[2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = area[q[i] / NTB];
+      for (int i = 0; i < 2; ++i) a[i] = area[q[i] / NTB];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (j + i < j1) s += a[i].x * tab[(int)a[i].y * NTB + q[i] % NTB];
+      for (int i = 0; i < 2; ++i)
+        if (j + i < j1) s += a[i].x * tab[__double2loint(a[i].y) * NTB + q[i] % NTB];
     }
     if (!waited) pdl_wait();  // an earlier kernel may still read vals
     waited = true;
@@ -102,7 +100,8 @@ __global__ void __launch_bounds__(kFaceThreads) k_gather_sum(int64_t n, const in
 
 // Saddle entry k: K's entry src (>= 0), B's entry -(src + 1), eye_lam
 // (kSrcLamDiag) or zero (kSrcZero, a B^T B entry outside K).  Bound by the latency of
-// two dependent loads: four entries per thread, and their sources read before the wait.
+// two dependent loads: four entries per thread, and their sources read before the wait
+// (1.26 M entries: 3.2 us, with two or eight per thread 3.8 and 3.6).
 __global__ void __launch_bounds__(kFaceThreads) k_saddle_fill(int64_t n, const int32_t* __restrict__ src,
                                                           const double* kv, const double* bv, double eye_lam,
                                                           double* __restrict__ out)
@@ -184,7 +183,7 @@ mg_status mg_lagrange_assemble(mg_lagrange* lg, int32_t quad, double* d_b_values
     tab += 4 * ntb;
   }
   MG_CUDA(launch_pdl(k_face_area, grid_for(lg->n_faces, kAreaThreads), kAreaThreads, st, lg->n_faces, lg->d_faces,
-                     m->d_conn, m->d_xyz, lg->d_face_area));
+                     m->d_xyz, lg->d_face_area));
   const auto gather = [&](auto kernel) {
     return launch_pdl(kernel, grid_for(lg->nnz_b), kFaceThreads, st, lg->nnz_b, lg->d_b_src_ptr, lg->d_b_src,
                       lg->d_face_area, tab, d_b_values);
