@@ -303,6 +303,7 @@ mg_status build_edges_device(mg_mesh* m, cudaStream_t st);    // edges on the GP
 // the device coordinates and node records (d_xyz, d_node_rec, d_lo_z, grid_split)
 // from the host coordinates; needs d_conn (mg_pattern.cu)
 mg_status build_node_records(mg_mesh* m);
+constexpr int64_t kStatsFloats = 8;  // d_lo_z holds that many at least (build_node_records)
 mg_status ensure_edges(mg_mesh* m);
 mg_status launch_assemble(mg_plan* p, int op, const double* d_coeff, double c, int quad, int prec,
                           void* d_values, cudaStream_t st);

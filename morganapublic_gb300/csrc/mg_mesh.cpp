@@ -305,7 +305,7 @@ mg_status mesh_device(mg_mesh* m)
   const int64_t N = m->n_nodes, E = m->n_elem;
   MG_CUDA(cudaMalloc(&m->d_xyz, sizeof(double4_32a) * std::max<int64_t>(N, 1)));
   MG_CUDA(cudaMalloc(&m->d_node_rec, 2 * sizeof(float4) * std::max<int64_t>(N, 1)));
-  MG_CUDA(cudaMalloc(&m->d_lo_z, sizeof(float) * std::max<int64_t>(N, 1)));
+  MG_CUDA(cudaMalloc(&m->d_lo_z, sizeof(float) * std::max<int64_t>(N, kStatsFloats)));
   MG_CUDA(cudaMalloc(&m->d_conn, sizeof(int4) * std::max<int64_t>(E, 1)));
   MG_CUDA(cudaMalloc(&m->d_dofs, sizeof(int32_t) * std::max<int64_t>(E * m->nb, 1)));
   MG_CUDA(cudaMemcpy(m->d_conn, m->conn.data(), sizeof(int4) * E, cudaMemcpyHostToDevice));

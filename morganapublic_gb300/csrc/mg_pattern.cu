@@ -12,9 +12,10 @@
 // union of every element's (test dof, field dof) couplings, columns sorted,
 // explicit zeros kept -- traitsMatrixBuilder.hpp:443-544 and the insert /
 // GlobalAssemble of buildEpetraCrs, :363-441, in morganaPublic), computed as
-//   1. one 64-bit key row << 32 | col per element coupling (E nb^2 keys),
-//   2. a radix sort of the keys and removal of duplicates (CUB),
-//   3. row starts by binary search over the sorted unique keys.
+//   1. one 64-bit key (row, col) per element coupling with row < col,
+//   2. a radix sort of the keys and removal of duplicates (CUB): the upper entries;
+//      the same with row and column swapped, sorted again: the lower ones,
+//   3. row starts by binary search over both, and each entry to its place.
 // The pattern is copied to the host (the export calls and the boundary-multiplier
 // build read it there) and, for the device plan build, kept on the device.
 #include <algorithm>
@@ -161,9 +162,10 @@ mg_status build_node_records(mg_mesh* m)
   const int64_t N = m->n_nodes, E = m->n_elem;
   m->grid_split = false;
   if (N == 0) return MG_OK;
-  double* raw = nullptr;
-  MG_CUDA(cudaMalloc(&raw, sizeof(double) * (3 * N + 4)));
-  unsigned long long* stats = reinterpret_cast<unsigned long long*>(raw + 3 * N);
+  // the coordinates as they are on the host (24 bytes a node) and the statistics wait in
+  // the records' own memory (32) and in lo's (kStatsFloats at least)
+  double* raw = reinterpret_cast<double*>(m->d_node_rec);
+  unsigned long long* stats = reinterpret_cast<unsigned long long*>(m->d_lo_z);
   uint32_t* min_alt = reinterpret_cast<uint32_t*>(stats + 3);
   const cudaStream_t st = cudaStreamLegacy;
   const uint32_t inf = 0x7f800000u;
@@ -201,7 +203,6 @@ mg_status build_node_records(mg_mesh* m)
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   }
-  cudaFree(raw);
   if (e != cudaSuccess) return cuda_error(e, "node records");
   m->grid_split = g.on != 0;
   return MG_OK;
@@ -214,39 +215,87 @@ static int key_bits(int64_t n)  // bits that hold every value < n
   return b;
 }
 
-// one thread per (element, test basis j): the element's nb couplings of row dofs[j]
+// ---------------------------------------------------------------- pattern --
+// The pattern is symmetric with a diagonal entry for every dof of an element, so only
+// the couplings row < column are sorted: nb (nb - 1) / 2 keys per element, P1 6 of 16,
+// P2 45 of 100, of 2 bits(ndof) bits; the lower entries are the unique ones with the
+// words swapped, sorted again (a sixth of the keys).  Measured at 64^3 P1 (25 M
+// couplings): all of them sorted 1.4 ms, the upper ones 0.7 and the lower ones 0.25,
+// from a third of the memory (its allocation and free: 0.6 -> 0.4 ms).
+
+// one thread per (element, test basis j): its couplings with the later basis functions
 __global__ void __launch_bounds__(256) k_pattern_keys(int64_t n_elem, int nb, int col_bits, const int32_t* __restrict__ dofs,
-                                                      unsigned long long* __restrict__ keys)
+                                                      unsigned long long* __restrict__ keys, int32_t* __restrict__ used)
 {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= n_elem * nb) return;
   const int64_t e = t / nb;
-  const unsigned long long row = (unsigned long long)(uint32_t)dofs[t];
-  unsigned long long* out = keys + t * nb;
-  for (int i = 0; i < nb; ++i) out[i] = (row << col_bits) | (uint32_t)dofs[e * nb + i];
+  const int j = (int)(t - e * nb);
+  const uint32_t a = (uint32_t)dofs[t];
+  used[a] = 1;
+  unsigned long long* out = keys + e * (nb * (nb - 1) / 2) + j * (2 * nb - 1 - j) / 2;
+  for (int i = j + 1; i < nb; ++i) {
+    const uint32_t b = (uint32_t)dofs[e * nb + i];
+    out[i - j - 1] = ((unsigned long long)min(a, b) << col_bits) | max(a, b);
+  }
 }
 
-// rowptr[r] = the first unique key with row >= r; colind from the low col_bits bits
-__global__ void __launch_bounds__(256) k_pattern_rows(int64_t nd, int64_t nnz, int col_bits, const unsigned long long* __restrict__ keys,
-                                                      int32_t* __restrict__ rowptr)
+__global__ void __launch_bounds__(256) k_pattern_swap(int64_t n, int col_bits, const unsigned long long* __restrict__ keys,
+                                                      unsigned long long* __restrict__ out)
 {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r > nd) return;
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k < n) out[k] = ((keys[k] & ((1ull << col_bits) - 1ull)) << col_bits) | (keys[k] >> col_bits);
+}
+
+// first of the n sorted keys with a row >= r
+__device__ __forceinline__ int64_t row_start(int64_t r, int64_t n, int col_bits, const unsigned long long* keys)
+{
   const unsigned long long target = (unsigned long long)r << col_bits;
-  int64_t lo = 0, hi = nnz;
+  int64_t lo = 0, hi = n;
   while (lo < hi) {
     const int64_t mid = (lo + hi) >> 1;
     if (keys[mid] < target) lo = mid + 1;
     else hi = mid;
   }
-  rowptr[r] = (int32_t)lo;
+  return lo;
 }
 
-__global__ void __launch_bounds__(256) k_pattern_cols(int64_t nnz, int col_bits, const unsigned long long* __restrict__ keys,
-                                                      int32_t* __restrict__ colind)
+// Starts of row r among the lower and the upper entries, the row pointer (diag: the
+// diagonal entries before row r), and the diagonal entry's column.
+__global__ void __launch_bounds__(256) k_pattern_rows(int64_t nd, int64_t n, int col_bits,
+                                                      const unsigned long long* __restrict__ lower,
+                                                      const unsigned long long* __restrict__ upper,
+                                                      const int32_t* __restrict__ diag, int32_t* __restrict__ lo_start,
+                                                      int32_t* __restrict__ up_start, int32_t* __restrict__ rowptr)
+{
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r > nd) return;
+  const int64_t lo = row_start(r, n, col_bits, lower), up = row_start(r, n, col_bits, upper);
+  lo_start[r] = (int32_t)lo;
+  up_start[r] = (int32_t)up;
+  rowptr[r] = (int32_t)(lo + up + diag[r]);
+}
+
+// A row holds its lower entries, its diagonal one and its upper ones: entry k of a list
+// goes to k plus the other two lists' entries before it.  Thread k < n: lower and
+// upper entry k; thread n + r: row r's diagonal.
+__global__ void __launch_bounds__(256) k_pattern_cols(int64_t nd, int64_t n, int col_bits,
+                                                      const unsigned long long* __restrict__ lower,
+                                                      const unsigned long long* __restrict__ upper,
+                                                      const int32_t* __restrict__ diag,
+                                                      const int32_t* __restrict__ lo_start,
+                                                      const int32_t* __restrict__ up_start, int32_t* __restrict__ colind)
 {
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (k < nnz) colind[k] = (int32_t)(keys[k] & ((1ull << col_bits) - 1ull));
+  const unsigned long long mask = (1ull << col_bits) - 1ull;
+  if (k < n) {
+    const int64_t rl = (int64_t)(lower[k] >> col_bits), ru = (int64_t)(upper[k] >> col_bits);
+    colind[k + up_start[rl] + diag[rl]] = (int32_t)(lower[k] & mask);
+    colind[k + lo_start[ru + 1] + diag[ru + 1]] = (int32_t)(upper[k] & mask);
+  } else if (k < n + nd) {
+    const int64_t r = k - n;
+    if (diag[r + 1] > diag[r]) colind[lo_start[r + 1] + up_start[r] + diag[r]] = (int32_t)r;
+  }
 }
 
 // local edge j of a tet joins its vertices kEdge[j][0] and kEdge[j][1]
@@ -404,36 +453,59 @@ mg_status build_pattern_device(mg_plan* p, DeviceScratch& scratch, cudaStream_t 
     return MG_OK;
   }
   BuildBuffers B(scratch);
-  unsigned long long *a, *b;
+  unsigned long long *a, *upper, *lower;
   int64_t* count;
   unsigned char* tmp;
-  int32_t *d_rowptr, *d_colind;
-  // keys of 2 bits(nd) bits: one pass of the sort per 8 (64^3 P1: 5 passes instead of 7
-  // with the row in the high word)
+  int32_t *used, *diag, *lo_start, *up_start, *d_rowptr, *d_colind;
+  const int64_t m_keys = E * (nb * (nb - 1) / 2);
   const int col_bits = std::max(1, key_bits(nd)), end_bit = 2 * col_bits;
-  size_t sort_bytes = 0, uniq_bytes = 0;
+  size_t sort_bytes = 0, uniq_bytes = 0, scan_bytes = 0;
   MG_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, (unsigned long long*)nullptr, (unsigned long long*)nullptr,
-                                         (int)n, 0, end_bit, st));
+                                         (int)m_keys, 0, end_bit, st));
   MG_CUDA(cub::DeviceSelect::Unique(nullptr, uniq_bytes, (unsigned long long*)nullptr, (unsigned long long*)nullptr,
-                                    (int64_t*)nullptr, (int)n, st));
-  MG_TRY(scratch.reserve(2 * sizeof(unsigned long long) * (size_t)n + std::max(sort_bytes, uniq_bytes) + 1024));
-  MG_TRY(B.temp(&a, n));
-  MG_TRY(B.temp(&b, n));
+                                    (int64_t*)nullptr, (int)m_keys, st));
+  MG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (int32_t*)nullptr, (int32_t*)nullptr, (int)(nd + 1), st));
+  const size_t tmp_bytes = std::max({sort_bytes, uniq_bytes, scan_bytes});
+  MG_TRY(scratch.reserve(2 * sizeof(unsigned long long) * (size_t)m_keys + 4 * sizeof(int32_t) * (size_t)(nd + 1) +
+                         tmp_bytes + 4096));
+  MG_TRY(B.temp(&a, m_keys));
+  MG_TRY(B.temp(&upper, m_keys));
+  MG_TRY(B.temp(&used, nd + 1));
+  MG_TRY(B.temp(&diag, nd + 1));
+  MG_TRY(B.temp(&lo_start, nd + 1));
+  MG_TRY(B.temp(&up_start, nd + 1));
   MG_TRY(B.temp(&count, 1));
-  MG_TRY(B.temp(&tmp, (int64_t)std::max(sort_bytes, uniq_bytes)));
+  MG_TRY(B.temp(&tmp, (int64_t)tmp_bytes));
   const int threads = 256;
-  k_pattern_keys<<<(int)((E * nb + threads - 1) / threads), threads, 0, st>>>(E, nb, col_bits, m->d_dofs, a);
+  MG_CUDA(cudaMemsetAsync(used, 0, sizeof(int32_t) * (nd + 1), st));
+  k_pattern_keys<<<(int)((E * nb + threads - 1) / threads), threads, 0, st>>>(E, nb, col_bits, m->d_dofs, a, used);
   MG_CUDA(cudaGetLastError());
-  MG_CUDA(cub::DeviceRadixSort::SortKeys(tmp, sort_bytes, a, b, (int)n, 0, end_bit, st));
-  MG_CUDA(cub::DeviceSelect::Unique(tmp, uniq_bytes, b, a, count, (int)n, st));
-  int64_t nnz = 0;
-  MG_CUDA(cudaMemcpyAsync(&nnz, count, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  size_t tb = tmp_bytes;
+  MG_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, used, diag, (int)(nd + 1), st));
+  tb = tmp_bytes;
+  MG_CUDA(cub::DeviceRadixSort::SortKeys(tmp, tb, a, upper, (int)m_keys, 0, end_bit, st));
+  tb = tmp_bytes;
+  MG_CUDA(cub::DeviceSelect::Unique(tmp, tb, upper, a, count, (int)m_keys, st));
+  std::swap(a, upper);  // the unique keys; a is free again
+  int64_t n_up = 0;
+  int32_t n_diag = 0;
+  MG_CUDA(cudaMemcpyAsync(&n_up, count, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  MG_CUDA(cudaMemcpyAsync(&n_diag, diag + nd, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   MG_CUDA(cudaStreamSynchronize(st));
+  const int64_t nnz = 2 * n_up + n_diag;
   if (nnz >= INT32_MAX) return set_error(MG_ERR_SIZE, "nnz above 2^31-1");
+  unsigned long long* swapped;
+  MG_TRY(B.temp(&swapped, n_up));
+  lower = a;
+  k_pattern_swap<<<(int)((n_up + threads - 1) / threads), threads, 0, st>>>(n_up, col_bits, upper, swapped);
+  tb = tmp_bytes;
+  MG_CUDA(cub::DeviceRadixSort::SortKeys(tmp, tb, swapped, lower, (int)n_up, 0, end_bit, st));
   MG_TRY(B.alloc(&d_rowptr, nd + 1));
   MG_TRY(B.alloc(&d_colind, nnz));
-  k_pattern_rows<<<(int)((nd + 1 + threads - 1) / threads), threads, 0, st>>>(nd, nnz, col_bits, a, d_rowptr);
-  k_pattern_cols<<<(int)((nnz + threads - 1) / threads), threads, 0, st>>>(nnz, col_bits, a, d_colind);
+  k_pattern_rows<<<(int)((nd + 1 + threads - 1) / threads), threads, 0, st>>>(nd, n_up, col_bits, lower, upper, diag,
+                                                                              lo_start, up_start, d_rowptr);
+  k_pattern_cols<<<(int)((n_up + nd + threads - 1) / threads), threads, 0, st>>>(nd, n_up, col_bits, lower, upper, diag,
+                                                                                 lo_start, up_start, d_colind);
   MG_CUDA(cudaGetLastError());
   p->colind.resize(nnz);
   MG_CUDA(cudaMemcpyAsync(p->rowptr.data(), d_rowptr, sizeof(int32_t) * (nd + 1), cudaMemcpyDeviceToHost, st));

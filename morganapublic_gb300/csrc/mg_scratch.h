@@ -44,6 +44,16 @@ class DeviceScratch {
       if (chunks_[c].size - (c == at_.chunk ? at_.used : 0) >= bytes) return MG_OK;
     return grow(bytes);
   }
+  // frees everything (nothing may be in use) if it is more than `limit`
+  void trim(size_t limit)
+  {
+    size_t all = 0;
+    for (const Chunk& c : chunks_) all += c.size;
+    if (all <= limit) return;
+    for (const Chunk& c : chunks_) cudaFree(c.base);
+    chunks_.clear();
+    at_ = Mark{0, 0};
+  }
   Mark mark() const { return at_; }
   void release(Mark m) { at_ = m; }
 

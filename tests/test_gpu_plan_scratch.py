@@ -30,3 +30,21 @@ def test_device_plan_matches_host_plan(n, order):
     a, b, c = (getattr(q, maps)() for q in (built, host, other))
     for k in b:
         assert np.array_equal(a[k], b[k]) and np.array_equal(c[k], b[k])
+
+
+@pytest.mark.parametrize("order", [1, 2])
+def test_nodes_without_elements_have_empty_rows(order):
+    import morganapublic_gb300 as mg
+    m = meshgen.kuhn_cube(3, jitter=0.1, seed=2, permute=True)
+    n = len(m.xyz)
+    # unused nodes before, between and after the used ones
+    place = np.arange(n) + 2 + 3 * (np.arange(n) >= n // 2)
+    xyz = np.full((n + 9, 3), 0.5)
+    xyz[place] = m.xyz
+    mesh = mg.Mesh(xyz, place[m.conn].astype(np.int32), order=order)
+    host, built = mg.MatrixBuilder(mesh), mg.MatrixBuilder(mesh, pattern_on_device=True)
+    for a, b in zip(built.pattern(), host.pattern()):
+        assert np.array_equal(a, b)
+    rows = np.diff(built.pattern()[0])
+    assert (rows[:n + 9] == 0).sum() == 9
+    assert bool((built.assemble("mass") == host.assemble("mass")).all())
