@@ -112,7 +112,10 @@ static int row_group(const mg_plan* p)
 
 // FP32 rows are streamed where the columns are 32-bit (16-bit offsets need each entry's
 // row) and rows are long.
-static bool stream_rows(const mg_plan* p) { return !p->d_coloff && p->nnz > 16 * p->ndof; }
+static bool stream_rows(const mg_plan* p)
+{
+  return !p->d_coloff && p->nnz > 16 * p->ndof && p->nnz < INT32_MAX - 1024;  // window ends in 32 bits
+}
 
 // CTAs covering every row once (G lanes per row), for the standalone SpMV.
 static int spmv_full_grid(int64_t rows, int G)
@@ -1301,14 +1304,20 @@ static mg_status cg_iterate(mg_plan* p, const V* vals, V* x, CgWork<V>& w, int G
   bool use_graph = true;
   cudaStreamCaptureStatus cs;
   MG_CUDA(cudaStreamIsCapturing(st, &cs));
-  const RowPartition* part = nullptr;
-  MG_TRY(resident_partition<V>(p, &part));
   constexpr int U = CgShape<V>::U;
-  const int threads = resident_threads<V>(part->max_rows, G);
-  const bool in_smem = resident_smem<V>(part->ctas, threads, part->max_rows, true) <= kResidentVectors;
-  const size_t smem = resident_smem<V>(part->ctas, threads, part->max_rows, in_smem);
   const int64_t bytes = p->nnz * (int64_t)(sizeof(V) + (p->d_coloff ? 2 : 4)) + 6 * n * (int64_t)sizeof(V);
-  bool resident = bytes <= kResidentBytes && smem <= kResidentVectors && cs == cudaStreamCaptureStatusNone;
+  bool resident = bytes <= kResidentBytes && cs == cudaStreamCaptureStatusNone;
+  const RowPartition* part = nullptr;
+  int threads = 0;
+  bool in_smem = false;
+  size_t smem = 0;
+  if (resident) {
+    MG_TRY(resident_partition<V>(p, &part));
+    threads = resident_threads<V>(part->max_rows, G);
+    in_smem = resident_smem<V>(part->ctas, threads, part->max_rows, true) <= kResidentVectors;
+    smem = resident_smem<V>(part->ctas, threads, part->max_rows, in_smem);
+    resident = smem <= kResidentVectors;
+  }
   const auto on_kernel = [&](auto&& f) -> mg_status {  // f(lanes per row, index type) of this system
     if constexpr (sizeof(V) == 8) {
       return p->d_coloff ? f(std::integral_constant<int, 1>(), int16_t()) : f(std::integral_constant<int, 1>(), int32_t());
