@@ -1326,6 +1326,19 @@ __device__ __forceinline__ typename Arith<MODE>::T em_value(const unsigned char*
 template <int MODE>
 __device__ __forceinline__ typename Arith<MODE>::Out run_sum(const unsigned char* em, const uint16_t* src, int32_t L)
 {
+  if constexpr (MODE == kF64) {
+    // no rows past L: an addition, of zero too, holds the FP64 pipe that bounds this mode
+    // (P1 128^3: 2.40 ms with them, 2.36 without)
+    double v = 0.0;
+    int32_t j = 0;
+    for (; j + 4 <= L; j += 4) {
+      const double x0 = em_value<MODE>(em, src[32 * j]), x1 = em_value<MODE>(em, src[32 * j + 32]),
+                   x2 = em_value<MODE>(em, src[32 * j + 64]), x3 = em_value<MODE>(em, src[32 * j + 96]);
+      v = (((v + x0) + x1) + x2) + x3;
+    }
+    for (; j < L; ++j) v += em_value<MODE>(em, src[32 * j]);
+    return v;
+  }
   SourceSum<MODE> sum;
   for (int32_t j = 0; j < L; j += 4) {
     const uint32_t i0 = src_row(src, j, L), i1 = src_row(src, j + 1, L), i2 = src_row(src, j + 2, L),
