@@ -92,10 +92,15 @@ __global__ void k_diag_coloff(int64_t nd, const int32_t* __restrict__ rowptr, co
     else hi = mid;
   }
   diag[r] = lo;
+  // one plain store per row that does not fit, and none of its later entries: an atomic
+  // per entry, all on one address, took 7.6 ms at P2 48^3
   for (int k = s0; k < rowptr[r + 1]; ++k) {
     const int64_t d = (int64_t)colind[k] - r;
-    if (d < INT16_MIN || d > INT16_MAX) atomicAnd(fits, 0);
-    else coloff[k] = (int16_t)d;
+    if (d < INT16_MIN || d > INT16_MAX) {
+      *fits = 0;
+      return;
+    }
+    coloff[k] = (int16_t)d;
   }
 }
 
@@ -183,17 +188,16 @@ __global__ void __launch_bounds__(256) k_upper_counts(int64_t nd, int nb, const 
   n_contrib[r] = c;
 }
 
-__global__ void __launch_bounds__(256) k_slot_map(int64_t nd, int nb, int64_t E, int aos,
-                                                  const int32_t* __restrict__ inc_ptr,
-                                                  const uint32_t* __restrict__ inc_q, const int32_t* __restrict__ dofs_m,
-                                                  const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
-                                                  const int32_t* __restrict__ up_first,
-                                                  const int32_t* __restrict__ src_first, int32_t* cur, int32_t* useg,
-                                                  int32_t* uslot, int32_t* umirror, int32_t* urow, uint32_t* src,
-                                                  int* bad)
+// The same for one row by one thread, searching each coupled column in the row: the rows
+// of a vertex with very many elements, where every entry against every element would
+// be quadratic.
+__device__ __noinline__ void slot_row_serial(int64_t r, int nb, int64_t E, int aos, const int32_t* __restrict__ inc_ptr,
+                                             const uint32_t* __restrict__ inc_q, const int32_t* __restrict__ dofs_m,
+                                             const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
+                                             const int32_t* __restrict__ up_first,
+                                             const int32_t* __restrict__ src_first, int32_t* cur, int32_t* useg,
+                                             int32_t* uslot, int32_t* umirror, int32_t* urow, uint32_t* src, int* bad)
 {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= nd) return;
   const int32_t r0 = rowptr[r], len = rowptr[r + 1] - r0;
   const int32_t* cols = colind + r0;
   const int kd = find_col(cols, len, (int32_t)r);  // first upper entry of the row
@@ -245,6 +249,89 @@ __global__ void __launch_bounds__(256) k_slot_map(int64_t nd, int nb, int64_t E,
   }
 }
 
+// Per upper entry of a row its CSR position, mirror and sources. A group of lanes takes a
+// row, a lane an upper entry: it looks for its column among the dofs of the row's
+// elements, which all lanes read at the same addresses, in ascending position; once to
+// count, then (offsets by a scan over the group) to write. The matches must add up to
+// the couplings that k_upper_counts found, or an entry is missing from the pattern.
+// Bound by the latency of those reads.  GB300: 1.0 ms at P1 128^3, 0.9 at P2 48^3 (one
+// thread per row, with a binary search of every coupled column in the row, twice: 5.1 and
+// 2.9 ms).
+constexpr int kSerialRow = 512;  // elements of a row above which one thread searches
+template <int NB, int G>
+__global__ void __launch_bounds__(256) k_slot_map(int64_t nd, int64_t E, int aos, const int32_t* __restrict__ inc_ptr,
+                                                  const uint32_t* __restrict__ inc_q, const int32_t* __restrict__ dofs_m,
+                                                  const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
+                                                  const int32_t* __restrict__ up_first,
+                                                  const int32_t* __restrict__ src_first, int32_t* cur, int32_t* useg,
+                                                  int32_t* uslot, int32_t* umirror, int32_t* urow, uint32_t* src,
+                                                  int* bad)
+{
+  constexpr int NU = NB * (NB + 1) / 2;
+  const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+  if (r >= nd) return;
+  const int lane = threadIdx.x % G;
+  const unsigned mask = (G == 32 ? 0xffffffffu : (1u << G) - 1u) << ((threadIdx.x & 31) / G * G);
+  const int32_t i0 = inc_ptr[r], i1 = inc_ptr[r + 1];
+  if (i1 - i0 > kSerialRow) {
+    if (lane == 0)
+      slot_row_serial(r, NB, E, aos, inc_ptr, inc_q, dofs_m, rowptr, colind, up_first, src_first, cur, useg, uslot,
+                      umirror, urow, src, bad);
+    return;
+  }
+  const int32_t r0 = rowptr[r], len = rowptr[r + 1] - r0;
+  const int32_t* cols = colind + r0;
+  const int kd = find_col(cols, len, (int32_t)r);  // first upper entry of the row
+  const int32_t u0 = up_first[r];
+  // place of `col` among the dofs of element p, or -1
+  const auto place = [&](int64_t p, int32_t col) {
+    int at = -1;
+    const int2* d = reinterpret_cast<const int2*>(dofs_m + p * NB);
+#pragma unroll
+    for (int j = 0; j < NB / 2; ++j) {
+      const int2 v = __ldg(d + j);
+      if (v.x == col) at = 2 * j;
+      if (v.y == col) at = 2 * j + 1;
+    }
+    return at;
+  };
+  int32_t pos = src_first[r];
+  for (int kb = kd; kb < len; kb += G) {
+    const int k = kb + lane;
+    const int32_t col = k < len ? cols[k] : -1;
+    int32_t c = 0;
+    for (int32_t t = i0; t < i1; ++t) c += place(inc_q[t] / NB, col) >= 0 ? 1 : 0;
+    int32_t before = c;
+#pragma unroll
+    for (int off = 1; off < G; off <<= 1) {
+      const int32_t o = __shfl_up_sync(mask, before, off, G);
+      if (lane >= off) before += o;
+    }
+    const int32_t total = __shfl_sync(mask, before, G - 1, G);
+    int32_t at = pos + before - c;
+    pos += total;
+    if (k < len) {
+      const int32_t t = u0 + (k - kd);
+      useg[t] = at;
+      uslot[t] = r0 + k;
+      urow[t] = (int32_t)r;
+      const int32_t m0 = rowptr[col], ml = rowptr[col + 1] - m0;
+      const int km = find_col(colind + m0, ml, (int32_t)r);
+      if (km >= ml || colind[m0 + km] != (int32_t)r) *bad = 1;
+      umirror[t] = m0 + km;
+    }
+    for (int32_t t = i0; t < i1; ++t) {
+      const uint32_t q = inc_q[t];
+      const int64_t p = q / NB;
+      const int j = place(p, col);
+      if (j >= 0) {
+        const int u = sym_index((int)(q - (uint32_t)p * NB), j, NB);
+        src[at++] = aos ? (uint32_t)(p * NU + u) : (uint32_t)(u * E + p);
+      }
+    }
+  }
+  if (lane == 0 && pos != src_first[r + 1]) *bad = 1;
+}
 
 // ---- the gather's layout: upper entries regrouped (diagonal entries first, each
 // class in CSR order) into groups of 32, one per warp; a group's sources stored
@@ -255,11 +342,13 @@ __global__ void k_group_keys(int64_t U, const int32_t* __restrict__ urow, const 
                              int32_t* __restrict__ ndiag)
 {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= U) return;
-  const bool dg = uslot[t] == umirror[t];
-  key[t] = ((uint32_t)(urow[t] / kGatherRowBlock) << 1) | (dg ? 0u : 1u);
-  id[t] = (uint32_t)t;
-  if (dg) atomicAdd(ndiag, 1);
+  const bool dg = t < U && uslot[t] == umirror[t];
+  if (t < U) {
+    key[t] = ((uint32_t)(urow[t] / kGatherRowBlock) << 1) | (dg ? 0u : 1u);
+    id[t] = (uint32_t)t;
+  }
+  const int n = __syncthreads_count(dg);
+  if (threadIdx.x == 0 && n > 0) atomicAdd(ndiag, n);
 }
 
 __global__ void k_group_len(int64_t G, int64_t U, const uint32_t* __restrict__ perm, const int32_t* __restrict__ useg,
@@ -587,9 +676,13 @@ mg_status build_slot_map(mg_plan* p, DeviceScratch& scratch, cudaStream_t st)
   MG_TRY(B.temp(&umirror, U));
   MG_TRY(B.temp(&urow, U));
   MG_TRY(B.temp(&src, C));
-  k_slot_map<<<grid_of(nd), 256, 0, st>>>(nd, nb, E, slot_map_aos(m->order) ? 1 : 0, inc_ptr, vout,
-                                           p->d_dofs_morton, p->d_rowptr, p->d_colind, up_first, src_first, cur, useg,
-                                           uslot, umirror, urow, src, bad);
+  const auto slot_map = [&](auto kernel, int lanes) {
+    kernel<<<grid_of(nd * lanes), 256, 0, st>>>(nd, E, slot_map_aos(m->order) ? 1 : 0, inc_ptr, vout, p->d_dofs_morton,
+                                                p->d_rowptr, p->d_colind, up_first, src_first, cur, useg, uslot,
+                                                umirror, urow, src, bad);
+  };
+  if (nb == 4) slot_map(k_slot_map<4, 8>, 8);  // P1 rows have about 8 upper entries, P2 ones 14
+  else slot_map(k_slot_map<10, 16>, 16);
   const int32_t last = (int32_t)C;
   MG_CUDA(cudaMemcpyAsync(useg + U, &last, sizeof(int32_t), cudaMemcpyHostToDevice, st));
   MG_CUDA(cudaGetLastError());

@@ -48,3 +48,26 @@ def test_nodes_without_elements_have_empty_rows(order):
     rows = np.diff(built.pattern()[0])
     assert (rows[:n + 9] == 0).sum() == 9
     assert bool((built.assemble("mass") == host.assemble("mass")).all())
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("n", [510, 512, 513, 700])
+def test_vertices_with_very_many_elements(n, order):
+    # a fan: n elements around the edge between two vertices, whose rows the plan builds
+    # by one thread each above 512 elements; against the oracle
+    import oracle as orc
+    from helpers import row_scaled_err
+
+    import morganapublic_gb300 as mg
+    angle = 2.0 * np.pi * np.arange(n) / n
+    ring = np.stack([np.cos(angle), np.sin(angle), np.zeros(n)], axis=1)
+    xyz = np.concatenate([ring, [[0.0, 0.0, -1.0], [0.0, 0.0, 1.0]]])
+    i = np.arange(n)
+    conn = np.stack([np.full(n, n), i, (i + 1) % n, np.full(n, n + 1)], axis=1).astype(np.int32)
+    b = mg.MatrixBuilder(mg.Mesh(xyz, conn, order=order), pattern_on_device=True)
+    kappa = meshgen.lognormal(n, 1.0, n)
+    got = b.assemble("mass_coeff", coeff=kappa, quad=4).cpu().numpy()
+    _, rp, ci, want = orc.full_operator("mass_coeff", order, 4, xyz, conn, coeff=kappa)
+    rowptr, colind = b.pattern()
+    assert np.array_equal(rowptr, rp) and np.array_equal(colind, ci)
+    assert row_scaled_err(rp, want, got) <= 1e-12
