@@ -456,7 +456,7 @@ __device__ __forceinline__ bool coef_not_finite(double c)
 // The coefficient and the vertex dofs of Morton element p.
 __device__ __forceinline__ double elem_coef(const ElemArgs& a, int64_t p)
 {
-  return a.coeff ? __ldg(a.coeff + a.elem_order[p]) : a.cconst;
+  return a.coeff ? a.coeff[a.elem_order[p]] : a.cconst;
 }
 __device__ __forceinline__ int4 elem_nodes(const ElemArgs& a, int64_t p)
 {
@@ -980,8 +980,8 @@ __global__ void __launch_bounds__(128, 4) k_elem_mat_pair(ElemArgs a)
   if (first >= E) return;
   // past the last element the pair repeats it (the same values stored again)
   const int64_t p0 = min(first + lane, E - 1), p1 = min(first + 32 + lane, E - 1);
-  const double c0 = a.coeff ? __ldg(a.coeff + a.elem_order[p0]) : a.cconst;
-  const double c1 = a.coeff ? __ldg(a.coeff + a.elem_order[p1]) : a.cconst;
+  const double c0 = a.coeff ? a.coeff[a.elem_order[p0]] : a.cconst;
+  const double c1 = a.coeff ? a.coeff[a.elem_order[p1]] : a.cconst;
   const auto vertices = [&](int64_t p) {
     const int2* d = reinterpret_cast<const int2*>(a.dofs_m + p * 10);
     const int2 x = __ldg(d), y = __ldg(d + 1);
@@ -1096,7 +1096,7 @@ __global__ void __launch_bounds__(256, 1) k_elem_mat_f64(ElemArgs a)
   const int64_t E = a.n_elem;
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p >= E) return;
-  const double coef = a.coeff ? __ldg(a.coeff + a.elem_order[p]) : a.cconst;
+  const double coef = a.coeff ? a.coeff[a.elem_order[p]] : a.cconst;
   const int32_t* dp = a.dofs_m + p * 10;
   Cof<double> f;
   geometry_f64(a.geo, make_int4(dp[0], dp[1], dp[2], dp[3]), f);
@@ -1278,7 +1278,7 @@ __device__ __forceinline__ void coef_fetch(double* smem, const double* c, int64_
   const int odd = (int)((reinterpret_cast<uintptr_t>(c + e) >> 3) & 1);
   const int64_t e0 = e - odd;
   if (e0 >= 0 && e0 + 1 < n) cp_async16(smem, c + e0);
-  else smem[odd] = __ldg(c + e);
+  else smem[odd] = c[e];
 }
 __device__ __forceinline__ double coef_slot(const double* smem, const double* c, int64_t e)
 {
@@ -1669,11 +1669,12 @@ __device__ __forceinline__ int dexp(double v) { return (int)((__double_as_longlo
 // v * 2^(1023 - emax) as a double-word value, by exponent arithmetic (emax = the
 // largest biased exponent of the group, a normal number).  Parts more than 2^-74
 // below the largest are dropped (a relative 2^-74 of the group).
+template <bool RENORM>
 __device__ __forceinline__ ff ff_rescaled(double v, int emax)
 {
   const long long b = __double_as_longlong(v);
   if (dexp(v) + 74 < emax) return ff{0.0f, 0.0f};
-  return ff_from_double_bits(__longlong_as_double(b - ((long long)(emax - 1023) << 52)));
+  return ff_from_double_bits<RENORM>(__longlong_as_double(b - ((long long)(emax - 1023) << 52)));
 }
 
 // v * 2^k for |k| <= 2044 (two exact power-of-two products unless the result
@@ -1763,7 +1764,7 @@ __device__ __forceinline__ void cached_geometry(const float2* det, const float2*
 // neighbouring dof values.
 // P1 is bound by instruction issue: dot products with one renormalisation each (instead of
 // one per operation) and five CTAs per SM took it from 52 to 45 us at P1 64^3 on GB300 (4:
-// 49, 6: 47.5).  Two elements per thread as packed pairs measured 59 to 68 us, and the
+// 49, 6: 47.5), no table staged and the plan read before the wait to 41.4.  Two elements per thread as packed pairs measured 59 to 68 us, and the
 // geometry formed from nodes staged per block 70 us: fewer warps for the same gathers.
 template <int ORDER>
 __global__ void __launch_bounds__(256, ORDER == 1 ? 5 : 1) k_adjoint(int64_t n_elem, const int32_t* elem_order, const int32_t* dofs_m,
@@ -1771,14 +1772,24 @@ __global__ void __launch_bounds__(256, ORDER == 1 ? 5 : 1) k_adjoint(int64_t n_e
                                                  double wsum, const double* u, const double* lam, double* grad)
 {
   constexpr int NB = ORDER == 1 ? 4 : 10, NU = ORDER == 1 ? 10 : 55;
-  __shared__ ff tab[6 * NU];
-  for (int i = threadIdx.x; i < 6 * NU; i += blockDim.x) tab[i] = ff_from_double(tables[i]);
-  __syncthreads();
+  __shared__ ff tab[ORDER == 1 ? 1 : 6 * NU];  // P1 takes the zero row sums, no table
+  // P1 is launched with programmatic dependence; P2, whose CTAs fill the SM's registers,
+  // takes 17 us without and 27 with it at 13 k elements
+  if constexpr (ORDER == 1) {
+    pdl_trigger();
+  } else {
+    for (int i = threadIdx.x; i < 6 * NU; i += blockDim.x) tab[i] = ff_from_double(tables[i]);
+    __syncthreads();
+  }
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n_elem) return;
+  if (i >= n_elem) {
+    if constexpr (ORDER == 1) pdl_wait();
+    return;
+  }
   const int64_t e = elem_order[i];
   const int32_t* dofs = dofs_m + i * NB;  // this element's dofs; the first four are its vertices
   const int4 n = ORDER == 1 ? reinterpret_cast<const int4*>(dofs_m)[i] : make_int4(dofs[0], dofs[1], dofs[2], dofs[3]);
+  if constexpr (ORDER == 1) pdl_wait();  // u, lambda and grad belong to the kernels before this one
   // FP64 differences to the first dof and the largest exponent of each group
   double du[NB - 1], dl[NB - 1];
   int eu = 0, el = 0;
@@ -1810,8 +1821,8 @@ __global__ void __launch_bounds__(256, ORDER == 1 ? 5 : 1) k_adjoint(int64_t n_e
     ff gu[3], gl[3], a[3], c[3];
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      a[b] = ff_rescaled(du[b], eu);
-      c[b] = ff_rescaled(dl[b], el);
+      a[b] = ff_rescaled<true>(du[b], eu);
+      c[b] = ff_rescaled<true>(dl[b], el);
     }
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
@@ -1823,8 +1834,8 @@ __global__ void __launch_bounds__(256, ORDER == 1 ? 5 : 1) k_adjoint(int64_t n_e
     ff ue[NB - 1], le[NB - 1];
 #pragma unroll
     for (int k = 0; k < NB - 1; ++k) {
-      ue[k] = ff_rescaled(du[k], eu);
-      le[k] = ff_rescaled(dl[k], el);
+      ue[k] = ff_rescaled<false>(du[k], eu);
+      le[k] = ff_rescaled<false>(dl[k], el);
     }
     ff g[6];
     metric<ff>(f, ff_make(1.0f) / f.det, g);
@@ -1906,12 +1917,12 @@ __global__ void __launch_bounds__(256) k_rhs_elem(int64_t n_elem, const int32_t*
     return;
   }
   const float2 dt = gdet[p];
-  const ff sdet = ff_rescaled(sd, es) * ff{dt.x, dt.y};
+  const ff sdet = ff_rescaled<false>(sd, es) * ff{dt.x, dt.y};
   ff v[NB];
   if (field) {
     ff fr[NB];
 #pragma unroll
-    for (int k = 0; k < NB; ++k) fr[k] = ff_rescaled(f[k], ef);
+    for (int k = 0; k < NB; ++k) fr[k] = ff_rescaled<false>(f[k], ef);
     if (ORDER == 1 && two_valued) {
       // M^_lk = o + (d - o) [l = k]: (M^ f)_l = o sum_k f_k + (d - o) f_l, with
       // d = tab(0,0) and o = tab(0,1) from the table
@@ -1985,7 +1996,8 @@ __global__ void __launch_bounds__(256) k_rhs_gather(int64_t ndof, const int32_t*
 // The two passes wrote and gathered 32 bytes per element through memory and issued 21
 // warp instructions per element, a third of them conversions: GB300, P1 96^3, 217 ->
 // 141 us (block kernel 126, shared nodes 14; bound by issue and the L1 data path, 61 %
-// each), and the map is built on the GPU (first call on a plan 76 -> 1.9 ms).
+// each), 134 with programmatic launches, the table staged only where it is used and
+// no FP64 comparisons; the map is built on the GPU (first call on a plan 76 -> 1.6 ms).
 struct RhsArgs {
   int64_t n_elem;
   const int32_t *elem_order, *bnode, *bnode_n;
@@ -2087,32 +2099,34 @@ __global__ void __launch_bounds__(256, 5) k_rhs_block(RhsArgs a)
   const int tid = threadIdx.x, lane = tid & 31, lp = tid + (tid & ~31);
   const int64_t blk = blockIdx.x, p0 = blk * kElemBlock, E = a.n_elem;
   const int64_t p1 = min(p0 + lp, E - 1), p2 = min(p0 + lp + 32, E - 1);  // past the end: the last element again
+  pdl_trigger();
   const int n_nodes = a.bnode_n[blk];
   const int32_t id = a.bnode[blk * kStageNodes + tid];
   // a warp's coefficient slots lie in the rows that only its own elements overwrite
   double* slot1 = reinterpret_cast<double*>(y + (lane >> 4) * kElemBlock + (lp - lane) + 4 * (lane & 15));
   double* slot2 = slot1 + kElemBlock;
   int64_t e1 = 0, e2 = 0;
-  if (a.scale) {
-    e1 = a.elem_order[p1], e2 = a.elem_order[p2];
-    coef_fetch(slot1, a.scale, e1, E);
-    coef_fetch(slot2, a.scale, e2, E);
-  }
-  asm volatile("cp.async.commit_group;\n" ::);
+  if (a.scale) e1 = a.elem_order[p1], e2 = a.elem_order[p2];
   cp_async16(s_pos + 8 * tid, a.bpos + blk * Y + 8 * tid);
-  asm volatile("cp.async.commit_group;\n" ::);
-  const double f = a.field ? __ldg(a.field + id) : 1.0;
   const float2 d1 = a.gdet[p1], d2 = a.gdet[p2];
   const uchar4 q1 = __ldg(a.elem_local + p1), q2 = __ldg(a.elem_local + p2);
   const int32_t out = a.bout[blk * kStageNodes + tid];
   for (int i = tid; i <= kStageNodes; i += 256) s_start[i] = a.bstart[blk * (kStageNodes + 1) + i];
-  if (tid < 10) tab[tid] = ff_from_double(a.mass[tid]);
-  asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+  if (a.form == kRhsTable && tid < 10) tab[tid] = ff_from_double(a.mass[tid]);
+  // up to here only the plan was read
+  pdl_wait();
+  if (a.scale) {
+    coef_fetch(slot1, a.scale, e1, E);
+    coef_fetch(slot2, a.scale, e2, E);
+  }
+  asm volatile("cp.async.commit_group;\n" ::);
+  const double f = a.field ? a.field[id] : 1.0;
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
   const double s1 = a.scale ? coef_slot(slot1, a.scale, e1) : 1.0, s2 = a.scale ? coef_slot(slot2, a.scale, e2) : 1.0;
   // largest and smallest biased exponents of f, s and det over the block; zeros do not
   // count for the smallest, subnormals count as exponent zero
   {
-    const auto low = [](double v) { return v == 0.0 ? 0x7ff : dexp(v); };
+    const auto low = [](double v) { return (__double_as_longlong(v) << 1) == 0 ? 0x7ff : dexp(v); };
     const auto fexp = [](float v) { return (int)((__float_as_uint(v) >> 23) & 0xffu); };
     int m[6] = {dexp(f), 0x7ff - low(f), max(dexp(s1), dexp(s2)), 0x7ff - min(low(s1), low(s2)),
                 max(fexp(d1.x), fexp(d2.x)), 0x7ff - min(fexp(d1.x), fexp(d2.x))};
@@ -2122,7 +2136,6 @@ __global__ void __launch_bounds__(256, 5) k_rhs_block(RhsArgs a)
       if (lane == 0) red[k][tid >> 5] = m[k];
     }
   }
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
   int m[6];
 #pragma unroll
@@ -2198,11 +2211,12 @@ __global__ void __launch_bounds__(256, 5) k_rhs_block(RhsArgs a)
 // One thread per node: the partials of a node with elements in several blocks in
 // ascending block; nodes outside every element get zero.
 __global__ void __launch_bounds__(256) k_rhs_shared(int64_t n, const int32_t* __restrict__ ptr,
-                                                    const double* __restrict__ partial, double* __restrict__ b)
+                                                    const double* partial, double* __restrict__ b)
 {
+  pdl_trigger();
   const int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (d >= n) return;
-  const int q0 = __ldg(ptr + d), q1 = __ldg(ptr + d + 1);
+  const int q0 = d < n ? __ldg(ptr + d) : 0, q1 = d < n ? __ldg(ptr + d + 1) : 1;
+  pdl_wait();  // every thread, so that this kernel's end implies the one before's
   if (q1 - q0 == 1) return;
   double v = 0.0;
   for (int q = q0; q < q1; ++q) v += partial[q];
@@ -2347,13 +2361,12 @@ mg_status mg_adjoint_grad(mg_plan* p, const double* d_u, const double* d_lambda,
   MG_TRY(plan_geometry(p, st));
   if (blocks > 0) {
     if (m->order == 1)
-      k_adjoint<1><<<blocks, threads, 0, st>>>(m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det,
-                                               p->d_geo_cof, d_tab, t->wsum, d_u, d_lambda, d_grad);
+      MG_CUDA(launch_pdl(k_adjoint<1>, blocks, threads, st, m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det,
+                         p->d_geo_cof, d_tab, t->wsum, d_u, d_lambda, d_grad));
     else
-      k_adjoint<2><<<blocks, threads, 0, st>>>(m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det,
-                                               p->d_geo_cof, d_tab, t->wsum, d_u, d_lambda, d_grad);
+      MG_CUDA(launch_k(false, k_adjoint<2>, blocks, threads, st, m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det,
+                         p->d_geo_cof, d_tab, t->wsum, d_u, d_lambda, d_grad));
   }
-  MG_CUDA(cudaGetLastError());
   return MG_OK;
 }
 
@@ -2399,10 +2412,9 @@ mg_status mg_assemble_rhs(mg_plan* p, const double* d_field, const double* d_ele
                     p->d_geo_det,    d_tab + 6 * nu,  d_field,          d_elem_scale, p->d_rhs_bpos,
                     p->d_rhs_bstart, p->d_rhs_bout,   p->d_rhs_partial, d_b,          form,
                     form == kRhsTable ? 1.0 : off};
-    k_rhs_block<<<(unsigned)p->n_blocks, 256, 0, st>>>(a);
-    MG_CUDA(cudaGetLastError());
-    k_rhs_shared<<<(unsigned)((p->ndof + 255) / 256), 256, 0, st>>>(p->ndof, p->d_rhs_ptr, p->d_rhs_partial, d_b);
-    MG_CUDA(cudaGetLastError());
+    MG_CUDA(launch_pdl(k_rhs_block, (int)p->n_blocks, 256, st, a));
+    MG_CUDA(launch_pdl(k_rhs_shared, (int)((p->ndof + 255) / 256), 256, st, p->ndof, (const int32_t*)p->d_rhs_ptr,
+                       (const double*)p->d_rhs_partial, d_b));
     return MG_OK;
   }
   MG_TRY(plan_rhs_map(p));

@@ -165,13 +165,14 @@ __device__ __forceinline__ double f2d_bits(float f)
 __device__ __forceinline__ double ff_to_double_bits(ff a) { return f2d_bits(a.hi) + f2d_bits(a.lo); }
 
 // double -> hi + lo: the top 24 bits of the significand (truncated, exact) and the
-// next 29 bits rounded to nearest, renormalised -- |x - hi - lo| <= 2^-48 |x|.
+// next 29 bits rounded to nearest, renormalised where RENORM -- |x - hi - lo| <= 2^-48 |x|.
 // lo is built without an integer-to-float conversion (which GB300 issues at a
 // small fraction of the FP32 rate): with mlo the low 29 significand bits, lo =
 // RN(mlo 2^(e-52)) is the float sum of two exact terms, the top 23 and the low 6
 // bits of mlo, each obtained as (2^k (1 + bits 2^-23)) - 2^k from a float built
 // with that exponent.  For |x| in about 2^-74 .. 2^127 and x = 0; other values
 // fall back to the FP64 conversions.
+template <bool RENORM = true>
 __device__ __forceinline__ ff ff_from_double_bits(double x)
 {
   const uint64_t u = (uint64_t)__double_as_longlong(x);
@@ -190,8 +191,9 @@ __device__ __forceinline__ ff ff_from_double_bits(double x)
   const float lo = __uint_as_float(__float_as_uint(__fadd_rn(f1, f2)) ^ sign);
   // hi is truncated, so lo has hi's sign and up to its ulp; renormalised, it is at most
   // half an ulp of either sign, and the lo * lo that products drop has no bias (P1
-  // load vector from truncated parts: 3.3e-15 against 2.2e-15)
-  return fast_two_sum(hi, lo);
+  // load vector from truncated parts: 3.3e-15 against 2.2e-15; the P2 adjoint and load
+  // vector, whose own sums leave more, are no more exact for it and up to 1 us slower)
+  return RENORM ? fast_two_sum(hi, lo) : ff{hi, lo};
 }
 
 }  // namespace mg
