@@ -1517,20 +1517,6 @@ __global__ void __launch_bounds__(256) k_shared_sum(int64_t n_groups, const int3
   }
 }
 
-// Sets the dynamic shared-memory limit of a kernel once per device (the first
-// assembly of each kind on a device).
-template <typename K>
-static mg_status allow_smem(K kernel, size_t bytes, std::once_flag (&once)[64])
-{
-  int dev = 0;
-  MG_CUDA(cudaGetDevice(&dev));
-  cudaError_t err = cudaSuccess;
-  std::call_once(once[dev & 63],
-                 [&] { err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
-  MG_CUDA(err);
-  return MG_OK;
-}
-
 template <int MODE, bool SPLIT>
 static mg_status launch_block_t(mg_plan* p, const ElemArgs& a, void* d_values, cudaStream_t st)
 {

@@ -1,9 +1,13 @@
-// Kernel launches with programmatic dependent launch, and its device-side calls.
+// Kernel launches with programmatic dependent launch, its device-side calls, and the
+// shared-memory limit of a kernel.
 #pragma once
 
+#include <mutex>
 #include <utility>
 
 #include <cuda_runtime.h>
+
+#include "mg_internal.h"
 
 namespace mg {
 
@@ -38,6 +42,21 @@ template <typename... KArgs, typename... Args>
 static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t st, Args&&... args)
 {
   return launch_k(true, kernel, grid, block, st, std::forward<Args>(args)...);
+}
+
+// Sets the dynamic shared-memory limit of a kernel once per device, to the most that any
+// launch of it takes: the limit belongs to the kernel on the device, so one set to a
+// single launch's need would change under the launches of other host threads.
+template <typename K>
+static mg_status allow_smem(K kernel, size_t bytes, std::once_flag (&once)[64])
+{
+  int dev = 0;
+  MG_CUDA(cudaGetDevice(&dev));
+  cudaError_t err = cudaSuccess;
+  std::call_once(once[dev & 63],
+                 [&] { err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
+  MG_CUDA(err);
+  return MG_OK;
 }
 
 }  // namespace mg

@@ -1285,7 +1285,8 @@ template <typename V, int G, int U, typename I>
 static mg_status resident_fits(int ctas, int threads, size_t smem, bool* fits)
 {
   const auto kernel = k_cg_resident<V, G, U, I>;
-  MG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static std::once_flag once[64];
+  MG_TRY(allow_smem(kernel, kResidentVectors, once));  // smem <= kResidentVectors (cg_iterate)
   int per_sm = 0;
   MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
   *fits = (int64_t)per_sm * sm_count() >= ctas;
