@@ -1977,8 +1977,9 @@ __global__ void __launch_bounds__(256) k_rhs_gather(int64_t ndof, const int32_t*
 // written, another one a partial, added in block order by k_rhs_shared.
 //   y_l = s det (M^ f)_l
 // f (converted once per node), s and det are scaled by the powers of two of their largest
-// values in the block; where their spreads together exceed 2^70, or a value is Inf,
-// NaN or subnormal, the block runs in FP64 (rhs_block_f64).
+// values in the block; where their spreads together exceed 2^70, a value is Inf, NaN or
+// subnormal, or a determinant is 2^127 or more (its inverse power would be
+// subnormal), the block runs in FP64 (rhs_block_f64).
 // The two passes wrote and gathered 32 bytes per element through memory and issued 21
 // warp instructions per element, a third of them conversions: GB300, P1 96^3, 217 ->
 // 141 us (block kernel 126, shared nodes 14; bound by issue and the L1 data path, 61 %
@@ -1995,7 +1996,7 @@ struct RhsArgs {
   const int32_t* bout;     // per block kStageNodes outputs: node, or -1 - partial slot
   double *partial, *b;
   int form;     // of M^ f
-  double unit;  // factor of the sums (1 with the full table)
+  double unit;  // factor of the sums (1 with the full table), a normal number
 };
 // M^ f: u (sum_k f_k + f_l) where the table is u (1 + [l = k]) (the symmetric cards of two
 // and more degrees), u sum_k f_k where it is constant (the one-point card), else the
@@ -2130,7 +2131,7 @@ __global__ void __launch_bounds__(256, 5) k_rhs_block(RhsArgs a)
   const int lf = 0x7ff - m[1], ls = 0x7ff - m[3], ld = 0x7ff - m[5];
   // (all zero: the largest is 0 and the smallest 0x7ff)
   const int spread = (ef > 0 ? ef - lf : 0) + (es > 0 ? es - ls : 0) + (ed - ld);
-  if (ef == 0x7ff || es == 0x7ff || lf == 0 || ls == 0 || ed == 0xff || ld == 0 || spread > 70) {
+  if (ef == 0x7ff || es == 0x7ff || lf == 0 || ls == 0 || ed >= 0xfe || ld == 0 || spread > 70) {
     rhs_block_f64(a, reinterpret_cast<double*>(y), s_pos, s_start, n_nodes, out);
     return;
   }
@@ -2190,7 +2191,10 @@ __global__ void __launch_bounds__(256, 5) k_rhs_block(RhsArgs a)
       const bool two = j + 1 < j1;
       sum.add(ff{em_at(yh, o0), em_at(yl, o0)}, two ? ff{em_at(yh, o1), em_at(yl, o1)} : ff{0.0f, 0.0f});
     }
-    rhs_put(a, out, scale_pow2(a.unit * sum.result(), (ef > 0 ? ef - 1023 : 0) + (es > 0 ? es - 1023 : 0) + (ed - 127)));
+    // det's power goes into the factor (2^-27 .. 1): with the others it would leave
+    // scale_pow2's range
+    const double unit = __longlong_as_double(__double_as_longlong(a.unit) + ((long long)(ed - 127) << 52));
+    rhs_put(a, out, scale_pow2(unit * sum.result(), (ef > 0 ? ef - 1023 : 0) + (es > 0 ? es - 1023 : 0)));
   }
 }
 
@@ -2390,10 +2394,10 @@ mg_status mg_assemble_rhs(mg_plan* p, const double* d_field, const double* d_ele
     // every block's nodes fit the stage: one pass
     MG_TRY(build_rhs_map(p, st));
     const double diag = t->mass[0] - t->mass[1], off = t->mass[1], ulps = 8.0 * DBL_EPSILON * std::fabs(t->mass[0]);
-    const int form = !two_valued                          ? kRhsTable
-                     : std::fabs(diag - off) <= ulps      ? kRhsSumPlus
-                     : std::fabs(diag) <= ulps            ? kRhsSum
-                                                          : kRhsTable;
+    const int form = !two_valued || std::fabs(off) < 0x1p-27 ? kRhsTable
+                     : std::fabs(diag - off) <= ulps         ? kRhsSumPlus
+                     : std::fabs(diag) <= ulps               ? kRhsSum
+                                                             : kRhsTable;
     const RhsArgs a{m->n_elem,       p->d_elem_order, p->d_bnode,       p->d_bnode_n, p->d_elem_local,
                     p->d_geo_det,    d_tab + 6 * nu,  d_field,          d_elem_scale, p->d_rhs_bpos,
                     p->d_rhs_bstart, p->d_rhs_bout,   p->d_rhs_partial, d_b,          form,
