@@ -275,7 +275,9 @@ __device__ __forceinline__ float rows_dot_stream(int64_t row0, int64_t n, const 
     __syncwarp();
   }
   const ff t = two_sum(sum.hi, __shfl_xor_sync(0xffffffffu, sum.hi, 1));
-  return __fadd_rn(t.hi, __fadd_rn(t.lo, __fadd_rn(sum.lo, __shfl_xor_sync(0xffffffffu, sum.lo, 1))));
+  const float low = __fadd_rn(t.lo, __fadd_rn(sum.lo, __shfl_xor_sync(0xffffffffu, sum.lo, 1)));
+  // an Inf or NaN sum is the row's value: its errors are NaN
+  return isfinite(t.hi) ? __fadd_rn(t.hi, low) : t.hi;
 }
 
 // Dot-product accumulation: FP64 for FP64 vectors; for FP32 vectors a
