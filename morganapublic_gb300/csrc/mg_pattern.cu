@@ -113,8 +113,10 @@ __global__ void __launch_bounds__(256) k_min_altitude(int64_t E, const int4* __r
 #pragma unroll
     for (int k = 0; k < 4; ++k) big = fmaxf(big, c[k][0] * c[k][0] + c[k][1] * c[k][1] + c[k][2] * c[k][2]);
     const float det = d[0][0] * c[0][0] + d[0][1] * c[0][1] + d[0][2] * c[0][2];
+    // squares below the floats (elements under 2^-37 or so) leave Inf or NaN: zero, as
+    // faces of that size rule out an altitude of 2^-20
     const float alt = fabsf(det) * rsqrtf(big);
-    atomicMin(&mn, alt > 0.0f ? __float_as_uint(alt) : 0u);  // NaN counts as zero
+    atomicMin(&mn, alt > 0.0f && alt < INFINITY ? __float_as_uint(alt) : 0u);
   }
   __syncthreads();
   if (threadIdx.x == 0) atomicMin(min_alt, mn);
