@@ -294,7 +294,7 @@ mg_status mg_assemble_host(mg_plan* plan, int32_t op, const double* h_coeff, dou
 
 /* Load vector b_i = sum_e s_e int_e f_h phi_i (f_h the nodal P1/P2 field d_field,
    or 1 when d_field is NULL; s_e = d_elem_scale[e] or 1 when NULL), written to
-   d_b (ndof doubles).  Element vectors in double-word arithmetic (FP64-accurate
+   d_b (ndof doubles; it may overlap d_field or d_elem_scale).  Element vectors in double-word arithmetic (FP64-accurate
    at any scale of s and f), then one FP64 sum per dof in a fixed order:
    deterministic, no atomics.  The first call on a plan builds the sums' map (P1
    meshes whose 512-element blocks hold at most 256 nodes each: about 14 bytes per

@@ -1995,6 +1995,7 @@ struct RhsArgs {
   const uint16_t* bstart;  // per block kStageNodes + 1 starts
   const int32_t* bout;     // per block kStageNodes outputs: node, or -1 - partial slot
   double *partial, *b;
+  const int32_t* all_partial;  // rhs_ptr where b may overlap an input, else null (rhs_put)
   int form;     // of M^ f
   double unit;  // factor of the sums (1 with the full table), a normal number
 };
@@ -2003,10 +2004,13 @@ struct RhsArgs {
 // full table.  u multiplies the node's sum in FP64.
 enum { kRhsTable = 0, kRhsSumPlus = 1, kRhsSum = 2 };
 
+// Where b overlaps the field or the scale, which other blocks may still read, every sum
+// goes to its partial slot (a node with one has it at rhs_ptr[node]).
 __device__ __forceinline__ void rhs_put(const RhsArgs& a, int32_t out, double v)
 {
-  if (out >= 0) a.b[out] = v;
-  else a.partial[-1 - (int64_t)out] = v;
+  if (out < 0) a.partial[-1 - (int64_t)out] = v;
+  else if (a.all_partial) a.partial[a.all_partial[out]] = v;
+  else a.b[out] = v;
 }
 
 // The block in native FP64 (any scale), with the rules of k_rhs_elem: NaN where s or an f
@@ -2198,16 +2202,17 @@ __global__ void __launch_bounds__(256, 5) k_rhs_block(RhsArgs a)
   }
 }
 
-// One thread per node: the partials of a node with elements in several blocks in
-// ascending block; nodes outside every element get zero.
+// One thread per node: the partials of a node with elements in several blocks (or of
+// every node, where all are partial) in ascending block; nodes outside every element get
+// zero.
 __global__ void __launch_bounds__(256) k_rhs_shared(int64_t n, const int32_t* __restrict__ ptr,
-                                                    const double* partial, double* __restrict__ b)
+                                                    const double* partial, int all_partial, double* __restrict__ b)
 {
   pdl_trigger();
   const int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int q0 = d < n ? __ldg(ptr + d) : 0, q1 = d < n ? __ldg(ptr + d + 1) : 1;
+  const int q0 = d < n ? __ldg(ptr + d) : 0, q1 = d < n ? __ldg(ptr + d + 1) : 0;
   pdl_wait();  // every thread, so that this kernel's end implies the one before's
-  if (q1 - q0 == 1) return;
+  if (d >= n || (q1 - q0 == 1 && !all_partial)) return;
   double v = 0.0;
   for (int q = q0; q < q1; ++q) v += partial[q];
   b[d] = v;
@@ -2398,13 +2403,18 @@ mg_status mg_assemble_rhs(mg_plan* p, const double* d_field, const double* d_ele
                      : std::fabs(diag - off) <= ulps         ? kRhsSumPlus
                      : std::fabs(diag) <= ulps               ? kRhsSum
                                                              : kRhsTable;
+    const auto overlaps = [&](const double* q, int64_t n) {
+      const uintptr_t b0 = reinterpret_cast<uintptr_t>(d_b), q0 = reinterpret_cast<uintptr_t>(q);
+      return q && q0 < b0 + sizeof(double) * (size_t)p->ndof && b0 < q0 + sizeof(double) * (size_t)n;
+    };
+    const bool in_place = overlaps(d_field, p->ndof) || overlaps(d_elem_scale, m->n_elem);
     const RhsArgs a{m->n_elem,       p->d_elem_order, p->d_bnode,       p->d_bnode_n, p->d_elem_local,
                     p->d_geo_det,    d_tab + 6 * nu,  d_field,          d_elem_scale, p->d_rhs_bpos,
-                    p->d_rhs_bstart, p->d_rhs_bout,   p->d_rhs_partial, d_b,          form,
-                    form == kRhsTable ? 1.0 : off};
+                    p->d_rhs_bstart, p->d_rhs_bout,   p->d_rhs_partial, d_b,          in_place ? p->d_rhs_ptr : nullptr,
+                    form,            form == kRhsTable ? 1.0 : off};
     MG_CUDA(launch_pdl(k_rhs_block, (int)p->n_blocks, 256, st, a));
     MG_CUDA(launch_pdl(k_rhs_shared, (int)((p->ndof + 255) / 256), 256, st, p->ndof, (const int32_t*)p->d_rhs_ptr,
-                       (const double*)p->d_rhs_partial, d_b));
+                       (const double*)p->d_rhs_partial, in_place ? 1 : 0, d_b));
     return MG_OK;
   }
   MG_TRY(plan_rhs_map(p));
