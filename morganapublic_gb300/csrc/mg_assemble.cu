@@ -1547,6 +1547,7 @@ static mg_status plan_gather(mg_plan* p)
     const int64_t n = (int64_t)nunique(p->mesh->order) * p->mesh->n_elem;
     MG_CUDA(cudaMalloc(&p->d_em, sizeof(double) * (size_t)(n + 1)));
     MG_CUDA(cudaMemset(static_cast<double*>(p->d_em) + n, 0, sizeof(double)));
+    MG_TRY(legacy_done());
   }
   return MG_OK;
 }
@@ -2241,7 +2242,7 @@ mg_status mg_plan_status(mg_plan* p)
   MG_CUDA(cudaMemcpy(&flags, p->d_counters + 4, sizeof(flags), cudaMemcpyDeviceToHost));
   if (flags) {
     const uint32_t zero = 0u;
-    MG_CUDA(cudaMemcpy(p->d_counters + 4, &zero, sizeof(zero), cudaMemcpyHostToDevice));
+    MG_TRY(copy_to_device(p->d_counters + 4, &zero, sizeof(zero)));
   }
   if (flags & 1u)
     return set_error(MG_ERR_INVALID_ARG, "assembly: the coefficient array holds NaN or Inf (the values are not usable)");

@@ -24,6 +24,22 @@ mg_status cuda_error(cudaError_t e, const char* what);
     if (_e != cudaSuccess) return ::mg::cuda_error(_e, #call); \
   } while (0)
 
+// Waits for what this thread put on the legacy stream: a copy from pageable memory may
+// return when it is staged and a fill at once, and a stream made non-blocking is not
+// ordered after either.
+inline mg_status legacy_done()
+{
+  MG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+  return MG_OK;
+}
+// Host memory to the device, complete for every stream when it returns
+inline mg_status copy_to_device(void* d, const void* h, size_t bytes)
+{
+  if (bytes == 0) return MG_OK;
+  MG_CUDA(cudaMemcpy(d, h, bytes, cudaMemcpyHostToDevice));
+  return legacy_done();
+}
+
 // NVTX range over one C-ABI call (header-only NVTX3: no cost and no library
 // dependency unless a profiler is attached)
 struct NvtxRange {

@@ -546,8 +546,7 @@ template <typename T>
 static mg_status upload(T** d, const std::vector<T>& h)
 {
   MG_CUDA(cudaMalloc(d, sizeof(T) * std::max<size_t>(h.size(), 1)));
-  if (!h.empty()) MG_CUDA(cudaMemcpy(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
-  return MG_OK;
+  return copy_to_device(*d, h.data(), sizeof(T) * h.size());
 }
 
 static void free_device(mg_lagrange* lg)

@@ -137,8 +137,7 @@ template <typename T>
 static mg_status upload(T** dst, const std::vector<T>& src)
 {
   MG_CUDA(cudaMalloc(dst, sizeof(T) * std::max<size_t>(src.size(), 1)));
-  if (!src.empty()) MG_CUDA(cudaMemcpy(*dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice));
-  return MG_OK;
+  return copy_to_device(*dst, src.data(), sizeof(T) * src.size());
 }
 
 mg_status plan_device(mg_plan* p)
@@ -255,7 +254,7 @@ mg_status plan_tables(mg_plan* p, int quad, const RefTables** t, const double** 
   flat.insert(flat.end(), rt.bary.begin(), rt.bary.end());
   double* d = nullptr;
   MG_CUDA(cudaMalloc(&d, sizeof(double) * flat.size()));
-  MG_CUDA(cudaMemcpy(d, flat.data(), sizeof(double) * flat.size(), cudaMemcpyHostToDevice));
+  MG_TRY(copy_to_device(d, flat.data(), sizeof(double) * flat.size()));
   p->tables.push_back(rt);
   p->d_tables.push_back(d);
   *t = &p->tables.back();

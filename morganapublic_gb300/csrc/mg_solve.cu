@@ -1248,10 +1248,10 @@ static mg_status resident_partition(mg_plan* p, const RowPartition** out)
   for (int k = 0; k < ctas; ++k) max_rows = std::max(max_rows, part[k + 1] - part[k]);
   int32_t* d = nullptr;
   MG_CUDA(cudaMalloc(&d, sizeof(int32_t) * part.size()));
-  const cudaError_t e = cudaMemcpy(d, part.data(), sizeof(int32_t) * part.size(), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
+  const mg_status copied = copy_to_device(d, part.data(), sizeof(int32_t) * part.size());
+  if (copied != MG_OK) {
     cudaFree(d);
-    return cuda_error(e, "CG row partition");
+    return copied;
   }
   rp.d_rows = d;
   rp.max_rows = max_rows;
