@@ -1260,7 +1260,7 @@ static mg_status resident_partition(mg_plan* p, const RowPartition** out)
 }
 
 template <typename V, int G, int U, typename I>
-static mg_status resident_launch(mg_plan* p, const RowPartition* part, const V* vals, V* x, CgWork<V>& w, int threads, size_t smem,
+static cudaError_t resident_launch(mg_plan* p, const RowPartition* part, const V* vals, V* x, CgWork<V>& w, int threads, size_t smem,
                                  bool in_smem, unsigned int epoch, cudaStream_t st)
 {
   const auto kernel = k_cg_resident<V, G, U, I>;
@@ -1277,12 +1277,10 @@ static mg_status resident_launch(mg_plan* p, const RowPartition* part, const V* 
   const I* ci;
   if constexpr (sizeof(I) == 2) ci = p->d_coloff;
   else ci = p->d_colind;
-  MG_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const int32_t*)part->d_rows, part->max_rows, (const int32_t*)p->d_rowptr, ci,
-                             vals, w.dinv, x, w.r, w.z, w.p, w.q, in_smem ? 1 : 0, w.gather, epoch, kResidentIters, w.s));
-  return MG_OK;
+  return cudaLaunchKernelEx(&cfg, kernel, (const int32_t*)part->d_rows, part->max_rows, (const int32_t*)p->d_rowptr, ci,
+                            vals, w.dinv, x, w.r, w.z, w.p, w.q, in_smem ? 1 : 0, w.gather, epoch, kResidentIters, w.s);
 }
-// Whether all CTAs of the kernel can be resident at once (else the caller takes the
-// three-kernel iteration).
+// Whether all CTAs of the kernel can be resident at once on the whole device.
 template <typename V, int G, int U, typename I>
 static mg_status resident_fits(int ctas, int threads, size_t smem, bool* fits)
 {
@@ -1295,7 +1293,9 @@ static mg_status resident_fits(int ctas, int threads, size_t smem, bool* fits)
   return MG_OK;
 }
 
-// Runs CG on A (vals) from the state set up by k_cg_start until `done`.
+// Runs CG on A (vals) from the state set up by k_cg_start until `done`: by the resident
+// kernel, or by the three kernels where the system is too large for it or its launch is
+// refused (a process or stream that has a part of the SMs), from the state it is in.
 template <typename V>
 static mg_status cg_iterate(mg_plan* p, const V* vals, V* x, CgWork<V>& w, int G, int nb, int maxit,
                             cudaStream_t st, CgScalars* h_s, unsigned int* epoch)
@@ -1337,9 +1337,15 @@ static mg_status cg_iterate(mg_plan* p, const V* vals, V* x, CgWork<V>& w, int G
   if (resident) {
     for (;;) {
       MG_CUDA(cudaMemsetAsync(w.gather.count, 0, sizeof(unsigned int), st));
+      cudaError_t refused = cudaSuccess;
       MG_TRY(on_kernel([&](auto g, auto i) {
-        return resident_launch<V, decltype(g)::value, U, decltype(i)>(p, part, vals, x, w, threads, smem, in_smem, *epoch, st);
+        refused = resident_launch<V, decltype(g)::value, U, decltype(i)>(p, part, vals, x, w, threads, smem, in_smem, *epoch, st);
+        return MG_OK;
       }));
+      if (refused != cudaSuccess) {
+        cudaGetLastError();  // an error of the context comes up again below
+        break;
+      }
       *epoch += 2 * kResidentIters;
       MG_CUDA(cudaMemcpyAsync(h_s, w.s, sizeof(CgScalars), cudaMemcpyDeviceToHost, st));
       MG_CUDA(cudaStreamSynchronize(st));
