@@ -614,8 +614,9 @@ __global__ void __launch_bounds__(kSolveThreads) k_cg_dir(int64_t n, const V* __
 // epoch: a word is current when its epoch is, with no fence and no reset.  Two
 // sets alternate: a CTA writes its words of the sum after next only when it has the
 // next one's total, which CTA 0 publishes after reading all partials of both.
-// Every wait is bounded (kSpinLimit polls): a CTA that gives up records done = 9
-// and returns, the others follow.
+// Every wait is bounded (spin_limit polls): a CTA that gives up records done = 9 and
+// returns, the others follow; the caller starts again from the x they leave with the
+// three kernels.
 //
 // What bounds it (GB300, P1 64^3, FP64): the FP64 pipe, 22 operations a row or 10 us of
 // an iteration, then the exchanges (~2 us each; every CTA polling every
@@ -623,7 +624,8 @@ __global__ void __launch_bounds__(kSolveThreads) k_cg_dir(int64_t n, const V* __
 // K1..K3 took 39.6 us an iteration there and 24 us at any small size.
 template <typename V> constexpr int kResidentThreads = sizeof(V) == 8 ? 512 : 768;
 constexpr int kResidentIters = 512;  // iterations per launch (the host looks in between)
-constexpr int kSpinLimit = 1 << 21;
+constexpr int kSpinLimit = 1 << 21;  // polls: a second or so
+constexpr int kGaveUp = 9;           // CgScalars::done of a wait that ran out
 constexpr int kMaxResidentCtas = 1024;
 
 // Exchange buffer: 2 sets of 4 words (2 values) per CTA, 2 sets of totals on a line of
@@ -654,9 +656,9 @@ __device__ __forceinline__ void publish(unsigned long long* w, double v, unsigne
 }
 // Waits for NV values published at w; false when the wait ran out.
 template <int NV>
-__device__ __forceinline__ bool receive(const unsigned long long* w, unsigned int epoch, double (&v)[NV])
+__device__ __forceinline__ bool receive(const unsigned long long* w, unsigned int epoch, int spin_limit, double (&v)[NV])
 {
-  for (int spin = 0; spin < kSpinLimit; ++spin) {
+  for (int spin = 0; spin < spin_limit; ++spin) {
     ulonglong2 x[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) x[k] = ld_relaxed2(w + 2 * k);
@@ -683,7 +685,7 @@ __device__ __forceinline__ bool receive(const unsigned long long* w, unsigned in
 // thread c waits for CTA c's partials, its warp k adds the k-th ones in a fixed order.
 template <typename V, int NV>
 __device__ __forceinline__ bool grid_sum(const typename Dot<V>::A (&v)[NV], typename Dot<V>::A* red, double* gat,
-                                         const GatherBuf& gb, unsigned int epoch, double (&total)[NV])
+                                         const GatherBuf& gb, unsigned int epoch, int spin_limit, double (&total)[NV])
 {
   using D = Dot<V>;
   const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, C = gridDim.x;
@@ -718,7 +720,7 @@ __device__ __forceinline__ bool grid_sum(const typename Dot<V>::A (&v)[NV], type
   if (blockIdx.x == 0) {
     for (int c = tid; c < C; c += T) {
       double p[NV];
-      ok = receive<NV>(set + 4 * c, epoch, p) && ok;
+      ok = receive<NV>(set + 4 * c, epoch, spin_limit, p) && ok;
 #pragma unroll
       for (int k = 0; k < NV; ++k) gat[k * C + c] = p[k];
     }
@@ -736,7 +738,7 @@ __device__ __forceinline__ bool grid_sum(const typename Dot<V>::A (&v)[NV], type
     }
   } else if (tid == 0) {
     double p[NV];
-    ok = receive<NV>(result, epoch, p);
+    ok = receive<NV>(result, epoch, spin_limit, p);
 #pragma unroll
     for (int k = 0; k < NV; ++k) gat[NV * C + k] = p[k];
   }
@@ -749,7 +751,7 @@ __device__ __forceinline__ bool grid_sum(const typename Dot<V>::A (&v)[NV], type
 // All CTAs' global writes before the barrier are seen by all CTAs' plain loads after it:
 // one thread's fence releases the CTA's writes, and after the wait drops its stale L1
 // lines.  `target`: the arrivals of all CTAs so far and at this barrier.
-__device__ __forceinline__ bool grid_barrier(const GatherBuf& gb, unsigned int target)
+__device__ __forceinline__ bool grid_barrier(const GatherBuf& gb, unsigned int target, int spin_limit)
 {
   __syncthreads();
   bool ok = true;
@@ -757,12 +759,12 @@ __device__ __forceinline__ bool grid_barrier(const GatherBuf& gb, unsigned int t
     __threadfence();
     asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(gb.count) : "memory");
     int spin = 0;
-    for (; spin < kSpinLimit; ++spin) {
+    for (; spin < spin_limit; ++spin) {
       unsigned int f;
       asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(gb.count) : "memory");
       if ((int)(f - target) >= 0) break;
     }
-    ok = spin < kSpinLimit;
+    ok = spin < spin_limit;
     __threadfence();
   }
   return __syncthreads_and(ok) != 0;
@@ -799,16 +801,17 @@ template <typename V, int G, int U, typename I>
 __global__ void __launch_bounds__(kResidentThreads<V>, 1)
     k_cg_resident(const int32_t* __restrict__ part, int max_rows, const int32_t* __restrict__ rp,
                   const I* __restrict__ ci, const V* __restrict__ val, V* dinv, V* x, V* r, V* z, V* p, V* q_out,
-                  int in_smem, GatherBuf gb, unsigned int epoch, int iters, CgScalars* s)
+                  int in_smem, GatherBuf gb, unsigned int epoch, int iters, CgScalars* s, int spin_limit)
 {
   using D = Dot<V>;
   extern __shared__ __align__(16) unsigned char smem[];
   double* gat = reinterpret_cast<double*>(smem);
   typename D::A* red = reinterpret_cast<typename D::A*>(gat + 2 * gridDim.x + 2);
   int32_t* srp = reinterpret_cast<int32_t*>(red + 2 * blockDim.x + 8);  // the rows' starts
-  if (s->done) return;
-  const int r0 = part[blockIdx.x], rows = part[blockIdx.x + 1] - r0;
   const int tid = threadIdx.x, T = blockDim.x;
+  // one reading for the CTA: another one that gave up may set it meanwhile
+  if (__syncthreads_or(tid == 0 && s->done != 0)) return;
+  const int r0 = part[blockIdx.x], rows = part[blockIdx.x + 1] - r0;
   // the rows' vectors: in shared memory, or where they are
   V *sx = x + r0, *sr = r + r0, *sd = dinv + r0, *sp = p + r0, *sq = q_out + r0;
   if (in_smem) {
@@ -867,7 +870,7 @@ __global__ void __launch_bounds__(kResidentThreads<V>, 1)
       }
     }
     double tot[1];
-    if (!grid_sum<V, 1>(acc, red, gat, gb, ++epoch, tot)) { done = 9; break; }
+    if (!grid_sum<V, 1>(acc, red, gat, gb, ++epoch, spin_limit, tot)) { done = kGaveUp; break; }
     pq = tot[0];
     alpha = rz / pq;
     if (!(pq > 0.0) || !isfinite(alpha)) { done = 2; break; }  // A not SPD on the Krylov space
@@ -884,7 +887,7 @@ __global__ void __launch_bounds__(kResidentThreads<V>, 1)
       D::mac(acc2[1], ri, ri);
     }
     double tot2[2];
-    if (!grid_sum<V, 2>(acc2, red, gat, gb, ++epoch, tot2)) { done = 9; break; }
+    if (!grid_sum<V, 2>(acc2, red, gat, gb, ++epoch, spin_limit, tot2)) { done = kGaveUp; break; }
     rz_prev = rz;
     beta = tot2[0] / rz;
     rz = tot2[0];
@@ -901,7 +904,7 @@ __global__ void __launch_bounds__(kResidentThreads<V>, 1)
       sp[i] = pi;
       p[r0 + i] = pi;
     }
-    if (!grid_barrier(gb, arrivals += gridDim.x)) { done = 9; break; }
+    if (!grid_barrier(gb, arrivals += gridDim.x, spin_limit)) { done = kGaveUp; break; }
   }
   for (int i = tid; i < rows; i += T) {
     if (in_smem) {
@@ -910,7 +913,7 @@ __global__ void __launch_bounds__(kResidentThreads<V>, 1)
     }
     z[r0 + i] = sd[i] * sr[i];
   }
-  if (tid == 0 && (blockIdx.x == 0 || done == 9)) {
+  if (tid == 0 && (blockIdx.x == 0 || done == kGaveUp)) {
     if (blockIdx.x == 0) {
       s->rz = rz;
       s->rz_prev = rz_prev;
@@ -1278,7 +1281,7 @@ static cudaError_t resident_launch(mg_plan* p, const RowPartition* part, const V
   if constexpr (sizeof(I) == 2) ci = p->d_coloff;
   else ci = p->d_colind;
   return cudaLaunchKernelEx(&cfg, kernel, (const int32_t*)part->d_rows, part->max_rows, (const int32_t*)p->d_rowptr, ci,
-                            vals, w.dinv, x, w.r, w.z, w.p, w.q, in_smem ? 1 : 0, w.gather, epoch, kResidentIters, w.s);
+                            vals, w.dinv, x, w.r, w.z, w.p, w.q, in_smem ? 1 : 0, w.gather, epoch, kResidentIters, w.s, kSpinLimit);
 }
 // Whether all CTAs of the kernel can be resident at once on the whole device.
 template <typename V, int G, int U, typename I>
@@ -1296,9 +1299,11 @@ static mg_status resident_fits(int ctas, int threads, size_t smem, bool* fits)
 // Runs CG on A (vals) from the state set up by k_cg_start until `done`: by the resident
 // kernel, or by the three kernels where the system is too large for it or its launch is
 // refused (a process or stream that has a part of the SMs), from the state it is in.
+// *try_resident: whether the kernel may be tried; false after a wait of it ran out, done is
+// kGaveUp then and x holds every row's value of one of the iterations.
 template <typename V>
 static mg_status cg_iterate(mg_plan* p, const V* vals, V* x, CgWork<V>& w, int G, int nb, int maxit,
-                            cudaStream_t st, CgScalars* h_s, unsigned int* epoch)
+                            cudaStream_t st, CgScalars* h_s, unsigned int* epoch, bool* try_resident)
 {
   const int64_t n = p->ndof;
   const int vb = vec_blocks<V>(n);
@@ -1309,7 +1314,7 @@ static mg_status cg_iterate(mg_plan* p, const V* vals, V* x, CgWork<V>& w, int G
   MG_CUDA(cudaStreamIsCapturing(st, &cs));
   constexpr int U = CgShape<V>::U;
   const int64_t bytes = p->nnz * (int64_t)(sizeof(V) + (p->d_coloff ? 2 : 4)) + 6 * n * (int64_t)sizeof(V);
-  bool resident = bytes <= kResidentBytes && cs == cudaStreamCaptureStatusNone;
+  bool resident = *try_resident && bytes <= kResidentBytes && cs == cudaStreamCaptureStatusNone;
   const RowPartition* part = nullptr;
   int threads = 0;
   bool in_smem = false;
@@ -1349,7 +1354,7 @@ static mg_status cg_iterate(mg_plan* p, const V* vals, V* x, CgWork<V>& w, int G
       *epoch += 2 * kResidentIters;
       MG_CUDA(cudaMemcpyAsync(h_s, w.s, sizeof(CgScalars), cudaMemcpyDeviceToHost, st));
       MG_CUDA(cudaStreamSynchronize(st));
-      if (h_s->done == 9) return set_error(MG_ERR_CUDA, "CG: a wait between the kernel's CTAs ran out");
+      if (h_s->done == kGaveUp) *try_resident = false;
       if (h_s->done) return MG_OK;
     }
   }
@@ -1553,9 +1558,16 @@ mg_status mg_cg_solve(mg_plan* p, const double* d_values, const double* d_b, dou
   MG_CUDA(cudaEventCreate(&e1));
   MG_CUDA(cudaEventRecord(e0, st));
   CgScalars* hs = reinterpret_cast<CgScalars*>(p->h_pinned);
-  mg_status s = cg_start<double>(p, d_values, d_b, d_x, 0, precond == MG_PREC_JACOBI, rtol, maxit, w, G, nb, st);
-  unsigned int epoch = 0;
-  if (s == MG_OK) s = cg_iterate<double>(p, d_values, d_x, w, G, nb, maxit, st, hs, &epoch);
+  mg_status s = MG_OK;
+  int before = 0;  // iterations of a resident kernel that gave up
+  bool try_resident = true;
+  for (;;) {
+    s = cg_start<double>(p, d_values, d_b, d_x, 0, precond == MG_PREC_JACOBI, rtol, maxit - before, w, G, nb, st);
+    unsigned int epoch = 0;
+    if (s == MG_OK) s = cg_iterate<double>(p, d_values, d_x, w, G, nb, maxit - before, st, hs, &epoch, &try_resident);
+    if (s != MG_OK || hs->done != kGaveUp) break;
+    before += hs->iter;
+  }
   MG_CUDA(cudaEventRecord(e1, st));
   MG_CUDA(cudaEventSynchronize(e1));
   float ms = 0.f;
@@ -1565,7 +1577,7 @@ mg_status mg_cg_solve(mg_plan* p, const double* d_values, const double* d_b, dou
   if (s != MG_OK) return s;
   MG_CUDA(cudaMemcpy(hs, w.s, sizeof(CgScalars), cudaMemcpyDeviceToHost));
   if (info) {
-    info->iterations = hs->iter;
+    info->iterations = before + hs->iter;
     info->outer_iterations = 0;
     info->converged = hs->done == 1;
     info->rel_residual = rel_residual(hs->rr, hs->bb);
@@ -1607,7 +1619,7 @@ mg_status mg_cg_refined(mg_plan* p, const double* d_values64, const float* d_val
   MG_CUDA(cudaEventRecord(e0, st));
   int anchors = 0, inner = 0;
   unsigned int epoch = 0;
-  bool converged = false;
+  bool converged = false, try_resident = true;
   double relres = INFINITY, bb64 = 1.0;
   mg_status s = MG_OK;
   // FP64 residual of the current x (into r64, s64->rr, s64->bb)
@@ -1643,21 +1655,23 @@ mg_status mg_cg_refined(mg_plan* p, const double* d_values64, const float* d_val
       MG_CUDA(cudaMemcpyAsync(w.s, hs, sizeof(CgScalars), cudaMemcpyHostToDevice, st));
     }
     while (s == MG_OK) {
-      s = cg_iterate<float>(p, d_values32, x32, w, G, nb, max_inner, st, hs, &epoch);
+      s = cg_iterate<float>(p, d_values32, x32, w, G, nb, max_inner, st, hs, &epoch, &try_resident);
       if (s != MG_OK) break;
       inner = hs->iter;
       const int why = hs->done;
       if (why == 2) { s = set_error(MG_ERR_NOT_CONVERGED, "refined CG breakdown: p.Ap <= 0"); break; }
       // anchor: x += x32, r64 = b - A64 x
       k_anchor_x<<<eb, 256, 0, st>>>(n, d_x, x32);
-      ++anchors;
+      if (why != kGaveUp) ++anchors;
       s = residual64();
       if (s != MG_OK) break;
       if (relres <= rtol) { converged = true; break; }
       if (why == 3 || anchors >= max_outer) break;
-      // replace the FP32 residual, keep the direction, resume
+      // replace the FP32 residual, keep the direction, resume; after a wait that ran out the
+      // direction is of no one iteration, and z takes its place
       k_anchor_r<<<eb, kSolveThreads, 0, st>>>(n, r64, w.r, w.z, w.dinv, w.partials, w.s);
-      launch_k(false, k_cg_dir<float>, eb, kSolveThreads, st, n, (const float*)w.z, w.p, (const CgScalars*)w.s);
+      if (why == kGaveUp) MG_CUDA(cudaMemcpyAsync(w.p, w.z, sizeof(float) * (size_t)n, cudaMemcpyDeviceToDevice, st));
+      else launch_k(false, k_cg_dir<float>, eb, kSolveThreads, st, n, (const float*)w.z, w.p, (const CgScalars*)w.s);
       MG_CUDA(cudaGetLastError());
     }
   }

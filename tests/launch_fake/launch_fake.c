@@ -1,5 +1,6 @@
-/* Preloaded before libcudart: cooperative launches are refused, all of them or all
-   after the first, as the runtime refuses a grid that cannot be resident. */
+/* Preloaded before libcudart: cooperative launches are refused as the runtime refuses a
+   grid that cannot be resident, or run with another limit on the polls of their waits
+   (the resident CG's last argument); all of them, or all after the first. */
 #define _GNU_SOURCE
 #include <dlfcn.h>
 #include <stdlib.h>
@@ -19,12 +20,19 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* fu
     real = (launch_t)dlsym(rt ? rt : RTLD_NEXT, "cudaLaunchKernelExC");
     if (!real) abort();
   }
-  const char* mode = getenv("FAKE_LAUNCH");
+  const char *mode = getenv("FAKE_LAUNCH"), *spins = getenv("FAKE_SPINS");
   for (unsigned int i = 0; i < config->numAttrs; ++i)
     if (config->attrs[i].id == cudaLaunchAttributeCooperative && config->attrs[i].val.cooperative) {
       ++cooperative_launches;
-      if (mode && (!strcmp(mode, "refuse") || (!strcmp(mode, "refuse_later") && cooperative_launches > 1)))
-        return cudaErrorCooperativeLaunchTooLarge;
+      const int now = mode && (!strstr(mode, "later") || cooperative_launches > 1);
+      if (now && !strncmp(mode, "refuse", 6)) return cudaErrorCooperativeLaunchTooLarge;
+      if (now && !strncmp(mode, "give_up", 7)) {
+        int limit = spins ? atoi(spins) : 0;
+        void* a[17];
+        memcpy(a, args, sizeof(a));
+        a[16] = &limit;
+        return real(config, func, a);
+      }
     }
   return real(config, func, args);
 }

@@ -1,6 +1,6 @@
 """CG where the resident kernel does not run to its end: a fake of the launch call,
-preloaded into a child process, refuses it, at once or when it is launched again; the
-solve goes on with the three kernels."""
+preloaded into a child process, refuses it, or lets its waits run out after a few polls,
+at once or when it is launched again; the solve goes on with the three kernels."""
 import os
 import subprocess
 import sys
@@ -31,7 +31,7 @@ for n, order, sigma, precond in ((6, 1, 1.0, "jacobi"), (9, 2, 1.0, None), (14, 
     assert fake.fake_cooperative_launches() > 0
     assert info.converged and info.rel_residual <= 1e-11
     assert float((rhs - b.apply(A, x)).norm() / rhs.norm()) <= 1e-10
-    if mode == "refuse":
+    if mode in ("refuse", "give_up:0"):  # nothing was done before
         assert torch.equal(x, y) and info.iterations == ref.iterations
     else:
         assert abs(info.iterations - ref.iterations) <= 2 + ref.iterations // 20
@@ -62,7 +62,7 @@ def fake(tmp_path_factory):
 
 
 def _run(fake, mode):
-    env = dict(os.environ, LD_PRELOAD=fake, FAKE_LAUNCH=mode)
+    env = dict(os.environ, LD_PRELOAD=fake, FAKE_LAUNCH=mode.split(":")[0], FAKE_SPINS=mode.split(":")[-1])
     r = subprocess.run([sys.executable, "-c", CHILD.format(root=ROOT, here=HERE, mode=mode)], env=env, text=True,
                        stdout=subprocess.PIPE, stderr=subprocess.STDOUT, timeout=300)
     assert r.returncode == 0 and "fallback ok" in r.stdout, r.stdout[-3000:]
@@ -70,4 +70,9 @@ def _run(fake, mode):
 
 @pytest.mark.parametrize("mode", ["refuse", "refuse_later"])
 def test_refused_launch(fake, mode):
+    _run(fake, mode)
+
+
+@pytest.mark.parametrize("mode", ["give_up:0", "give_up:1", "give_up:6", "give_up:50", "give_up_later:0", "give_up_later:20"])
+def test_wait_ran_out(fake, mode):
     _run(fake, mode)
