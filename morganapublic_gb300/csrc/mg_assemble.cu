@@ -1980,7 +1980,7 @@ __global__ void __launch_bounds__(256) k_rhs_gather(int64_t ndof, const int32_t*
 // f (converted once per node), s and det are scaled by the powers of two of their largest
 // values in the block; where their spreads together exceed 2^70, a value is Inf, NaN or
 // subnormal, or a determinant is 2^127 or more (its inverse power would be
-// subnormal), the block runs in FP64 (rhs_block_f64).
+// subnormal), every element takes its own (rhs_block_wide).
 // The two passes wrote and gathered 32 bytes per element through memory and issued 21
 // warp instructions per element, a third of them conversions: GB300, P1 96^3, 217 ->
 // 141 us (block kernel 126, shared nodes 14; bound by issue and the L1 data path, 61 %
@@ -2014,46 +2014,119 @@ __device__ __forceinline__ void rhs_put(const RhsArgs& a, int32_t out, double v)
   else a.b[out] = v;
 }
 
-// The block in native FP64 (any scale), with the rules of k_rhs_elem: NaN where s or an f
-// of the element is Inf or NaN, zero where s or all f are zero or subnormal.
-static __device__ __noinline__ void rhs_block_f64(const RhsArgs& a, double* y, const uint16_t* s_pos, const uint16_t* s_start,
-                                                  int n_nodes, int32_t out)
+// (M^ f)_l s det of a pair, without the unit, in the form's arithmetic
+__device__ __forceinline__ void rhs_pair(int form, const ff* tab, const ff2 (&F)[4], ff2 sd, ff2 (&v)[4])
 {
+  const auto add = [](ff2 x, ff2 z) {
+    const ff2 t = f2_two_sum(x.hi, z.hi);
+    return f2_fast_two_sum(t.hi, t.lo + (x.lo + z.lo));
+  };
+  const auto dup = [](ff t) { return ff2_make(t, t); };
+  if (form != kRhsTable) {
+    const ff2 x = f2_two_sum(F[0].hi, F[1].hi), z = f2_two_sum(F[2].hi, F[3].hi), w = f2_two_sum(x.hi, z.hi);
+    const f2 slo = ((F[0].lo + F[1].lo) + (F[2].lo + F[3].lo)) + ((x.lo + z.lo) + w.lo);
+    const ff2 one = ff2_mul(f2_fast_two_sum(w.hi, slo), sd);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const ff2 t = f2_two_sum(w.hi, F[l].hi);
+      v[l] = form == kRhsSum ? one : ff2_mul(f2_fast_two_sum(t.hi, slo + (t.lo + F[l].lo)), sd);
+    }
+  } else {
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      ff2 t = ff2_mul(dup(tab[sym_index(l, 0, 4)]), F[0]);
+#pragma unroll
+      for (int k = 1; k < 4; ++k) t = add(t, ff2_mul(dup(tab[sym_index(l, k, 4)]), F[k]));
+      v[l] = ff2_mul(t, sd);
+    }
+  }
+}
+
+// One element's share of rhs_block_wide: s and f near one, the power of two that was taken
+// out (with the determinant's, 0 or 64, apart), and whether the vector is NaN (s or an f
+// Inf or NaN) or zero (s, or all f, zero or subnormal), the rules of k_rhs_elem.
+struct RhsElement {
+  ff F[4], s, det;
+  int k, kdet;
+  bool nan, zero;
+};
+__device__ __forceinline__ RhsElement rhs_element(const double* f, uchar4 q, double s, float2 d)
+{
+  RhsElement e;
+  const double v[4] = {f[q.x], f[q.y], f[q.z], f[q.w]};
+  const int es = dexp(s), ef = max(max(dexp(v[0]), dexp(v[1])), max(dexp(v[2]), dexp(v[3])));
+  e.nan = es == 0x7ff || ef == 0x7ff;
+  e.zero = es == 0 || ef == 0;
+  e.k = (es - 1023) + (ef - 1023);
+  e.kdet = fabsf(d.x) >= 0x1p64f ? 64 : 0;  // products with a larger one may overflow
+  const float dscale = e.kdet ? 0x1p-64f : 1.0f;
+  e.det = ff{d.x * dscale, d.y * dscale};
+  if (e.nan || e.zero) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) e.F[k] = ff{0.0f, 0.0f};
+    e.s = ff{0.0f, 0.0f};
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      // (subnormal, and not 2^-74 of the largest: its exponent is no power of two to take out)
+      e.F[k] = dexp(v[k]) == 0 && ef <= 74 ? ff_from_double(scale_pow2(v[k], 1023 - ef)) : ff_rescaled<true>(v[k], ef);
+    e.s = ff_rescaled<true>(s, es);
+  }
+  return e;
+}
+__device__ __forceinline__ double rhs_value(const RhsElement& e, ff v)
+{
+  if (e.nan) return __longlong_as_double(0x7ff8000000000000ll);
+  const double x = ff_to_double_bits(v);
+  // in the normal range the powers go into the exponent, off the FP64 pipe
+  const int ex = dexp(x), k = e.k + e.kdet;
+  if (ex == 0 || ex == 0x7ff) return x;
+  if (ex + k >= 1 && ex + k <= 2046) return __longlong_as_double(__double_as_longlong(x) + ((long long)k << 52));
+  return scale_pow2(x * (e.kdet ? 0x1p64 : 1.0), e.k);
+}
+
+// Shared memory of a block
+struct RhsShared {
+  __align__(16) float y[8 * kElemBlock];       // element vectors: high parts, low parts (or doubles)
+  __align__(16) float f[2 * kStageNodes];      // the nodes' f: high parts, low parts (or doubles)
+  __align__(16) uint16_t pos[4 * kElemBlock];
+  uint16_t start[kStageNodes + 1];
+  ff tab[10];
+  int red[6][8];
+};
+
+// A block whose values spread too far for one scale: s and f of every element by their own
+// powers of two, as k_rhs_elem takes them, and the element vectors as doubles.  GB300,
+// P1 96^3, every block of this kind: 210 us, 727 with the block in native FP64 (the
+// two-pass form: 216; two FP64 products per entry for its power of two: 228).
+static __device__ __noinline__ void rhs_block_wide(const RhsArgs& a, RhsShared& sh, int n_nodes, int32_t out)
+{
+  double *y = reinterpret_cast<double*>(sh.y), *s_f = reinterpret_cast<double*>(sh.f);
+  // everything is read again, so that the common path holds nothing for this one
   const int64_t p0 = (int64_t)blockIdx.x * kElemBlock;
-  const int32_t* id = a.bnode + (int64_t)blockIdx.x * kStageNodes;
-  for (int lp = threadIdx.x; lp < kElemBlock; lp += blockDim.x) {
-    const int64_t p = p0 + lp;
-    if (p >= a.n_elem) break;
-    const uchar4 l4 = a.elem_local[p];
-    const int l[4] = {l4.x, l4.y, l4.z, l4.w};
-    const double s = a.scale ? a.scale[a.elem_order[p]] : 1.0;
-    double f[4] = {1.0, 1.0, 1.0, 1.0};
-    int ef = 0;
-    for (int k = 0; k < 4; ++k) {
-      if (a.field) f[k] = a.field[id[l[k]]];
-      ef = max(ef, dexp(f[k]));
-    }
-    const int es = dexp(s);
-    const float2 d = a.gdet[p];
-    // s and f near one, scaled back at the end: the products stay inside the range
-    const bool dead = es == 0x7ff || ef == 0x7ff || es == 0 || ef == 0;
-    const double sd = dead ? 0.0 : scale_pow2(s, 1023 - es) * ((double)d.x + (double)d.y);
-    for (int i = 0; i < 4; ++i) {
-      double v = 0.0;
-      if (!dead) {
-        for (int k = 0; k < 4; ++k) v += a.mass[sym_index(i, k, 4)] * scale_pow2(f[k], 1023 - ef);
-        v = scale_pow2(v * sd, (es - 1023) + (ef - 1023));
-      } else if (es == 0x7ff || ef == 0x7ff) {
-        v = __longlong_as_double(0x7ff8000000000000ll);
-      }
-      y[i * kElemBlock + lp] = v;
-    }
+  const int lp = threadIdx.x + (threadIdx.x & ~31);
+  const int64_t p1 = min(p0 + lp, a.n_elem - 1), p2 = min(p0 + lp + 32, a.n_elem - 1);
+  s_f[threadIdx.x] = a.field ? a.field[a.bnode[(int64_t)blockIdx.x * kStageNodes + threadIdx.x]] : 1.0;
+  __syncthreads();
+  const RhsElement e1 = rhs_element(s_f, a.elem_local[p1], a.scale ? a.scale[a.elem_order[p1]] : 1.0, a.gdet[p1]);
+  const RhsElement e2 = rhs_element(s_f, a.elem_local[p2], a.scale ? a.scale[a.elem_order[p2]] : 1.0, a.gdet[p2]);
+  ff2 F[4], v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) F[k] = ff2_make(e1.F[k], e2.F[k]);
+  rhs_pair(a.form, sh.tab, F, ff2_mul(ff2_make(e1.s, e2.s), ff2_make(e1.det, e2.det)), v);
+  const ff u = ff_from_double_bits(a.unit);
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    const ff2 w = ff2_mul(v[l], ff2_make(u, u));
+    const float2 h = f2_get(w.hi), lo = f2_get(w.lo);
+    y[l * kElemBlock + lp] = rhs_value(e1, ff{h.x, lo.x});
+    y[l * kElemBlock + lp + 32] = rhs_value(e2, ff{h.y, lo.y});
   }
   __syncthreads();
   if ((int)threadIdx.x < n_nodes) {
-    double v = 0.0;
-    for (int j = s_start[threadIdx.x]; j < s_start[threadIdx.x + 1]; ++j) v += y[s_pos[j] / 4];
-    rhs_put(a, out, v);
+    double sum = 0.0;
+    for (int j = sh.start[threadIdx.x]; j < sh.start[threadIdx.x + 1]; ++j) sum += y[sh.pos[j] / 4];
+    rhs_put(a, out, sum);
   }
 }
 
@@ -2082,12 +2155,11 @@ struct NodeSum {
 __global__ void __launch_bounds__(256, 5) k_rhs_block(RhsArgs a)
 {
   constexpr int Y = 4 * kElemBlock;
-  __shared__ __align__(16) float y[2 * Y];  // element vectors: high parts, low parts (or doubles)
-  __shared__ float s_fh[kStageNodes], s_fl[kStageNodes];
-  __shared__ __align__(16) uint16_t s_pos[Y];
-  __shared__ uint16_t s_start[kStageNodes + 1];
-  __shared__ ff tab[10];
-  __shared__ int red[6][8];
+  __shared__ RhsShared sh;
+  float *const y = sh.y, *const s_fh = sh.f, *const s_fl = sh.f + kStageNodes;
+  uint16_t *const s_pos = sh.pos, *const s_start = sh.start;
+  ff* const tab = sh.tab;
+  int(&red)[6][8] = sh.red;
   const int tid = threadIdx.x, lane = tid & 31, lp = tid + (tid & ~31);
   const int64_t blk = blockIdx.x, p0 = blk * kElemBlock, E = a.n_elem;
   const int64_t p1 = min(p0 + lp, E - 1), p2 = min(p0 + lp + 32, E - 1);  // past the end: the last element again
@@ -2137,7 +2209,7 @@ __global__ void __launch_bounds__(256, 5) k_rhs_block(RhsArgs a)
   // (all zero: the largest is 0 and the smallest 0x7ff)
   const int spread = (ef > 0 ? ef - lf : 0) + (es > 0 ? es - ls : 0) + (ed - ld);
   if (ef == 0x7ff || es == 0x7ff || lf == 0 || ls == 0 || ed >= 0xfe || ld == 0 || spread > 70) {
-    rhs_block_f64(a, reinterpret_cast<double*>(y), s_pos, s_start, n_nodes, out);
+    rhs_block_wide(a, sh, n_nodes, out);
     return;
   }
   {
@@ -2156,30 +2228,8 @@ __global__ void __launch_bounds__(256, 5) k_rhs_block(RhsArgs a)
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       F[k] = ff2{f2_make(s_fh[i1[k]], s_fh[i2[k]]), f2_make(s_fl[i1[k]], s_fl[i2[k]])};
-    const auto add = [](ff2 x, ff2 z) {
-      const ff2 t = f2_two_sum(x.hi, z.hi);
-      return f2_fast_two_sum(t.hi, t.lo + (x.lo + z.lo));
-    };
-    const auto dup = [](ff t) { return ff2_make(t, t); };
     ff2 v[4];
-    if (a.form != kRhsTable) {
-      const ff2 x = f2_two_sum(F[0].hi, F[1].hi), z = f2_two_sum(F[2].hi, F[3].hi), w = f2_two_sum(x.hi, z.hi);
-      const f2 slo = ((F[0].lo + F[1].lo) + (F[2].lo + F[3].lo)) + ((x.lo + z.lo) + w.lo);
-      const ff2 one = ff2_mul(f2_fast_two_sum(w.hi, slo), sd);
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        const ff2 t = f2_two_sum(w.hi, F[l].hi);
-        v[l] = a.form == kRhsSum ? one : ff2_mul(f2_fast_two_sum(t.hi, slo + (t.lo + F[l].lo)), sd);
-      }
-    } else {
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        ff2 t = ff2_mul(dup(tab[sym_index(l, 0, 4)]), F[0]);
-#pragma unroll
-        for (int k = 1; k < 4; ++k) t = add(t, ff2_mul(dup(tab[sym_index(l, k, 4)]), F[k]));
-        v[l] = ff2_mul(t, sd);
-      }
-    }
+    rhs_pair(a.form, tab, F, sd, v);
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
       em_pair(y, l, lp, v[l].hi);
