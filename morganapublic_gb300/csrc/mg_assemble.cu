@@ -440,8 +440,12 @@ struct ElemArgs {
   const double* coeff;        // per element in the caller's order, or null
   double cconst;              // used when coeff is null
   const double* tables;       // unique-entry tables: stiff[6][nu], mass[nu], P2: bary[kBaryTerms]
-  double wsum;
+  double wsum;                // times 2^g, see len_scale
   float w_hi, w_lo;           // wsum as a double-word
+  // the element kernels see the mesh times 2^-g (mg_mesh::geo_exp): a stiffness is 2^g of
+  // theirs, in wsum (P1) and len_scale (P2), a mass 2^(3g), in two factors
+  float len_scale, vol_scale1, vol_scale2;
+  float sc_min, sc_max;       // the double-word range of coefficient times determinant
   int stiff;
   void* em;                   // out: nu x n_elem entries
   uint32_t* flags;            // bit 0: NaN / Inf coefficient; bit 1: outside the double-word range
@@ -650,6 +654,20 @@ __device__ __forceinline__ ff2 pair_quotient(f2 nh, f2 nl, ff2 det)
   return f2_fast_two_sum(q1, q2 + q3);
 }
 
+// Coefficient times determinant of a pair, from the kernels' scale to the mesh's;
+// double-words outside their range are recorded.
+__device__ __forceinline__ f2 true_volume(const ElemArgs& a, f2 v)
+{
+  return v * f2_make(a.vol_scale1, a.vol_scale1) * f2_make(a.vol_scale2, a.vol_scale2);
+}
+__device__ __forceinline__ ff2 true_volume(const ElemArgs& a, ff2 v)
+{
+  const float2 h = f2_get(v.hi);
+  const auto ok = [&](float x) { return x == 0.0f || (fabsf(x) >= a.sc_min && fabsf(x) < a.sc_max); };
+  if (!ok(h.x) || !ok(h.y)) atomicOr(a.flags, 2u);
+  return ff2{true_volume(a, v.hi), true_volume(a, v.lo)};
+}
+
 // From the pair's edges J and coefficients; node(e): the global vertex ids of
 // element e of the pair (for the rare paths).
 template <typename Node>
@@ -735,9 +753,7 @@ __device__ __forceinline__ void p1_pair_dw(const ElemArgs& a, const ff* mass, co
     }
     const f2 nc = -coef.hi, p = coef.hi * det.hi;
     const f2 lo = fma2(coef.hi, det.lo, coef.lo * det.hi);
-    const ff2 sc = f2_fast_two_sum(p, lo - fma2(nc, det.hi, p));
-    const float2 sh = f2_get(sc.hi);
-    if (!dw_scale_ok(sh.x) || !dw_scale_ok(sh.y)) atomicOr(a.flags, 2u);
+    const ff2 sc = true_volume(a, f2_fast_two_sum(p, lo - fma2(nc, det.hi, p)));
     const f2 ns = -sc.hi;
 #pragma unroll
     for (int u = 0; u < 10; ++u) {
@@ -834,7 +850,7 @@ __device__ __forceinline__ void p1_pair_f32(const ElemArgs& a, const float* mass
       det = f2_make(degen0 ? abs_geometry_fp64<float>(a.geo.xyz, node(0)).det : d.x,
                     degen1 ? abs_geometry_fp64<float>(a.geo.xyz, node(1)).det : d.y);
     }
-    const f2 sc = coef * det;
+    const f2 sc = true_volume(a, coef * det);
 #pragma unroll
     for (int u = 0; u < 10; ++u) em_pair(em, u, lp, sc * f2_make(mass[u], mass[u]));
   }
@@ -1014,6 +1030,8 @@ __global__ void __launch_bounds__(128, 4) k_elem_mat_pair(ElemArgs a)
         const float2 dl = f2_get(f.det.lo), ch = f2_get(coef.hi), cl = f2_get(coef.lo);
         s = ff2_make(ff_div(ff{ch.x, cl.x}, ff{dh.x, dl.x}), ff_div(ff{ch.y, cl.y}, ff{dh.y, dl.y}));
       }
+      const f2 ls = f2_make(a.len_scale, a.len_scale);
+      s = ff2{s.hi * ls, s.lo * ls};
       ff2 g[10];
       f2 nC[3][3];
 #pragma unroll
@@ -1038,9 +1056,7 @@ __global__ void __launch_bounds__(128, 4) k_elem_mat_pair(ElemArgs a)
       for (int i = 0; i < 10; ++i) ng[i] = -g[i].hi;
       p2_stiffness(g, ng, tab, a.em, E, p0, p1);
     } else {
-      const ff2 sc = ff2_mul(coef, f.det);
-      const float2 sh = f2_get(sc.hi);
-      if (!dw_scale_ok(sh.x) || !dw_scale_ok(sh.y)) atomicOr(a.flags, 2u);
+      const ff2 sc = true_volume(a, ff2_mul(coef, f.det));
       const f2 ns = -sc.hi;
 #pragma unroll 5
       for (int u = 0; u < NU; ++u) {
@@ -1069,7 +1085,7 @@ __global__ void __launch_bounds__(128, 4) k_elem_mat_pair(ElemArgs a)
     const f2 coef = f2_make(A::from(c0), A::from(c1));
     if (a.stiff) {
       const float2 dh = f2_get(det), ch = f2_get(coef);
-      const f2 s = f2_make(ch.x / dh.x, ch.y / dh.y);
+      const f2 s = f2_make(ch.x / dh.x, ch.y / dh.y) * f2_make(a.len_scale, a.len_scale);
       f2 g[10];
 #pragma unroll
       for (int k = 0; k < 4; ++k)
@@ -1078,7 +1094,7 @@ __global__ void __launch_bounds__(128, 4) k_elem_mat_pair(ElemArgs a)
           g[g_index(k, l)] = s * fma2(C[k][2], C[l][2], fma2(C[k][1], C[l][1], C[k][0] * C[l][0]));
       p2_stiffness(g, g, tab, a.em, E, p0, p1);
     } else {
-      const f2 sc = coef * det;
+      const f2 sc = true_volume(a, coef * det);
 #pragma unroll 5
       for (int u = 0; u < NU; ++u) em_pair_put(a.em, E, u, p0, p1, sc * f2_make(tab[u].x, tab[u].y));
     }
@@ -1586,13 +1602,19 @@ static mg_status launch_assemble_gather(mg_plan* p, int op, const double* d_coef
   a.n_elem = m->n_elem;
   a.elem_order = p->d_elem_order;
   a.dofs_m = p->d_dofs_morton;
-  a.geo = GeoPtrs{m->d_xyz, m->d_node_rec, m->d_lo_z};
+  const int ge = prec == MG_F64_NATIVE ? 0 : m->geo_exp;  // native FP64 reads the coordinates as they are
+  a.geo = GeoPtrs{ge ? m->d_xyz_rec : m->d_xyz, m->d_node_rec, m->d_lo_z};
   a.coeff = needs_coeff ? d_coeff : nullptr;
   a.cconst = op == MG_OP_STIFF_CONST ? c : 1.0;
   a.tables = d_tab;
-  a.wsum = t->wsum;
-  a.w_hi = (float)t->wsum;
-  a.w_lo = (float)(t->wsum - (double)a.w_hi);
+  a.wsum = std::ldexp(t->wsum, ge);
+  a.w_hi = (float)a.wsum;
+  a.w_lo = (float)(a.wsum - (double)a.w_hi);
+  a.len_scale = std::ldexp(1.0f, ge);
+  a.vol_scale1 = std::ldexp(1.0f, 3 * ge / 2);
+  a.vol_scale2 = std::ldexp(1.0f, 3 * ge - 3 * ge / 2);
+  a.sc_min = std::ldexp(1.0f, -96 - 3 * ge);
+  a.sc_max = std::ldexp(1.0f, 113 - 3 * ge);
   a.stiff = (op == MG_OP_STIFF_KAPPA || op == MG_OP_STIFF_CONST);
   a.em = p->d_em;
   a.flags = p->d_counters + 4;
@@ -1748,7 +1770,8 @@ __device__ __forceinline__ void cached_geometry(const float2* det, const float2*
 
 // Elements are visited along a Morton curve of their centroids (elem_order,
 // dofs_m = their dofs in that order), so neighbouring threads gather
-// neighbouring dof values.
+// neighbouring dof values.  factor: 2^g of the geometry cache's scale (mg_mesh::geo_exp),
+// for P1 times the card's weights.
 // P1 is bound by instruction issue: dot products with one renormalisation each (instead of
 // one per operation) and five CTAs per SM took it from 52 to 45 us at P1 64^3 on GB300 (4:
 // 49, 6: 47.5), no table staged and the plan read before the wait to 41.4.  Two elements per thread as packed pairs measured 59 to 68 us, and the
@@ -1756,7 +1779,7 @@ __device__ __forceinline__ void cached_geometry(const float2* det, const float2*
 template <int ORDER>
 __global__ void __launch_bounds__(256, ORDER == 1 ? 5 : 1) k_adjoint(int64_t n_elem, const int32_t* elem_order, const int32_t* dofs_m,
                                                  const float2* gdet, const float2* gcof, const double* tables,
-                                                 double wsum, const double* u, const double* lam, double* grad)
+                                                 double factor, const double* u, const double* lam, double* grad)
 {
   constexpr int NB = ORDER == 1 ? 4 : 10, NU = ORDER == 1 ? 10 : 55;
   __shared__ ff tab[ORDER == 1 ? 1 : 6 * NU];  // P1 takes the zero row sums, no table
@@ -1803,7 +1826,7 @@ __global__ void __launch_bounds__(256, ORDER == 1 ? 5 : 1) k_adjoint(int64_t n_e
   cached_geometry(gdet, gcof, n_elem, i, f);
   ff s = ff_make(0.0f);
   if (ORDER == 1) {
-    // lambda^T K u = (wsum / det) (sum_b dl_b C_b) . (sum_b du_b C_b), C_b the cofactor columns
+    // lambda^T K u = (factor / det) (sum_b dl_b C_b) . (sum_b du_b C_b), C_b the cofactor columns
     // (one renormalisation per dot product instead of one per operation)
     ff gu[3], gl[3], a[3], c[3];
 #pragma unroll
@@ -1816,7 +1839,7 @@ __global__ void __launch_bounds__(256, ORDER == 1 ? 5 : 1) k_adjoint(int64_t n_e
       gu[r] = ff_dot3(a, f.c[r]);
       gl[r] = ff_dot3(c, f.c[r]);
     }
-    s = ff_dot3(gl, gu) * (ff_from_double_bits(wsum) / f.det);
+    s = ff_dot3(gl, gu) * (ff_from_double_bits(factor) / f.det);
   } else {
     ff ue[NB - 1], le[NB - 1];
 #pragma unroll
@@ -1825,7 +1848,7 @@ __global__ void __launch_bounds__(256, ORDER == 1 ? 5 : 1) k_adjoint(int64_t n_e
       le[k] = ff_rescaled<false>(dl[k], el);
     }
     ff g[6];
-    metric<ff>(f, ff_make(1.0f) / f.det, g);
+    metric<ff>(f, ff_make((float)factor) / f.det, g);
 #pragma unroll
     for (int a = 1; a < NB; ++a) {
       ff row = ff_make(0.0f);
@@ -1868,7 +1891,7 @@ __device__ __forceinline__ ff ff_scaled(double v, int emax)
 template <int ORDER>
 __global__ void __launch_bounds__(256) k_rhs_elem(int64_t n_elem, const int32_t* elem_order, const int32_t* dofs_m,
                                                   const float2* gdet, const double* mass, const double* field,
-                                                  const double* scale, double* y, int two_valued)
+                                                  const double* scale, double* y, int two_valued, double volume)
 {
   constexpr int NB = ORDER == 1 ? 4 : 10, NU = ORDER == 1 ? 10 : 55;
   __shared__ ff tab[NU];
@@ -1936,8 +1959,11 @@ __global__ void __launch_bounds__(256) k_rhs_elem(int64_t n_elem, const int32_t*
   // back to the true scale 2^k2
   const int k2 = (es - 1023) + (ef - 1023);
 #pragma unroll
-  for (int l = 0; l < NB / 2; ++l)
-    out[l] = make_double2(ff_to_double_pow2(v[2 * l], k2), ff_to_double_pow2(v[2 * l + 1], k2));
+  for (int l = 0; l < NB / 2; ++l) {
+    double2 w = make_double2(ff_to_double_pow2(v[2 * l], k2), ff_to_double_pow2(v[2 * l + 1], k2));
+    if (volume != 1.0) w = make_double2(w.x * volume, w.y * volume);  // from the geometry cache's scale
+    out[l] = w;
+  }
 }
 
 // Pass 2, G lanes per dof: b_i = the FP64 sum of its element-vector entries,
@@ -1998,6 +2024,7 @@ struct RhsArgs {
   double *partial, *b;
   const int32_t* all_partial;  // rhs_ptr where b may overlap an input, else null (rhs_put)
   int form;     // of M^ f
+  int det_exp;  // gdet holds 2^-det_exp of the determinants (3 mg_mesh::geo_exp)
   double unit;  // factor of the sums (1 with the full table), a normal number
 };
 // M^ f: u (sum_k f_k + f_l) where the table is u (1 + [l = k]) (the symmetric cards of two
@@ -2074,15 +2101,15 @@ __device__ __forceinline__ RhsElement rhs_element(const double* f, uchar4 q, dou
   }
   return e;
 }
-__device__ __forceinline__ double rhs_value(const RhsElement& e, ff v)
+__device__ __forceinline__ double rhs_value(const RhsElement& e, int det_exp, ff v)
 {
   if (e.nan) return __longlong_as_double(0x7ff8000000000000ll);
   const double x = ff_to_double_bits(v);
   // in the normal range the powers go into the exponent, off the FP64 pipe
-  const int ex = dexp(x), k = e.k + e.kdet;
+  const int ex = dexp(x), kdet = e.kdet + det_exp, k = e.k + kdet;
   if (ex == 0 || ex == 0x7ff) return x;
   if (ex + k >= 1 && ex + k <= 2046) return __longlong_as_double(__double_as_longlong(x) + ((long long)k << 52));
-  return scale_pow2(x * (e.kdet ? 0x1p64 : 1.0), e.k);
+  return scale_pow2(x * __longlong_as_double((long long)(kdet + 1023) << 52), e.k);
 }
 
 // Shared memory of a block
@@ -2119,8 +2146,8 @@ static __device__ __noinline__ void rhs_block_wide(const RhsArgs& a, RhsShared& 
   for (int l = 0; l < 4; ++l) {
     const ff2 w = ff2_mul(v[l], ff2_make(u, u));
     const float2 h = f2_get(w.hi), lo = f2_get(w.lo);
-    y[l * kElemBlock + lp] = rhs_value(e1, ff{h.x, lo.x});
-    y[l * kElemBlock + lp + 32] = rhs_value(e2, ff{h.y, lo.y});
+    y[l * kElemBlock + lp] = rhs_value(e1, a.det_exp, ff{h.x, lo.x});
+    y[l * kElemBlock + lp + 32] = rhs_value(e2, a.det_exp, ff{h.y, lo.y});
   }
   __syncthreads();
   if ((int)threadIdx.x < n_nodes) {
@@ -2248,7 +2275,7 @@ __global__ void __launch_bounds__(256, 5) k_rhs_block(RhsArgs a)
     }
     // det's power goes into the factor (2^-27 .. 1): with the others it would leave
     // scale_pow2's range
-    const double unit = __longlong_as_double(__double_as_longlong(a.unit) + ((long long)(ed - 127) << 52));
+    const double unit = __longlong_as_double(__double_as_longlong(a.unit) + ((long long)(ed - 127 + a.det_exp) << 52));
     rhs_put(a, out, scale_pow2(unit * sum.result(), (ef > 0 ? ef - 1023 : 0) + (es > 0 ? es - 1023 : 0)));
   }
 }
@@ -2373,7 +2400,7 @@ static mg_status plan_geometry(mg_plan* p, cudaStream_t st)
     cudaFree(det);
     return set_error(MG_ERR_ALLOC, "element geometry cache: out of device memory");
   }
-  const GeoPtrs geo{m->d_xyz, m->d_node_rec, m->d_lo_z};
+  const GeoPtrs geo{m->geo_exp ? m->d_xyz_rec : m->d_xyz, m->d_node_rec, m->d_lo_z};
   const unsigned blocks = (unsigned)((E + 255) / 256);
   const auto kernel = m->order == 1 ? (m->grid_split ? k_elem_geometry<4, true> : k_elem_geometry<4, false>)
                                     : (m->grid_split ? k_elem_geometry<10, true> : k_elem_geometry<10, false>);
@@ -2408,10 +2435,10 @@ mg_status mg_adjoint_grad(mg_plan* p, const double* d_u, const double* d_lambda,
   if (blocks > 0) {
     if (m->order == 1)
       MG_CUDA(launch_pdl(k_adjoint<1>, blocks, threads, st, m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det,
-                         p->d_geo_cof, d_tab, t->wsum, d_u, d_lambda, d_grad));
+                         p->d_geo_cof, d_tab, std::ldexp(t->wsum, m->geo_exp), d_u, d_lambda, d_grad));
     else
       MG_CUDA(launch_k(false, k_adjoint<2>, blocks, threads, st, m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det,
-                         p->d_geo_cof, d_tab, t->wsum, d_u, d_lambda, d_grad));
+                         p->d_geo_cof, d_tab, std::ldexp(1.0, m->geo_exp), d_u, d_lambda, d_grad));
   }
   return MG_OK;
 }
@@ -2462,7 +2489,7 @@ mg_status mg_assemble_rhs(mg_plan* p, const double* d_field, const double* d_ele
     const RhsArgs a{m->n_elem,       p->d_elem_order, p->d_bnode,       p->d_bnode_n, p->d_elem_local,
                     p->d_geo_det,    d_tab + 6 * nu,  d_field,          d_elem_scale, p->d_rhs_bpos,
                     p->d_rhs_bstart, p->d_rhs_bout,   p->d_rhs_partial, d_b,          in_place ? p->d_rhs_ptr : nullptr,
-                    form,            form == kRhsTable ? 1.0 : off};
+                    form,            3 * m->geo_exp,  form == kRhsTable ? 1.0 : off};
     MG_CUDA(launch_pdl(k_rhs_block, (int)p->n_blocks, 256, st, a));
     MG_CUDA(launch_pdl(k_rhs_shared, (int)((p->ndof + 255) / 256), 256, st, p->ndof, (const int32_t*)p->d_rhs_ptr,
                        (const double*)p->d_rhs_partial, in_place ? 1 : 0, d_b));
@@ -2470,12 +2497,13 @@ mg_status mg_assemble_rhs(mg_plan* p, const double* d_field, const double* d_ele
   }
   MG_TRY(plan_rhs_map(p));
   if (eblocks > 0) {
+    const double volume = std::ldexp(1.0, 3 * m->geo_exp);
     if (m->order == 1)
       k_rhs_elem<1><<<eblocks, threads, 0, st>>>(m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det,
-                                                 d_tab + 6 * nu, d_field, d_elem_scale, p->d_rhs_y, two_valued);
+                                                 d_tab + 6 * nu, d_field, d_elem_scale, p->d_rhs_y, two_valued, volume);
     else
       k_rhs_elem<2><<<eblocks, threads, 0, st>>>(m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det,
-                                                 d_tab + 6 * nu, d_field, d_elem_scale, p->d_rhs_y, 0);
+                                                 d_tab + 6 * nu, d_field, d_elem_scale, p->d_rhs_y, 0, volume);
     MG_CUDA(cudaGetLastError());
   }
   // two lanes per dof when dofs sum more than 16 entries on average (P1: ~24),

@@ -109,12 +109,15 @@ struct mg_mesh {
   std::vector<int32_t> tri_geo;     //   and their geoIds (2nd tag)
   // device copies
   double4_32a* d_xyz = nullptr;      // (x, y, z, 0)
+  double4_32a* d_xyz_rec = nullptr;  // the same times 2^-geo_exp, where that is not 1
   // x = hi + mid + lo (three floats per coordinate), packed so that one 32-byte
   // sector holds a node's (hi.xyz, mid.xyz, lo.x, lo.y); lo.z apart.  grid_split:
   // hi and mid are multiples of per-axis units, so that differences of the hi and
   // of the mid parts are exact (build_node_records); else each part is the
   // remainder rounded to a float, and the sum is exact
+  // Both of 2^-geo_exp x: 0 but for very small meshes (build_node_records).
   bool grid_split = false;
+  int geo_exp = 0;
   float4* d_node_rec = nullptr;  // 2 float4 per node
   float* d_lo_z = nullptr;
   int4* d_conn = nullptr;        // vertex node ids
@@ -191,7 +194,7 @@ struct mg_plan {
   int32_t* d_rhs_bout = nullptr;      // kStageNodes per block
   double* d_rhs_partial = nullptr;    // one per (block, node)
   // element geometry in double-word form (built on the first call that needs it:
-  // load vector, adjoint), Morton order p: det[p] and cofactor k of element p at
+  // load vector, adjoint) on the node records' scale, Morton order p: det[p] and cofactor k of element p at
   // cof[k * n_elem + p] (k = 3 r + c), each (hi, lo) floats
   float2* d_geo_det = nullptr;
   float2* d_geo_cof = nullptr;

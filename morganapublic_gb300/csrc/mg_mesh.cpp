@@ -322,6 +322,7 @@ static void free_mesh(mg_mesh* m)
 {
   if (!m) return;
   cudaFree(m->d_xyz);
+  cudaFree(m->d_xyz_rec);
   cudaFree(m->d_node_rec);
   cudaFree(m->d_lo_z);
   cudaFree(m->d_conn);

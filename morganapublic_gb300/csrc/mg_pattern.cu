@@ -41,6 +41,14 @@ namespace mg {
 // would leave the normal floats, take the general split (each part the remainder
 // rounded to a float, exact), whose differences cost error-free sums.
 
+// The records of a mesh that lies within 2^kSmallMesh of the origin are of its coordinates
+// times a power of two that brings the largest near one: the element kernels' products
+// of cofactors, the fourth power of an edge, would leave the normal floats (a mesh of
+// 1e-9 edges: FP64 stiffness to 5e-9, of 1e-12 edges: zero).  The power, which only
+// shifts exponents, is taken back with the entries' weights.  The least keeps 2^geo_exp
+// and its products with the weights normal floats.
+constexpr int kSmallMesh = -8, kLeastGeoExp = -90;
+
 // stats: per axis the largest |x| (bits of a double), then the smallest altitude
 // over 2^emax (bits of a float)
 __global__ void __launch_bounds__(256) k_node_xyz(int64_t N, const double* __restrict__ raw, double4_32a* __restrict__ xyz,
@@ -124,7 +132,8 @@ __global__ void __launch_bounds__(256) k_min_altitude(int64_t E, const int4* __r
 
 struct SplitGrid {
   int on;
-  int e[3];  // per axis
+  int e[3];      // per axis, of scale * x
+  double scale;  // a power of two
 };
 
 __device__ __forceinline__ void split3(double x, const SplitGrid& g, int k, float& h, float& m, float& l)
@@ -145,11 +154,14 @@ __device__ __forceinline__ void split3(double x, const SplitGrid& g, int k, floa
 }
 
 __global__ void __launch_bounds__(256) k_node_split(int64_t N, const double4_32a* __restrict__ xyz, SplitGrid g,
-                                                    float4* __restrict__ rec, float* __restrict__ loz)
+                                                    double4_32a* __restrict__ scaled, float4* __restrict__ rec,
+                                                    float* __restrict__ loz)
 {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const double4_32a p = xyz[i];
+  double4_32a p = xyz[i];
+  p.x *= g.scale, p.y *= g.scale, p.z *= g.scale;
+  if (scaled) scaled[i] = p;
   float h[3], m[3], l[3];
   split3(p.x, g, 0, h[0], m[0], l[0]);
   split3(p.y, g, 1, h[1], m[1], l[1]);
@@ -163,6 +175,7 @@ mg_status build_node_records(mg_mesh* m)
 {
   const int64_t N = m->n_nodes, E = m->n_elem;
   m->grid_split = false;
+  m->geo_exp = 0;
   if (N == 0) return MG_OK;
   // the coordinates as they are on the host (24 bytes a node) and the statistics wait in
   // the records' own memory (32) and in lo's (kStatsFloats at least)
@@ -189,6 +202,11 @@ mg_status build_node_records(mg_mesh* m)
     for (int k = 0; k < 3; ++k) {
       g.e[k] = grid_exponent(h[k]);
       emax = std::max(emax, g.e[k]);
+    }
+    m->geo_exp = emax < kSmallMesh ? std::max(emax, kLeastGeoExp) : 0;
+    g.scale = pow2(-m->geo_exp);
+    for (int k = 0; k < 3; ++k) {
+      g.e[k] -= m->geo_exp;
       if (g.e[k] < -50 || g.e[k] > 100) fits = false;
     }
     if (fits && eb > 0) {
@@ -201,7 +219,10 @@ mg_status build_node_records(mg_mesh* m)
     }
   }
   if (e == cudaSuccess) {
-    k_node_split<<<nb, 256, 0, st>>>(N, m->d_xyz, g, m->d_node_rec, m->d_lo_z);
+    if (m->geo_exp != 0) e = cudaMalloc(&m->d_xyz_rec, sizeof(double4_32a) * N);
+  }
+  if (e == cudaSuccess) {
+    k_node_split<<<nb, 256, 0, st>>>(N, m->d_xyz, g, m->d_xyz_rec, m->d_node_rec, m->d_lo_z);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   }
