@@ -513,7 +513,8 @@ __device__ __forceinline__ bool cancels(float t0, float t1, float t2, float det)
 __device__ __forceinline__ bool diag_spread(float k0, float k1, float k2, float k3)
 {
   k0 = fabsf(k0), k1 = fabsf(k1), k2 = fabsf(k2), k3 = fabsf(k3);
-  return fmaxf(fmaxf(k0, k1), fmaxf(k2, k3)) > 64.0f * fminf(fminf(k0, k1), fminf(k2, k3));
+  // true where all are NaN, of a scale factor above the floats
+  return !(fmaxf(fmaxf(k0, k1), fmaxf(k2, k3)) <= 64.0f * fminf(fminf(k0, k1), fminf(k2, k3)));
 }
 
 // The node records of a block: its unique nodes staged in shared memory, indexed by
