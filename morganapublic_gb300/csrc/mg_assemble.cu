@@ -1889,7 +1889,9 @@ __device__ __forceinline__ ff ff_scaled(double v, int emax)
 // mass table of the quadrature card.  Double-word arithmetic; s_e and the f_k
 // are rescaled by powers of two (their largest exponents), so the result keeps
 // FP64 accuracy at any scale, and is written as an IEEE double.
-template <int ORDER>
+// SCALED: the geometry cache is on another scale than the mesh (volume = 2^(3 geo_exp)); the
+// test in one kernel for both took P2 32^3 from 43.2 to 45.1 us.
+template <int ORDER, bool SCALED>
 __global__ void __launch_bounds__(256) k_rhs_elem(int64_t n_elem, const int32_t* elem_order, const int32_t* dofs_m,
                                                   const float2* gdet, const double* mass, const double* field,
                                                   const double* scale, double* y, int two_valued, double volume)
@@ -1962,7 +1964,7 @@ __global__ void __launch_bounds__(256) k_rhs_elem(int64_t n_elem, const int32_t*
 #pragma unroll
   for (int l = 0; l < NB / 2; ++l) {
     double2 w = make_double2(ff_to_double_pow2(v[2 * l], k2), ff_to_double_pow2(v[2 * l + 1], k2));
-    if (volume != 1.0) w = make_double2(w.x * volume, w.y * volume);  // from the geometry cache's scale
+    if constexpr (SCALED) w = make_double2(w.x * volume, w.y * volume);
     out[l] = w;
   }
 }
@@ -2499,12 +2501,12 @@ mg_status mg_assemble_rhs(mg_plan* p, const double* d_field, const double* d_ele
   MG_TRY(plan_rhs_map(p));
   if (eblocks > 0) {
     const double volume = std::ldexp(1.0, 3 * m->geo_exp);
-    if (m->order == 1)
-      k_rhs_elem<1><<<eblocks, threads, 0, st>>>(m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det,
-                                                 d_tab + 6 * nu, d_field, d_elem_scale, p->d_rhs_y, two_valued, volume);
-    else
-      k_rhs_elem<2><<<eblocks, threads, 0, st>>>(m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det,
-                                                 d_tab + 6 * nu, d_field, d_elem_scale, p->d_rhs_y, 0, volume);
+    const auto elements = [&](auto kernel) {
+      kernel<<<eblocks, threads, 0, st>>>(m->n_elem, p->d_elem_order, p->d_dofs_morton, p->d_geo_det, d_tab + 6 * nu,
+                                          d_field, d_elem_scale, p->d_rhs_y, m->order == 1 ? two_valued : 0, volume);
+    };
+    if (m->order == 1) elements(m->geo_exp == 0 ? k_rhs_elem<1, false> : k_rhs_elem<1, true>);
+    else elements(m->geo_exp == 0 ? k_rhs_elem<2, false> : k_rhs_elem<2, true>);
     MG_CUDA(cudaGetLastError());
   }
   // two lanes per dof when dofs sum more than 16 entries on average (P1: ~24),
