@@ -297,8 +297,8 @@ mg_status mg_assemble_host(mg_plan* plan, int32_t op, const double* h_coeff, dou
    d_b (ndof doubles; it may overlap d_field or d_elem_scale).  Element vectors in double-word arithmetic (FP64-accurate
    at any scale of s and f), then one FP64 sum per dof in a fixed order:
    deterministic, no atomics.  The first call on a plan builds the sums' map (P1
-   meshes whose 512-element blocks hold at most 256 nodes each: about 14 bytes per
-   element, built on the GPU; others: 4 bytes per element-vector entry and a work
+   meshes whose 512-element blocks hold at most 256 nodes each: 15 bytes per element
+   and 4 per node, built on the GPU; others: 4 bytes per element-vector entry and a work
    buffer of 8) and the element-geometry cache (80 bytes per element) on the device, and
    waits for them: make that first call before capturing a CUDA graph.
    Replaces: vectorBuilder<localVectorEL3d<fnEL3dA|fnEL3dB>>::buildEpetraVector
@@ -493,14 +493,14 @@ mg_status mg_lagrange_export_products(const mg_lagrange* lg, int32_t which, int3
                                       int32_t* h_slot);
 
 /* Values of B (nnz_b doubles, device) with the face card quad (MG_FACE_QUAD_*):
-   one thread per face computes its nt x nb block, then one thread per entry of
-   B sums its blocks' contributions in the reference's insertion order
-   (deterministic, no atomics).  The first device call on a handle (this one,
-   mg_saddle_assemble, mg_saddle_spmv or mg_lagrange_apply) uploads its tables
-   and waits for the copies: make it before capturing a CUDA graph.  The face
-   blocks go through one staging buffer of the handle, so calls of this
-   function on one handle that overlap on the GPU (other streams or host
-   threads) race: serialise them. */
+   one thread per face computes twice its area, then one thread per entry of B sums
+   area times the entry of the card's unit-face table over its faces, in the
+   reference's insertion order (deterministic, no atomics).  The first device
+   call on a handle (this one, mg_saddle_assemble, mg_saddle_spmv or
+   mg_lagrange_apply) uploads its tables and waits for the copies: make it before
+   capturing a CUDA graph.  The face areas go through one buffer of the handle, so
+   calls of this function on one handle that overlap on the GPU (other streams or
+   host threads) race: serialise them. */
 mg_status mg_lagrange_assemble(mg_lagrange* lg, int32_t quad, double* d_b_values, void* stream);
 /* mg_lagrange_assemble with the values copied to host memory (nnz_b doubles):
    what buildEpetraCrs hands to Epetra for localMatrixLA3d.  Synchronous. */

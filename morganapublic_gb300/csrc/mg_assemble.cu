@@ -9,10 +9,11 @@
 //                  and written to the entry and its mirror; entries whose elements
 //                  span blocks get a partial sum per block, added in block order by
 //                  k_shared_sum;
-//   P2 (two passes) k_elem_mat: one thread per element, its 55 unique entries to
-//                  the plan's element-matrix array; k_slot_gather: one thread
-//                  per diagonal or upper CSR entry, the sum of its entries in
-//                  ascending Morton position (the plan's slot map).
+//   P2 (two passes) k_elem_mat_pair: two elements per thread, packed, their 55
+//                  unique entries to the plan's element-matrix array;
+//                  k_slot_gather: one thread per diagonal or upper CSR entry, the
+//                  sum of its entries in ascending Morton position (the plan's
+//                  slot map).
 // No atomics touch values; the per-entry summation order is fixed by the plan,
 // so the results are bitwise reproducible.
 //
@@ -304,33 +305,13 @@ __device__ __forceinline__ void metric(const Cof<T>& f, T s, T g[6])
     g[p] = s * (f.c[0][pa[p]] * f.c[0][pb[p]] + f.c[1][pa[p]] * f.c[1][pb[p]] + f.c[2][pa[p]] * f.c[2][pb[p]]);
 }
 
-// sum_{p<6} g[p] tab[p * NU + u] (the P2 metric contraction).  Double-word:
-// error-free products of the high words chained with two_sum, the low-order
-// terms in one float, one renormalisation (instead of one per operation).
-template <typename T>
-__device__ __forceinline__ T metric_dot(const T g[6], const T* tab, int NU, int u)
+// sum_{p<6} g[p] tab[p * NU + u] (the P2 metric contraction)
+__device__ __forceinline__ double metric_dot(const double g[6], const double* tab, int NU, int u)
 {
-  T v = g[0] * tab[u];
+  double v = g[0] * tab[u];
 #pragma unroll
   for (int k = 1; k < 6; ++k) v = v + g[k] * tab[k * NU + u];
   return v;
-}
-template <>
-__device__ __forceinline__ ff metric_dot<ff>(const ff g[6], const ff* tab, int NU, int u)
-{
-  const ff t0 = tab[u];
-  const ff p0 = two_prod(g[0].hi, t0.hi);
-  float hi = p0.hi;
-  float lo = __fmaf_rn(g[0].hi, t0.lo, __fmaf_rn(g[0].lo, t0.hi, p0.lo));
-#pragma unroll
-  for (int k = 1; k < 6; ++k) {
-    const ff t = tab[k * NU + u];
-    const ff q = two_prod(g[k].hi, t.hi);
-    const ff s = two_sum(hi, q.hi);
-    hi = s.hi;
-    lo = __fadd_rn(lo, __fadd_rn(s.lo, __fmaf_rn(g[k].hi, t.lo, __fmaf_rn(g[k].lo, t.hi, q.lo))));
-  }
-  return two_sum(hi, lo);
 }
 
 // ------------------------------------------------------------ assembly --
@@ -877,8 +858,9 @@ __host__ __device__ constexpr int g_index(int a, int b)
   return a <= b ? a * 4 - a * (a - 1) / 2 + (b - a) : b * 4 - b * (b - 1) / 2 + (a - b);
 }
 
-// sum_k g[i_k] t[k], N terms (i0 .. i3 the indices): double-word as in metric_dot,
-// packed; table entries as (hi, hi, lo, lo)
+// sum_k g[i_k] t[k], N terms (i0 .. i3 the indices): packed; double-word: error-free
+// products of the high words chained with two_sum, the low-order terms in one float,
+// one renormalisation; table entries as (hi, hi, lo, lo)
 template <int N>
 __device__ __forceinline__ ff2 bary_sum(const ff2 (&g)[10], const f2 (&ng)[10], const float4* t, int i0, int i1, int i2, int i3)
 {
@@ -1122,7 +1104,7 @@ __global__ void __launch_bounds__(256, 1) k_elem_mat_f64(ElemArgs a)
     double g[6];
     metric<double>(f, coef / f.det, g);
 #pragma unroll 5
-    for (int u = 0; u < NU; ++u) em_put(a.em, u * E + p, metric_dot<double>(g, tab, NU, u));
+    for (int u = 0; u < NU; ++u) em_put(a.em, u * E + p, metric_dot(g, tab, NU, u));
   } else {
     const double sc = coef * f.det;
 #pragma unroll 5
@@ -1231,10 +1213,10 @@ __global__ void __launch_bounds__(256) k_slot_gather(int64_t n_groups, int64_t n
 // launched with programmatic dependent launch: what they read of the plan overlaps
 // the tail of the kernel before.
 //
-// What bounds it on GB300 (P1 128^3, FP64, one assembly 949 -> 709 us; FP32 at 64^3
-// 75 -> 61 us, both with k_shared_sum).  One element per thread and scalar
+// What bounds it on GB300 (P1 128^3, FP64, one assembly 949 -> 711 us; FP32 at 64^3
+// 74 -> 56 us, both with k_shared_sum).  One element per thread and scalar
 // double-words took 46 warp instructions per element at 57 % issue.  The packed
-// pairs with grid-split coordinates take 27, and left latency as the bound:
+// pairs with grid-split coordinates take 30, and left latency as the bound:
 //   - random vertex and coefficient loads need an L1 line each while in flight,
 //     and the blocks' shared memory leaves few lines: nodes staged by cp.async 833 ->
 //     743 us, coefficients by cp.async 782 -> 745 us;
@@ -1867,14 +1849,11 @@ __global__ void __launch_bounds__(256, ORDER == 1 ? 5 : 1) k_adjoint(int64_t n_e
   grad[e] = -ff_to_double_pow2(s, (eu - 1023) + (el - 1023));
 }
 
-// v 2^(1023 - emax) as a double-word value, emax the block's largest biased exponent;
-// zero below the normal doubles, and some value of 2^-100 where v is more than 74
-// binades below the largest (nonzero, and negligible beside it)
+// v 2^(1023 - emax) as a double-word value, emax the block's largest biased exponent and
+// v zero or a normal number within 2^70 of it
 __device__ __forceinline__ ff ff_scaled(double v, int emax)
 {
-  const int e = dexp(v);
-  if (e == 0) return ff{0.0f, 0.0f};
-  if (e + 74 < emax) return ff{0x1p-100f, 0.0f};
+  if (dexp(v) == 0) return ff{0.0f, 0.0f};
   return ff_from_double_bits(__longlong_as_double(__double_as_longlong(v) - ((long long)(emax - 1023) << 52)));
 }
 
@@ -2014,7 +1993,8 @@ __global__ void __launch_bounds__(256) k_rhs_gather(int64_t ndof, const int32_t*
 // warp instructions per element, a third of them conversions: GB300, P1 96^3, 217 ->
 // 141 us (block kernel 126, shared nodes 14; bound by issue and the L1 data path, 61 %
 // each), 134 with programmatic launches, the table staged only where it is used and
-// no FP64 comparisons; the map is built on the GPU (first call on a plan 76 -> 1.6 ms).
+// no FP64 comparisons, 123 with the powers of two in the factor's exponent and the spread
+// blocks out of line; the map is built on the GPU (first call on a plan 76 -> 1.6 ms).
 struct RhsArgs {
   int64_t n_elem;
   const int32_t *elem_order, *bnode, *bnode_n;

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kAreaThreads) k_face_area(int64_t n_faces, con
 
 // vals[k] = sum over j in [ptr[k], ptr[k+1]), in list order, of area2 of face src[j] / nt
 // nb times the entry src[j] % (nt nb) of its local face's table.  Bound by the latency
-// of its loads: the list's are taken four at a time and before the wait.
+// of its loads: the list's are taken two at a time, the first ones before the wait.
 template <int NTB>
 __global__ void __launch_bounds__(kFaceThreads) k_gather_sum(int64_t n, const int32_t* __restrict__ ptr,
                                                              const int32_t* __restrict__ src,

@@ -69,7 +69,7 @@ __global__ void k_elem_keys(int64_t E, const int4* __restrict__ conn, const doub
   ids[e] = (int32_t)e;
 }
 
-// row weight max(len, 4) in Morton order
+// the elements' dofs in Morton order
 __global__ void k_dofs_morton(int64_t E, int nb, const int32_t* __restrict__ elem_order, const int32_t* __restrict__ dofs,
                               int32_t* __restrict__ out)
 {
@@ -137,8 +137,10 @@ mg_status upload_to(BuildBuffers& B, T** d, const std::vector<T>& h, cudaStream_
 //      dof's list ascends in q, hence in p);
 //   2. one thread per row: its upper entries and their contributions counted;
 //      exclusive scans give each row's first upper entry and first source;
-//   3. one thread per row: per-entry counts (a binary search of each coupled
-//      column in the row), their prefix, then the sources in incidence order.
+//   3. a group of lanes per row, a lane per upper entry: its column looked for among the
+//      dofs of the row's elements, to count its sources, then (offsets by a scan over the
+//      group) to write them in incidence order; rows of more than kSerialRow elements
+//      by one thread that searches each coupled column in the row.
 
 __global__ void k_iota32(int64_t n, uint32_t* v)
 {
