@@ -2052,8 +2052,8 @@ __device__ __forceinline__ void rhs_pair(int form, const ff* tab, const ff2 (&F)
   }
 }
 
-// One element's share of rhs_block_wide: s and f near one, the power of two that was taken
-// out (with the determinant's, 0 or 64, apart), and whether the vector is NaN (s or an f
+// One element's share of rhs_block_wide: s, f and det near one, the powers of two that were
+// taken out (the determinant's apart), and whether the vector is NaN (s or an f
 // Inf or NaN) or zero (s, or all f, zero or subnormal), the rules of k_rhs_elem.
 struct RhsElement {
   ff F[4], s, det;
@@ -2068,8 +2068,9 @@ __device__ __forceinline__ RhsElement rhs_element(const double* f, uchar4 q, dou
   e.nan = es == 0x7ff || ef == 0x7ff;
   e.zero = es == 0 || ef == 0;
   e.k = (es - 1023) + (ef - 1023);
-  e.kdet = fabsf(d.x) >= 0x1p64f ? 64 : 0;  // products with a larger one may overflow
-  const float dscale = e.kdet ? 0x1p-64f : 1.0f;
+  // (products of a determinant as it is may overflow, or lose their errors below the floats)
+  e.kdet = min(max((int)((__float_as_uint(d.x) >> 23) & 0xffu) - 127, -126), 126);
+  const float dscale = __uint_as_float((uint32_t)(127 - e.kdet) << 23);
   e.det = ff{d.x * dscale, d.y * dscale};
   if (e.nan || e.zero) {
 #pragma unroll
@@ -2107,7 +2108,7 @@ struct RhsShared {
 
 // A block whose values spread too far for one scale: s and f of every element by their own
 // powers of two, as k_rhs_elem takes them, and the element vectors as doubles.  GB300,
-// P1 96^3, every block of this kind: 210 us, 727 with the block in native FP64 (the
+// P1 96^3, every block of this kind: 213 us, 727 with the block in native FP64 (the
 // two-pass form: 216; two FP64 products per entry for its power of two: 228).
 static __device__ __noinline__ void rhs_block_wide(const RhsArgs& a, RhsShared& sh, int n_nodes, int32_t out)
 {

@@ -62,3 +62,19 @@ def test_spread(n, field, quad):
     # entry is rounded to the doubles' spacing there
     entries = np.bincount(m.conn.ravel(), minlength=N)
     assert np.all(np.abs(got - ref) <= 1e-13 * mag + entries * np.longdouble(2) ** -1075)
+
+
+@pytest.mark.parametrize("quad", [1, 4, 64])
+@pytest.mark.parametrize("n", [5, 20])
+@pytest.mark.parametrize("size", [1e-9, 1e9])
+def test_spread_with_small_and_large_determinants(n, size, quad):
+    # (size 1e-9, and an offset that keeps the coordinates near one: determinants of 2^-103)
+    import morganapublic_gb300 as mg
+    m = meshgen.kuhn_cube(n, jitter=0.2, seed=2, permute=True)
+    xyz = m.xyz * size + 1.0
+    rng = np.random.default_rng(n)
+    f, s = rng.uniform(-2, 2, len(xyz)), rng.uniform(0.5, 2, len(m.conn))
+    f[::13] = 1e-30
+    got = mg.MatrixBuilder(mg.Mesh(xyz, m.conn, order=1)).build_vector(field=f, elem_scale=s, quad=quad).cpu().numpy()
+    ref, mag = _reference(xyz, m.conn, f, s, quad)
+    assert np.all(np.abs(got - ref) <= 1e-13 * mag)
