@@ -62,7 +62,8 @@ def fake(tmp_path_factory):
 
 
 def _run(fake, mode):
-    env = dict(os.environ, LD_PRELOAD=fake, FAKE_LAUNCH=mode.split(":")[0], FAKE_SPINS=mode.split(":")[-1])
+    preload = " ".join(filter(None, [os.environ.get("LD_PRELOAD"), fake]))
+    env = dict(os.environ, LD_PRELOAD=preload, FAKE_LAUNCH=mode.split(":")[0], FAKE_SPINS=mode.split(":")[-1])
     r = subprocess.run([sys.executable, "-c", CHILD.format(root=ROOT, here=HERE, mode=mode)], env=env, text=True,
                        stdout=subprocess.PIPE, stderr=subprocess.STDOUT, timeout=300)
     assert r.returncode == 0 and "fallback ok" in r.stdout, r.stdout[-3000:]
